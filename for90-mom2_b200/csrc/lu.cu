@@ -2,9 +2,11 @@
 //
 // Replaces ZGETRF + ZGETRS of solve_multi_linsys (linalg.f90:159-180).
 // Right-looking blocked LU, panel width nb:
-//   panel_kernel   cooperative, one CTA per SM, the panel held in shared
-//                  memory; per column one bounded grid barrier, pivot =
-//                  first row of largest |re|+|im| (izamax), FP64 arithmetic;
+//   panel          pivot = row of largest |re|+|im| (izamax); on one
+//                  thread-block cluster with the rows in registers
+//                  (lu_panel.cu), or, too tall for it, panel_kernel:
+//                  cooperative, one CTA per SM, the panel in shared memory,
+//                  one bounded exchange through global memory per column;
 //   laswp_kernel   the panel's row interchanges on the other columns;
 //   diag_inv       inverses of the unit-lower and upper diagonal blocks;
 //   TRSM as GEMM   U12 = inv(L11) A12, then A22 -= L21 U12 (plain library
@@ -311,189 +313,6 @@ __global__ void __launch_bounds__(kPanelThreads, 1) panel_kernel(PanelArgs a) {
       st2(A + (row0 + ii) + (a.j0 + c) * a.lda, low ? cmul(v, rp) : v);
     }
   }
-}
-
-// ---- short panels: one thread-block cluster, exchange in distributed shared memory ----
-
-constexpr int kMaxCluster = 16;
-// rows per CTA of a cluster panel (slab + pushed rows in shared memory): 176
-// with the FP64 slab, 352 with the FP32 slab of the mixed path
-template <typename T> constexpr int kClusterRows = sizeof(typename SlabOf<T>::type) == 8 ? 352 : 176;
-
-__device__ __forceinline__ unsigned map_shared(const void *p, unsigned rank) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-  unsigned r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void st_cluster_u64(unsigned addr, unsigned long long v) {
-  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
-}
-__device__ __forceinline__ double2 ld_cluster_d2(unsigned addr) {
-  double2 v;
-  asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(addr) : "memory");
-  return v;
-}
-// Every thread of every CTA of the cluster; orders shared-memory accesses
-// across the cluster (release / acquire).
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void st_cluster_d2(unsigned addr, double2 v) {
-  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(v.x), "d"(v.y) : "memory");
-}
-__device__ __forceinline__ void st_cluster_d2(unsigned addr, float2 v) {
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
-}
-
-// The same panel factorisation as panel_kernel for panels of at most
-// kClusterRows<T> * kMaxCluster rows, on a grid that is exactly one cluster of
-// P CTAs (all co-scheduled by the hardware).  Per column each CTA pushes
-// its packed candidate key and the candidate row (and the owner of row col
-// that row) into every CTA's shared memory, then one cluster barrier; the
-// winner, the pivot row and the displaced row are then read locally.  The
-// pushed buffers alternate by column parity, so one barrier per column
-// suffices.  No global memory round trip and no spin-wait: every thread of
-// the cluster executes the same sequence of cluster barriers.
-template <typename T>
-__global__ void __launch_bounds__(kPanelThreads, 1) panel_cluster_kernel(PanelArgs a) {
-  using E = typename SlabOf<T>::type;
-  extern __shared__ __align__(16) unsigned char cluster_smem[];
-  E *slab = reinterpret_cast<E *>(cluster_smem);  // [nb][rpc] column-major, then the pushed rows
-  __shared__ unsigned long long w_key[kPanelThreads / 32];
-  __shared__ unsigned long long c_key[2][kMaxCluster];
-  __shared__ E s_prow_data[64];
-  __shared__ E s_rpc[64];  // 1 / pivot of each column (0: failed pivot)
-  __shared__ E s_rp;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, cta = blockIdx.x;  // cta == cluster rank
-  const int nb = a.nb, rpc = a.rpc, P = a.P;
-  E *recv_row = slab + (size_t)nb * rpc;           // [2][P][nb] candidate rows by sender
-  E *recv_col = recv_row + (size_t)2 * P * nb;    // [2][nb] row col, from its owner
-  T *A = reinterpret_cast<T *>(a.A);
-  const int64_t row0 = a.j0 + (int64_t)cta * rpc;
-  const int64_t rem = a.n - row0;
-  const int nrow = rem <= 0 ? 0 : (rem < rpc ? (int)rem : rpc);
-  for (int base = tid; base < nb * rpc; base += 8 * kPanelThreads) {
-    E v[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int idx = base + u * kPanelThreads;
-      const int c = idx / rpc, i = idx % rpc;
-      v[u] = (idx < nb * rpc && i < nrow) ? ld_slab<E>(A + (row0 + i) + (a.j0 + c) * a.lda)
-                                          : from_d2<E>(make_double2(0, 0));
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int idx = base + u * kPanelThreads;
-      if (idx < nb * rpc) slab[idx] = v[u];
-    }
-  }
-  __syncthreads();
-  const int S = kPanelThreads / rpc;  // threads per row (rpc <= kPanelThreads)
-  const int i = tid % rpc, sph = tid / rpc;
-  const bool mine = sph < S && i < nrow;
-  const int64_t g = row0 + i;  // global row of this thread
-  double cv = (mine && sph == 0) ? cabs1(slab[i]) : -1.0;  // candidate for column 0
-  for (int c = 0; c < nb; c++) {
-    const int64_t col = a.j0 + c;
-    const int par = c & 1;
-    // 1. CTA candidate; push key and row (and row col, if owned) to every CTA
-    const unsigned long long wk = warp_max_key(cv >= 0.0 ? pack_candidate(cv, g, a.j0, 0) : 0ull);
-    if (lane == 0) w_key[wid] = wk;
-    __syncthreads();
-    if (wid == 0) {
-      const unsigned long long bkey = warp_max_key(lane < kPanelThreads / 32 ? w_key[lane] : 0ull);
-      if (lane < P) st_cluster_u64(map_shared(&c_key[par][cta], (unsigned)lane), bkey);
-      if (bkey != 0ull) {
-        const int li = (int)(0xffffffu - (unsigned)((bkey >> 8) & 0xffffffu)) - (int)(row0 - a.j0);
-        const E v0 = slab[lane * rpc + li], v1 = slab[(lane + 32) * rpc + li];
-        E *dst = recv_row + ((size_t)par * P + cta) * nb;
-        for (int t = 0; t < P; t++) {
-          const unsigned base = map_shared(dst, (unsigned)t);
-          st_cluster_d2(base + (unsigned)(lane * sizeof(E)), v0);
-          st_cluster_d2(base + (unsigned)((lane + 32) * sizeof(E)), v1);
-        }
-      }
-      if (col >= row0 && col < row0 + nrow) {
-        const int li = (int)(col - row0);
-        const E v0 = slab[lane * rpc + li], v1 = slab[(lane + 32) * rpc + li];
-        E *dst = recv_col + (size_t)par * nb;
-        for (int t = 0; t < P; t++) {
-          const unsigned base = map_shared(dst, (unsigned)t);
-          st_cluster_d2(base + (unsigned)(lane * sizeof(E)), v0);
-          st_cluster_d2(base + (unsigned)((lane + 32) * sizeof(E)), v1);
-        }
-      }
-    }
-    cluster_sync();
-    // 2. the winner, read locally; swap
-    if (wid == 0) {
-      const unsigned long long k = lane < P ? c_key[par][lane] : 0ull;
-      const unsigned long long gkey = warp_max_key(k);
-      const int gw = __ffs(__ballot_sync(0xffffffffu, lane < P && k == gkey)) - 1;
-      const int gsrc = gw < 0 ? 0 : gw;
-      // no candidate (every entry of the column NaN): no interchange, failed pivot
-      const bool none = gkey == 0ull;
-      const int gr = none ? (int)col : (int)a.j0 + (int)(0xffffffu - (unsigned)((gkey >> 8) & 0xffffffu));
-      const bool own_p = gr != col && gr >= row0 && gr < row0 + nrow;
-      const bool own_c = col >= row0 && col < row0 + nrow;
-      const E *prow = recv_row + ((size_t)par * P + gsrc) * nb, *crow = recv_col + (size_t)par * nb;
-      for (int j = lane; j < nb; j += 32) {
-        const E pv = none ? crow[j] : prow[j];
-        s_prow_data[j] = pv;
-        if (own_p) slab[j * rpc + (gr - (int)row0)] = crow[j];  // row prow <- old row col
-        if (own_c) slab[j * rpc + (int)(col - row0)] = pv;      // row col  <- pivot row
-        if (j == c) {
-          // 1 / pivot, formed in FP64
-          const double2 pd = to_d2(pv);
-          const double pa = none ? 0.0 : pd.x * pd.x + pd.y * pd.y;
-          s_rp = from_d2<E>(pa != 0.0 ? make_double2(pd.x / pa, -pd.y / pa) : make_double2(0, 0));
-          s_rpc[c] = s_rp;
-          if (cta == 0 && pa == 0.0) atomicCAS(a.info, 0, (int)col + 1);
-        }
-      }
-      if (lane == 0 && cta == 0) a.ipiv[col] = gr;
-    }
-    __syncthreads();
-    // 3. rank-1 update of columns c+1 .. with l = a(i, c) / pivot formed by
-    //    each thread of the row (column c is scaled at the final store)
-    const E rp = s_rp;
-    const bool live = mine && g > col && (rp.x != 0 || rp.y != 0);
-    cv = -1.0;
-    const int own = (c + 1) % S;
-    if (mine && g > col) {
-      const int jst = c + 1 + ((sph - (c + 1)) % S + S) % S;
-      if (live) {
-        const E l = cmul(slab[c * rpc + i], rp);
-        for (int j = jst; j < nb; j += 4 * S) {
-          E x[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            if (j + u * S < nb) x[u] = slab[(j + u * S) * rpc + i];
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            if (j + u * S < nb) {
-              const E uu = s_prow_data[j + u * S];
-              x[u].x -= l.x * uu.x - l.y * uu.y;
-              x[u].y -= l.x * uu.y + l.y * uu.x;
-              slab[(j + u * S) * rpc + i] = x[u];
-            }
-        }
-      }
-      if (sph == own && c + 1 < nb) cv = cabs1(slab[(c + 1) * rpc + i]);
-    }
-  }
-  __syncthreads();
-  for (int idx = tid; idx < nb * rpc; idx += kPanelThreads) {
-    const int c = idx / rpc, ii = idx % rpc;
-    if (ii < nrow) {
-      const E v = slab[idx], rp = s_rpc[c];
-      const bool low = row0 + ii > a.j0 + c && (rp.x != 0 || rp.y != 0);
-      st2(A + (row0 + ii) + (a.j0 + c) * a.lda, low ? cmul(v, rp) : v);
-    }
-  }
-  cluster_sync();  // no CTA leaves while another may still address its shared memory
 }
 
 // The nb row interchanges of a panel (ipiv[j0 .. j0+nb), applied in order)
@@ -1454,49 +1273,20 @@ int panel_ctas(const Ctx *c, int64_t m, int64_t max_rows) {
   return (int)std::min<int64_t>(c->nsm, std::max<int64_t>(P, (m + max_rows - 1) / max_rows));
 }
 
-// One panel (rows j0 .. n of columns j0 .. j0+nb) on P CTAs.
+// Panels of m rows that run on one thread-block cluster (lu_panel.cu).
+template <typename T>
+bool on_cluster(const Ctx *c, int64_t m) {
+  return c->panel_cluster > 0 && c->nb == 64 && m <= panel_reg_rows(c, sizeof(T) == sizeof(float2));
+}
+
+// One panel (rows j0 .. n of columns j0 .. j0+nb) on one cluster, or on P CTAs.
 template <typename T>
 int launch_panel(Ctx *c, T *A, int64_t lda, int64_t n, int64_t j0, int P, int *ipiv, int *info, const LuWork &w,
                  cudaStream_t st = nullptr) {
   if (!st) st = c->stream;
   const int nb = c->nb;
   const int64_t m = n - j0;
-  if (c->panel_cluster > 0 && m <= (int64_t)kClusterRows<T> * c->panel_cluster) {
-    // short panel: one cluster, the smallest power of two with <= kClusterRows rows per CTA
-    int CL = 1;
-    while ((int64_t)kClusterRows<T> * CL < m) CL *= 2;
-    const int rpc = (int)((m + CL - 1) / CL);
-    PanelArgs pa;
-    pa.A = A;
-    pa.lda = lda;
-    pa.n = n;
-    pa.j0 = j0;
-    pa.nb = nb;
-    pa.rpc = rpc;
-    pa.P = CL;
-    pa.ipiv = ipiv;
-    pa.info = info;
-    pa.timeout = w.timeout;
-    pa.spin = wait_polls(c, 0);
-    pa.rec = nullptr;
-    pa.cand_data = nullptr;
-    pa.col_data = nullptr;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(CL);
-    cfg.blockDim = dim3(kPanelThreads);
-    cfg.dynamicSmemBytes = sizeof(typename SlabOf<T>::type) * ((size_t)nb * rpc + (size_t)2 * CL * nb + 2 * nb);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = CL;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    MOM_CUDA(c, cudaLaunchKernelEx(&cfg, panel_cluster_kernel<T>, pa));
-    c->launches++;
-    return MOM_OK;
-  }
+  if (on_cluster<T>(c, m)) return panel_reg(c, A, lda, n, j0, ipiv, info, w.timeout, st);
   const int rpc = (int)((m + P - 1) / P);
   P = (int)((m + rpc - 1) / rpc);
   const size_t smem = sizeof(typename SlabOf<T>::type) * (size_t)nb * rpc;
@@ -1805,7 +1595,7 @@ int lu_enqueue_la(Ctx *c, T *A, const LuWork &w) {
       int P = panel_ctas(c, nc, R);
       const int pcap = c->la_ctas > 0 ? c->la_ctas : 1;
       P = (int)std::max<int64_t>(std::min(P, pcap), (nc + R - 1) / R);
-      if (c->panel_cluster > 0 && nc <= (int64_t)kClusterRows<T> * c->panel_cluster) P = c->panel_cluster;
+      if (on_cluster<T>(c, nc)) P = c->panel_cluster;
       MOM_CUDA(c, cudaEventRecord(c->la_ev[1], sa));
       MOM_CUDA(c, cudaStreamWaitEvent(sb, c->la_ev[1], 0));
       MOM_TRY(factor_block(t0, sb, c->blas2, pmN, pcap));
@@ -2040,40 +1830,10 @@ cudaError_t set_smem(T *fn) {
 
 // Shared-memory opt-in of the LU kernels, once per context (outside any
 // stream capture and off the factorisation's critical path).
-// Largest cluster (power of two <= 16) with one panel CTA per SM that the
-// device can schedule; 0 when clusters are unavailable.
-template <typename T>
-int max_panel_cluster() {
-  if (cudaFuncSetAttribute(panel_cluster_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-    cudaGetLastError();
-    return 8;
-  }
-  for (int cl = kMaxCluster; cl >= 2; cl /= 2) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cl);
-    cfg.blockDim = dim3(kPanelThreads);
-    cfg.dynamicSmemBytes = sizeof(typename SlabOf<T>::type) * (64 * kClusterRows<T> + 2 * cl * 64 + 2 * 64);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cl;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, panel_cluster_kernel<T>, &cfg) == cudaSuccess && nclusters >= 1)
-      return cl;
-    cudaGetLastError();
-  }
-  return 0;
-}
-
 int lu_init_kernels(Ctx *c) {
   MOM_CUDA(c, set_smem(panel_kernel<double2>));
   MOM_CUDA(c, set_smem(panel_kernel<float2>));
-  MOM_CUDA(c, set_smem(panel_cluster_kernel<double2>));
-  MOM_CUDA(c, set_smem(panel_cluster_kernel<float2>));
-  c->panel_cluster = std::min(max_panel_cluster<double2>(), max_panel_cluster<float2>());
+  c->panel_cluster = panel_reg_max_cluster();
   const char *ec = std::getenv("MOM_PANEL_CLUSTER");
   if (ec) c->panel_cluster = std::max(0, std::min(c->panel_cluster, std::atoi(ec)));
   MOM_CUDA(c, set_smem(diag_inv_kernel<double2, 0>));
@@ -2156,7 +1916,7 @@ int tune_panels(Ctx *c, const T *A, Ctx::Tuned &t) {
     int best = c->nsm, last = -1;
     double best_ms = 1e30;
     // heights that run on one cluster have nothing to tune: one timed trial
-    const bool clustered = c->panel_cluster > 0 && m <= (int64_t)kClusterRows<T> * c->panel_cluster;
+    const bool clustered = on_cluster<T>(c, m);
     for (int cand : cands) {
       if (clustered && cand != cands[0]) break;
       const int P0 = (int)std::min<int64_t>(

@@ -218,8 +218,10 @@ struct Ctx {
   // autotuned per (matrix order, precision) at the first factorisation
   // (unless MOM_AUTOTUNE=0: one CTA per SM); MOM_PANEL_CTAS fixes a cap.
   int panel_cap_env = 0;
-  // Short panels run on one thread-block cluster of up to panel_cluster CTAs
-  // (the largest the device schedules; MOM_PANEL_CLUSTER caps it, 0 = off).
+  // Panels run on one thread-block cluster of up to panel_cluster CTAs (the
+  // largest the device schedules; MOM_PANEL_CLUSTER caps it, 0 = off), those
+  // too tall for it (over 32,768 rows in FP32, 16,384 in FP64 with 16 CTAs) on
+  // CTAs that exchange through global memory.
   int panel_cluster = 0;
   int outer_panels = 4;  // panels per outer block of the LU (MOM_LU_OUTER): trailing GEMMs have K = 64 * this
   int small_tc = 0;      // mixed path: K = 64 updates on the tensor cores too (MOM_SMALL_TC=1), else library FP32 GEMM
@@ -370,6 +372,15 @@ int matvec_acc(Ctx *c, const double2 *X, int nrhs, double2 *Y, double sign);
 int shg_solve(Ctx *c, double omega, const double *ri, const double *shri, const mom_nls *nls, int precision,
               double tol, int maxit, int *iters);
 void free_shg(DomDev &D);
+
+// lu_panel.cu: the 64-column panel at column j0 (rows j0 .. n) on one
+// thread-block cluster, for n - j0 <= panel_reg_rows().
+int panel_reg_max_cluster();
+int64_t panel_reg_rows(const Ctx *c, bool f32);
+int panel_reg(Ctx *c, float2 *A, int64_t lda, int64_t n, int64_t j0, int *ipiv, int *info, int *timeout,
+              cudaStream_t st);
+int panel_reg(Ctx *c, double2 *A, int64_t lda, int64_t n, int64_t j0, int *ipiv, int *info, int *timeout,
+              cudaStream_t st);
 
 // tc_gemm.cu: C -= L U (complex FP32) on the tensor cores, 3xTF32
 int tc_cgemm_update(Ctx *c, float2 *C, int64_t ldc, const float2 *L, int64_t ldl, const float2 *U, int64_t ldu, int m,
