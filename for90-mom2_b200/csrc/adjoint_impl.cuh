@@ -136,10 +136,14 @@ __device__ __forceinline__ void cross3(const S *a, const S *b, S *r) {
 }
 
 // Geometry of face f with the derivative seeded on coordinate scoord of node
-// snode (snode < 0: no geometric seed).
-template <int NQ>
-__device__ void face_build(const AdjTopo &t, int f, int snode, int scoord, FaceAll<Dual, NQ> &o) {
-  auto node = [&](int id, int k) { return Dual(t.nodes[3 * id + k], (id == snode && k == scoord) ? 1.0 : 0.0); };
+// snode (snode < 0: no geometric seed): vertices, edge vectors and normals,
+// area, centroid, RWG lengths and free vertices.
+__device__ __forceinline__ Dual seeded_node(const AdjTopo &t, int id, int k, int snode, int scoord) {
+  return Dual(t.nodes[3 * id + k], (id == snode && k == scoord) ? 1.0 : 0.0);
+}
+__device__ void face_geo(const AdjTopo &t, int f, int snode, int scoord, FaceGeoT<Dual> &g, Dual &area, Dual *cp,
+                         Dual *sl, Dual (*bn)[3]) {
+  auto node = [&](int id, int k) { return seeded_node(t, id, k, snode, scoord); };
   Dual p[3][3];
 #pragma unroll
   for (int v = 0; v < 3; v++)
@@ -157,49 +161,57 @@ __device__ void face_build(const AdjTopo &t, int f, int snode, int scoord, FaceA
   cross3(a, cc, b);
   const Dual nb = norm3(b);
 #pragma unroll
-  for (int i = 0; i < 3; i++) o.g.n[i] = b[i] / nb;
+  for (int i = 0; i < 3; i++) g.n[i] = b[i] / nb;
   const Dual l21 = norm3(p21), l32 = norm3(p32), l13 = norm3(p13);
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    o.g.s[0][i] = p21[i] / l21;
-    o.g.s[1][i] = p32[i] / l32;
-    o.g.s[2][i] = p13[i] / l13;
+    g.s[0][i] = p21[i] / l21;
+    g.s[1][i] = p32[i] / l32;
+    g.s[2][i] = p13[i] / l13;
   }
 #pragma unroll
   for (int e = 0; e < 3; e++) {
-    cross3(o.g.s[e], o.g.n, o.g.mm[e]);
-    const Dual l = norm3(o.g.mm[e]);
+    cross3(g.s[e], g.n, g.mm[e]);
+    const Dual l = norm3(g.mm[e]);
 #pragma unroll
-    for (int i = 0; i < 3; i++) o.g.mm[e][i] = o.g.mm[e][i] / l;
+    for (int i = 0; i < 3; i++) g.mm[e][i] = g.mm[e][i] / l;
   }
   Dual mp13[3] = {-p13[0], -p13[1], -p13[2]}, cr[3];
   cross3(mp13, p32, cr);
-  o.area = 0.5 * norm3(cr);
+  area = 0.5 * norm3(cr);
 #pragma unroll
-  for (int i = 0; i < 3; i++) o.cp[i] = (p[0][i] + p[1][i] + p[2][i]) / 3.0;
+  for (int i = 0; i < 3; i++) cp[i] = (p[0][i] + p[1][i] + p[2][i]) / 3.0;
 #pragma unroll
   for (int v = 0; v < 3; v++)
 #pragma unroll
-    for (int i = 0; i < 3; i++) o.g.v[v][i] = p[v][i];
-  for (int q = 0; q < NQ; q++)
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      o.qa[q][i] = c_qn[q][2] * p[0][i] + c_qn[q][0] * p[1][i] + c_qn[q][1] * p[2][i];
-      o.qr[q][i] = o.qa[q][i] - o.cp[i];
-    }
+    for (int i = 0; i < 3; i++) g.v[v][i] = p[v][i];
 #pragma unroll
   for (int e = 0; e < 3; e++) {
-    const int ea = t.fea[3 * f + e], eb = t.feb[3 * f + e], bn = t.fbn[3 * f + e];
+    const int ea = t.fea[3 * f + e], eb = t.feb[3 * f + e];
     Dual dl[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) dl[i] = node(ea, i) - node(eb, i);
-    o.sl[e] = t.fsign[3 * f + e] * norm3(dl);
+    sl[e] = t.fsign[3 * f + e] * norm3(dl);
+#pragma unroll
+    for (int i = 0; i < 3; i++) bn[e][i] = node(t.fbn[3 * f + e], i);
+  }
+}
+
+// The same with the quadrature points (absolute and from the centroid) and
+// the free vertices from the centroid.
+template <int NQ>
+__device__ void face_build(const AdjTopo &t, int f, int snode, int scoord, FaceAll<Dual, NQ> &o) {
+  face_geo(t, f, snode, scoord, o.g, o.area, o.cp, o.sl, o.bn);
+  for (int q = 0; q < NQ; q++)
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-      o.bn[e][i] = node(bn, i);
-      o.mu[e][i] = o.bn[e][i] - o.cp[i];
+      o.qa[q][i] = c_qn[q][2] * o.g.v[0][i] + c_qn[q][0] * o.g.v[1][i] + c_qn[q][1] * o.g.v[2][i];
+      o.qr[q][i] = o.qa[q][i] - o.cp[i];
     }
-  }
+#pragma unroll
+  for (int e = 0; e < 3; e++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) o.mu[e][i] = o.bn[e][i] - o.cp[i];
 }
 
 // blocks_from_moments in the scalar type S, with the test face's geometry in
@@ -304,38 +316,9 @@ struct AdjPairArgs {
   const double2 *lam, *xv;  // [R][n]
   const double2 *W;         // [n][n] column-major, W(r, c) = sum_o lambda_o[r] x_o[c]
   double *part;    // [gridDim.y][gridDim.x][max(R,1)][2]
-  // the assembly's FP64 geometry (partner faces that carry no derivative)
-  const double *qrel, *cp, *mu, *sl;
 };
 
 __device__ __forceinline__ Cd cdm(Cd a, double2 b) { return {a.re * b.x - a.im * b.y, a.re * b.y + a.im * b.x}; }
-
-// Adds the derivative blocks Sb, Kb of the pair (test m, source n) contracted
-// with the objectives into acc (the loop of pair_contract).
-__device__ __forceinline__ void contract_blocks(const AdjPairArgs &a, int m, int n, const Cx<Dual> *Sb,
-                                                const Cx<Dual> *Kb, Cd *acc) {
-  const int64_t N = a.t.N, ld = a.n;
-#pragma unroll 1
-  for (int p = 0; p < 3; p++) {
-    const int64_t r = a.t.hpar[3 * m + p];
-#pragma unroll 1
-    for (int q = 0; q < 3; q++) {
-      const int64_t cI = a.t.hpar[3 * n + q];
-      const Cd dS = dpart(Sb[3 * p + q]), dZ = dpart(cxm(a.Zsi, Sb[3 * p + q])), dK = dpart(Kb[3 * p + q]);
-      for (int o = 0; o < a.R; o++) {
-        const double2 *l = a.lam + (size_t)o * ld, *x = a.xv + (size_t)o * ld;
-        const double2 lr = l[r], lrN = l[r + N], xc = x[cI], xcN = x[cI + N];
-        const double2 jj = make_double2(lr.x * xc.x - lr.y * xc.y, lr.x * xc.y + lr.y * xc.x);
-        const double2 mm = make_double2(lrN.x * xcN.x - lrN.y * xcN.y, lrN.x * xcN.y + lrN.y * xcN.x);
-        const double2 mj = make_double2(lrN.x * xc.x - lrN.y * xc.y, lrN.x * xc.y + lrN.y * xc.x);
-        const double2 jm = make_double2(lr.x * xcN.x - lr.y * xcN.y, lr.x * xcN.y + lr.y * xcN.x);
-        const Cd t1 = cdm(dS, jj), t2 = cdm(dZ, mm), t3 = cdm(dK, make_double2(mj.x - jm.x, mj.y - jm.y));
-        acc[o].re += t1.re + t2.re + t3.re;
-        acc[o].im += t1.im + t2.im + t3.im;
-      }
-    }
-  }
-}
 
 // Adds d/dp (lambda_o^T A x_o) of pair (m, n) into acc[o] for the four
 // PMCHWT blocks [JJ] S, [MM] Zsi S, [MJ] K, [JM] -K (sysmat.f90:70-99).
@@ -424,96 +407,6 @@ __global__ void __launch_bounds__(kAdjThreads) adj_pair_kernel(AdjPairArgs a) {
     }
     __syncthreads();
   }
-}
-
-// ---- vertex mode with one dual face ---------------------------------------
-//
-// Item (vertex v, incident face f, axis): only the faces that touch v carry a
-// derivative.  The CTA builds f's dual record once in shared memory; a
-// partner x that does not touch v is read as FP64 from the assembly's arrays
-// and the far pairs (f, x) and (x, f) run with one dual and one plain face.
-// Partners that touch v, and near pairs (closed-form singular terms), take
-// the all-dual evaluation of adj_pair_kernel.  Same pairs, same contraction
-// and the same deterministic block sums.
-
-template <int NQ>
-__device__ __noinline__ void vertex_pairs_dual(const AdjPairArgs &a, int f, int x, int snode, int scoord,
-                                               const FaceAll<Dual, NQ> &ff, bool touches, Cd *acc) {
-  FaceAll<Dual, NQ> fx;
-  face_build<NQ>(a.t, x, snode, scoord, fx);
-  pair_contract<NQ>(a, f, x, ff, fx, acc);
-  if (!touches) pair_contract<NQ>(a, x, f, fx, ff, acc);
-}
-
-template <int NQ>
-__global__ void __launch_bounds__(kAdjThreads) adj_vertex_kernel(AdjPairArgs a) {
-  // the seeded face's dual record, built once per CTA (raw storage: Dual has
-  // a constructor, which a __shared__ object may not run)
-  __shared__ __align__(16) unsigned char ff_raw[sizeof(FaceAll<Dual, NQ>)];
-  FaceAll<Dual, NQ> &ff = *reinterpret_cast<FaceAll<Dual, NQ> *>(ff_raw);
-  const int item = blockIdx.y;
-  const int f = a.inc_face[item / 3], snode = a.inc_node[item / 3], scoord = item % 3;
-  if (threadIdx.x == 0) face_build<NQ>(a.t, f, snode, scoord, ff);
-  __syncthreads();
-  const int x = blockIdx.x * kAdjThreads + threadIdx.x;
-  Cd acc[kAdjMaxObj];
-#pragma unroll
-  for (int o = 0; o < kAdjMaxObj; o++) acc[o] = {0.0, 0.0};
-  if (x < a.t.F) {
-    const bool touches = a.t.fnode[3 * x] == snode || a.t.fnode[3 * x + 1] == snode || a.t.fnode[3 * x + 2] == snode;
-    const int64_t b1 = (int64_t)f * a.t.F + x, b2 = (int64_t)x * a.t.F + f;
-    const bool near = ((a.t.near_bits[b1 >> 5] >> (b1 & 31)) & 1u) || ((a.t.near_bits[b2 >> 5] >> (b2 & 31)) & 1u);
-    if (touches || near) {
-      vertex_pairs_dual<NQ>(a, f, x, snode, scoord, ff, touches, acc);
-    } else {
-      const double *qx = a.qrel + (size_t)x * NQ * 3;
-      const double *mux = a.mu + 9 * (size_t)x, *slx = a.sl + 3 * (size_t)x;
-      const Cx<Dual> fD = {a.c1.re * (kOofpi / 4.0), a.c1.im * (kOofpi / 4.0)};
-      const Cx<Dual> fH = {a.c2.re * kOofpi, a.c2.im * kOofpi};
-      Dual d[3];
-      Cx<Dual> Sb[9], Kb[9];
-      Moments<Dual> M;
-      // (f, x): dual test face, plain source
-#pragma unroll
-      for (int i = 0; i < 3; i++) d[i] = ff.cp[i] - a.cp[3 * x + i];
-      pair_moments<Dual, NQ, false, false, Dual, double, Dual>(&ff.qr[0][0], qx, 1, d, a.kr, a.ki, M);
-      blocks_generic<Dual, Dual, double, Dual>(M, ff.mu, reinterpret_cast<const double(*)[3]>(mux), ff.sl, slx, d, fD,
-                                               fH, kOofpi / 4.0, false, Sb, Kb);
-      contract_blocks(a, f, x, Sb, Kb, acc);
-      // (x, f): plain test face, dual source; the same point pairs, so its
-      // moments are those of (f, x) with the faces' roles exchanged
-#pragma unroll
-      for (int i = 0; i < 3; i++) d[i] = -d[i];
-      exchange_roles(M);
-      blocks_generic<Dual, double, Dual, Dual>(M, reinterpret_cast<const double(*)[3]>(mux), ff.mu, slx, ff.sl, d, fD,
-                                               fH, kOofpi / 4.0, false, Sb, Kb);
-      contract_blocks(a, x, f, Sb, Kb, acc);
-    }
-  }
-  __shared__ double red[kAdjThreads][2];
-  for (int o = 0; o < a.R; o++) {
-    red[threadIdx.x][0] = acc[o].re;
-    red[threadIdx.x][1] = acc[o].im;
-    __syncthreads();
-    for (int w = kAdjThreads / 2; w > 0; w >>= 1) {
-      if (threadIdx.x < w) {
-        red[threadIdx.x][0] += red[threadIdx.x + w][0];
-        red[threadIdx.x][1] += red[threadIdx.x + w][1];
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      double *out = a.part + (((size_t)blockIdx.y * gridDim.x + blockIdx.x) * a.R + o) * 2;
-      out[0] = red[0][0];
-      out[1] = red[0][1];
-    }
-    __syncthreads();
-  }
-}
-
-template <int NQ>
-void launch_adj_vertex(const dim3 &grid, cudaStream_t s, const AdjPairArgs &a) {
-  adj_vertex_kernel<NQ><<<grid, kAdjThreads, 0, s>>>(a);
 }
 
 // ---- permittivity mode on plain geometry ---------------------------------

@@ -453,7 +453,7 @@ int mom_gpu_create(int32_t device, mom_ctx **out) {
   const char *ae = std::getenv("MOM_ADJ_EPS_PLAIN");
   if (ae) c->adj_eps_plain = std::atoi(ae) != 0;
   const char *av = std::getenv("MOM_ADJ_VERTEX_PLAIN");
-  if (av) c->adj_vertex_plain = std::atoi(av) != 0;
+  if (av) c->adj_vertex_reverse = std::atoi(av) != 0;
   const char *ft = std::getenv("MOM_FUSED_TRSM");
   if (ft) c->fused_trsm = std::max(0, std::min(2, std::atoi(ft)));
   *out = c;

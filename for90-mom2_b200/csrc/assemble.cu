@@ -1280,6 +1280,7 @@ int load_matrix(Ctx *c, const double *A_host, int64_t ldh, int precision) {
 
 #include "adjoint_impl.cuh"
 #include "nfields_impl.cuh"
+#include "adjoint_nodes_impl.cuh"
 
 namespace {
 
@@ -1395,10 +1396,6 @@ int adjoint_eps(Ctx *c, double omega, const double *ri, int d, int R, const doub
   medium_duals(omega, ri, d, true, a);
   a.mode = 0;
   a.inc_node = a.inc_face = nullptr;
-  a.qrel = D.qrel;
-  a.cp = D.cp;
-  a.mu = D.mu;
-  a.sl = D.sl;
   a.R = R;
   a.lam = lam;
   a.xv = xv;
@@ -1489,28 +1486,23 @@ int adjoint_nodes(Ctx *c, double omega, const double *ri, int R, const double2 *
     a.lam = lam;
     a.xv = xv;
     a.W = nullptr;
-    a.qrel = D.qrel;
-    a.cp = D.cp;
-    a.mu = D.mu;
-    a.sl = D.sl;
+    if (c->adj_vertex_reverse) {
+      // objectives of one source share x: two at a time
+      for (int o = 0, no = 0; o < R; o += no) {
+        no = o + 1 < R && obj_src[o] == obj_src[o + 1] ? 2 : 1;
+        std::vector<double> h;
+        MOM_TRY(rev_nodes(c, d, a, o, no, h));
+        for (int k = 0; k < no; k++)
+          for (int e = 0; e < 9 * D.F; e++)
+            out[((size_t)(o + k) * total + off[d] + D.h_fnode[e / 3]) * 3 + e % 3] -= h[(size_t)k * 9 * D.F + e];
+      }
+      continue;
+    }
     const dim3 grid((D.F + kAdjThreads - 1) / kAdjThreads, 3 * D.ninc);
     const size_t nvals = (size_t)grid.x * grid.y * R * 2;
     MOM_TRY(ensure_buffer(c, &c->adj_part, &c->adj_part_bytes, sizeof(double) * nvals));
     a.part = (double *)c->adj_part;
-    if (c->adj_vertex_plain) {
-      switch (c->nq) {
-        case 1: launch_adj_vertex<1>(grid, c->stream, a); break;
-        case 3: launch_adj_vertex<3>(grid, c->stream, a); break;
-        case 4: launch_adj_vertex<4>(grid, c->stream, a); break;
-        case 7: launch_adj_vertex<7>(grid, c->stream, a); break;
-        case 13: launch_adj_vertex<13>(grid, c->stream, a); break;
-        default: return fail(c, MOM_ERR_ARG, "unsupported number of quadrature points");
-      }
-      c->launches++;
-      MOM_CUDA(c, cudaGetLastError());
-    } else {
-      MOM_TRY(adj_launch_pair(c, grid, a));
-    }
+    MOM_TRY(adj_launch_pair(c, grid, a));
     std::vector<double> h(nvals);
     std::vector<int> inode(D.ninc);
     MOM_CUDA(c, cudaMemcpyAsync(h.data(), a.part, sizeof(double) * nvals, cudaMemcpyDeviceToHost, c->stream));

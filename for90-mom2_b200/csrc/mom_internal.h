@@ -234,9 +234,9 @@ struct Ctx {
   // Permittivity gradients by adj_eps_kernel (FP64 geometry, dual numbers in
   // k only); MOM_ADJ_EPS_PLAIN=0 selects the all-dual adj_pair_kernel.
   int adj_eps_plain = 1;
-  // Vertex gradients by adj_vertex_kernel (the seeded face dual in shared
-  // memory, plain partners); MOM_ADJ_VERTEX_PLAIN=0 selects adj_pair_kernel.
-  int adj_vertex_plain = 1;
+  // Vertex gradients in reverse mode (adjoint_nodes_impl.cuh);
+  // MOM_ADJ_VERTEX_PLAIN=0 selects the forward-mode adj_pair_kernel.
+  int adj_vertex_reverse = 1;
   bool autotune = true;
   struct Tuned {
     int64_t n;
