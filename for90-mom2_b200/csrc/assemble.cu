@@ -51,7 +51,8 @@ __constant__ double c_qn[kMaxQ][3];
 namespace {
 
 constexpr int kPairThreads = 128;
-constexpr int kTestPerCta = 8;
+constexpr int kTestPerCta = 8;  // most test faces of one far-pair CTA
+constexpr int kPairWaves = 4;
 constexpr double kOofpi = 1.0 / (4.0 * kPi);  // green.f90:20-21
 
 template <typename T>
@@ -302,6 +303,7 @@ struct PairArgs {
   const double *tqrel, *tcp, *tmu;  // test faces (mapped by J^T for a group action g != identity)
   int ident;           // identity action: the self pair m == n has no K term
   int sym;             // identity action: each unordered pair once, both blocks written
+  int tests;           // test faces per CTA
   double inv_unit;     // 1/L0
   double kr, ki;       // k * L0
   Cd fD, fH;
@@ -309,7 +311,7 @@ struct PairArgs {
   double2 *blk;        // [F source][F test][18]
 };
 
-// One thread per source face n; the CTA walks kTestPerCta test faces.  In the
+// One thread per source face n; the CTA walks a.tests test faces.  In the
 // FP32 kernel the source face's FP64 geometry (centroid, edge vectors, edge
 // lengths) waits in shared memory while the point-pair loop runs, so it holds
 // no registers there (the FP64 kernel's point sources already fill the 48 KB
@@ -349,10 +351,10 @@ __global__ void __launch_bounds__(kPairThreads, MINB) pair_kernel(PairArgs a) {
       else r_ngeo[i] = g[i];
     }
   }
-  const int m0 = blockIdx.y * kTestPerCta;
+  const int m0 = blockIdx.y * a.tests;
   // with sym, a CTA whose test faces all come after its source faces has no work
   if (a.sym && (int64_t)m0 > (int64_t)blockIdx.x * kPairThreads + kPairThreads - 1) return;
-  for (int mi = 0; mi < kTestPerCta; mi++) {
+  for (int mi = 0; mi < a.tests; mi++) {
     const int m = m0 + mi;
     if (m >= a.F) break;
     __syncthreads();
@@ -1109,7 +1111,17 @@ int domain_blocks(Ctx *c, int d, int g, double omega, const double *ri, int prec
       pa.fH = {c2.re * L0 * kOofpi, c2.im * L0 * kOofpi};
       pa.fK = L0 * L0 * kOofpi / 4.0;
       pa.blk = blk;
-      dim3 grid((D.F + kPairThreads - 1) / kPairThreads, (D.F + kTestPerCta - 1) / kTestPerCta);
+      // Test faces per CTA: a CTA's test faces are a serial loop (57 us each
+      // in FP64), so few enough that the CTAs with work fill the resident
+      // slots (3 per SM) kPairWaves times; many enough, up to kTestPerCta,
+      // that the source faces are staged once for several.  Two domains of 80
+      // faces in FP64 took 0.91 ms with 8 test faces per CTA, 0.13 ms with one;
+      // from about 1,280 faces (2.8 ms) the choice makes no difference.
+      const int64_t cols = (D.F + kPairThreads - 1) / kPairThreads;
+      pa.tests = kTestPerCta;
+      while (pa.tests > 1 && cols * ((D.F + pa.tests - 1) / pa.tests) < (pa.sym ? 2 : 1) * kPairWaves * 3 * c->nsm)
+        pa.tests /= 2;
+      dim3 grid((unsigned)cols, (D.F + pa.tests - 1) / pa.tests);
       {
         ProfScope ps(c, kProfPair);
         if (precision == MOM_PREC_MIXED) {
