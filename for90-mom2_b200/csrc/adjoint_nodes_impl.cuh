@@ -1,5 +1,6 @@
 // d(lambda^T A x) / d(vertex coordinates) in reverse mode (no counterpart in
-// the reference).  Included by assemble.cu after adjoint_impl.cuh.
+// the reference).  Included by assemble.cu after adjoint_impl.cuh and
+// nfields_impl.cuh (complex vectors, the faces' affine currents).
 //
 // With the currents of a face written as affine fields, t(r) = a r + b times
 // 1 / area for lambda and for x (J and M), the quadrature of every face pair is
@@ -45,65 +46,9 @@ struct RevArgs {
   double *part;            // [split][no][F NQ][kRevVals]
 };
 
-// The affine currents of a face about its centroid: a = sum_p v_p sl_p / 2,
-// b = -sum_p v_p sl_p mu_p / 2, for the J and M halves of vector v.
-__global__ void rev_coef_kernel(int F, int N, const int *hpar, const double *sl, const double *mu, const double2 *v,
-                                double2 *coef) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= F) return;
-  for (int h = 0; h < 2; h++) {
-    Cd a = {0, 0}, b[3] = {{0, 0}, {0, 0}, {0, 0}};
-    for (int p = 0; p < 3; p++) {
-      const double2 c = v[hpar[3 * f + p] + (h ? N : 0)];
-      const double s = 0.5 * sl[3 * f + p];
-      a.re += s * c.x;
-      a.im += s * c.y;
-      for (int i = 0; i < 3; i++) {
-        const double t = s * mu[9 * (size_t)f + 3 * p + i];
-        b[i].re -= t * c.x;
-        b[i].im -= t * c.y;
-      }
-    }
-    double2 *o = coef + 8 * (size_t)f + 4 * h;
-    o[0] = make_double2(a.re, a.im);
-    for (int i = 0; i < 3; i++) o[1 + i] = make_double2(b[i].re, b[i].im);
-  }
-}
-
-__device__ __forceinline__ Cd cdad(Cd a, Cd b) { return {a.re + b.re, a.im + b.im}; }
-__device__ __forceinline__ Cd cdsb(Cd a, Cd b) { return {a.re - b.re, a.im - b.im}; }
-__device__ __forceinline__ Cd cds(Cd a, double s) { return {a.re * s, a.im * s}; }
-// acc + a b, acc - a b
-__device__ __forceinline__ Cd cfma(Cd a, Cd b, Cd acc) {
-  return {fma(a.re, b.re, fma(-a.im, b.im, acc.re)), fma(a.re, b.im, fma(a.im, b.re, acc.im))};
-}
-__device__ __forceinline__ Cd cfms(Cd a, Cd b, Cd acc) {
-  return {fma(-a.re, b.re, fma(a.im, b.im, acc.re)), fma(-a.re, b.im, fma(-a.im, b.re, acc.im))};
-}
-struct Cv {
-  Cd x, y, z;
-};
-__device__ __forceinline__ Cv cvcross(const Cv &a, const Cv &b) {
-  const Cd o = {0, 0};
-  return {cfms(a.z, b.y, cfma(a.y, b.z, o)), cfms(a.x, b.z, cfma(a.z, b.x, o)), cfms(a.y, b.x, cfma(a.x, b.y, o))};
-}
-__device__ __forceinline__ Cv cvadd(const Cv &a, const Cv &b) { return {cdad(a.x, b.x), cdad(a.y, b.y), cdad(a.z, b.z)}; }
-__device__ __forceinline__ Cv cvsub(const Cv &a, const Cv &b) { return {cdsb(a.x, b.x), cdsb(a.y, b.y), cdsb(a.z, b.z)}; }
-__device__ __forceinline__ Cv cvscale(Cd s, const Cv &a) { return {cmul(s, a.x), cmul(s, a.y), cmul(s, a.z)}; }
 __device__ __forceinline__ Cd cvdot(const Cv &a, const Cv &b, Cd acc) {
   return cfma(a.z, b.z, cfma(a.y, b.y, cfma(a.x, b.x, acc)));
 }
-// a D + b
-__device__ __forceinline__ Cv affine(Cd a, const double *D, const Cv &b) {
-  return {{fma(a.re, D[0], b.x.re), fma(a.im, D[0], b.x.im)},
-          {fma(a.re, D[1], b.y.re), fma(a.im, D[1], b.y.im)},
-          {fma(a.re, D[2], b.z.re), fma(a.im, D[2], b.z.im)}};
-}
-__device__ __forceinline__ Cd ld_c(const double2 *p) {
-  const double2 v = *p;
-  return {v.x, v.y};
-}
-__device__ __forceinline__ Cv ld_v(const double2 *p) { return {ld_c(p), ld_c(p + 1), ld_c(p + 2)}; }
 // symmetric matrix (xx, yy, zz, xy, xz, yz) times a vector
 __device__ __forceinline__ Cv symv(const Cd *s, const Cv &v) {
   const Cd o = {0, 0};
@@ -224,12 +169,12 @@ __global__ void __launch_bounds__(kRevThreads) rev_field_kernel(RevArgs a) {
           g = near ? Cd{-a.ki, a.kr} : Cd{0, 0};
           p = q = Cd{0, 0};
         }
-        g = cds(g, wj);
-        p = cds(p, wj);
-        q = cds(q, wj);
+        g = csc(g, wj);
+        p = csc(p, wj);
+        q = csc(q, wj);
         const double DD[6] = {D[0] * D[0], D[1] * D[1], D[2] * D[2], D[0] * D[1], D[0] * D[2], D[1] * D[2]};
-        g0 = cdad(g0, g);
-        p0 = cdad(p0, p);
+        g0 = cadd(g0, g);
+        p0 = cadd(p0, p);
 #pragma unroll
         for (int k = 0; k < 3; k++) {
           g1[k] = {fma(g.re, D[k], g1[k].re), fma(g.im, D[k], g1[k].im)};
@@ -261,8 +206,8 @@ __global__ void __launch_bounds__(kRevThreads) rev_field_kernel(RevArgs a) {
         add_v(s, 0, rj);
         add_v(s, 3, rm);
         const Cd c2g = cmul(a.c2, g0);
-        add_c(s, 6, cds(cmul(c2g, aJ), 2.0));
-        add_c(s, 7, cds(cmul(cmul(c2g, a.Z), aM), 2.0));
+        add_c(s, 6, csc(cmul(c2g, aJ), 2.0));
+        add_c(s, 7, csc(cmul(cmul(c2g, a.Z), aM), 2.0));
       };
       fields(NO, aXJ, aXM, XJ, XM, 1.0);  // dF / dT
       const Cv OXJ = own_v(NO, 0), OXM = own_v(NO, 3);
@@ -277,7 +222,7 @@ __global__ void __launch_bounds__(kRevThreads) rev_field_kernel(RevArgs a) {
         const Cd z0 = {0, 0};
         const Cd aj = cvdot(OXJ, TJ, cvdot(OTJ, XJ, z0)), am = cvdot(OXM, TM, cvdot(OTM, XM, z0));
         const Cd dj = cfma(odXJ, aTJ, cmul(own_c(o, 6), aXJ)), dm = cfma(odXM, aTM, cmul(own_c(o, 7), aXM));
-        const Cd alpha = cfma(a.c1, cfma(a.Z, am, aj), cds(cmul(a.c2, cfma(a.Z, dm, dj)), 2.0));
+        const Cd alpha = cfma(a.c1, cfma(a.Z, am, aj), csc(cmul(a.c2, cfma(a.Z, dm, dj)), 2.0));
         const Cv gj = cvadd(cvscale(aXJ, OTJ), cvscale(aTJ, OXJ)), gm = cvadd(cvscale(aXM, OTM), cvscale(aTM, OXM));
         const Cv gamma = cvscale(a.c1, cvadd(gj, cvscale(a.Z, gm)));
         Cv fo = cvsub(symv(p2, gamma), cvscale(alpha, P1));
@@ -391,16 +336,16 @@ __global__ void __launch_bounds__(64) rev_static_field_kernel(RevStaticArgs a) {
       const Cd z = h ? a.Z : Cd{1.0, 0.0}, c1 = cmul(a.c1, z), c2 = cmul(a.c2, z);
       for (int k = 0; k < 3; k++) {
         const Cd l = {f4 * ps.mL1[k] - f8.re * ps.mL3[k] / 3.0, -f8.im * ps.mL3[k] / 3.0};
-        const Cd Y = cds(cfma(al, l, cmul(y0, vv[k])), iA);
+        const Cd Y = csc(cfma(al, l, cmul(y0, vv[k])), iA);
         F[h][k] = cfma(c1, Y, F[h][k]);
       }
-      F[h][3] = cfma(c2, cds(cmul(al, y0), 2.0 * iA), F[h][3]);
+      F[h][3] = cfma(c2, csc(cmul(al, y0), 2.0 * iA), F[h][3]);
       K[h] = cvcross(Hn, affine(al, D0, b));
     }
     if (n != m)
       for (int k = 0; k < 3; k++) {
-        F[0][k] = cdsb(F[0][k], cds((&K[1].x)[k], iA));
-        F[1][k] = cdad(F[1][k], cds((&K[0].x)[k], iA));
+        F[0][k] = csub(F[0][k], csc((&K[1].x)[k], iA));
+        F[1][k] = cadd(F[1][k], csc((&K[0].x)[k], iA));
       }
   }
   const double *qr = a.qrel + (size_t)i * 3;
@@ -650,11 +595,10 @@ int rev_nodes(Ctx *c, int d, const AdjPairArgs &m, int o0, int no, std::vector<d
   char *b = (char *)c->adj_part;
   double2 *coef = (double2 *)b;
   const double2 *lam = m.lam + (size_t)o0 * m.n, *xv = m.xv + (size_t)o0 * m.n;
-  for (int v = 0; v <= no; v++) {
-    rev_coef_kernel<<<(F + 127) / 128, 128, 0, c->stream>>>(F, c->N, D.hpar, D.sl, D.mu,
-                                                             v < no ? lam + (size_t)v * m.n : xv, coef + 8 * (size_t)F * v);
-    c->launches++;
-  }
+  const dim3 cg((F + 127) / 128, no);
+  face_current_kernel<<<cg, 128, 0, c->stream>>>(F, c->N, D.hpar, D.sl, D.mu, lam, m.n, coef);
+  face_current_kernel<<<cg.x, 128, 0, c->stream>>>(F, c->N, D.hpar, D.sl, D.mu, xv, m.n, coef + 8 * (size_t)F * no);
+  c->launches += 2;
   RevArgs ra;
   ra.F = F;
   ra.no = no;

@@ -256,7 +256,8 @@ struct Ctx {
   double tc_flops = 0;     // FLOP executed by the tensor-core LU updates since creation
 
   // Adjoint buffers: objective gradients, adjoint currents, forward currents,
-  // block partial sums, and the dense objective matrix of the mean gradient.
+  // partial sums (adj_part; also of the near and far fields, so that a field
+  // map never moves the workspace that the captured LU works in), and the dense objective matrix of the mean gradient.
   void *adj = nullptr;
   size_t adj_bytes = 0;
   void *adj_part = nullptr;

@@ -4,196 +4,261 @@
 // kernel shares the closed-form static integrals (point_static) and the
 // quadrature weights (c_qw) of the assembly (inside namespace mom).
 //
-// For point r and source face f with RWG functions f_q = c_q (r' - p_q)
-// (c_q = s_q l_q / (2 A_f), div f_q = s_q l_q / A_f) the kernel needs
+// For point r and source face f with the RWG functions f_q = c_q (r' - p_q)
+// (c_q = s_q l_q / (2 A_f), div f_q = s_q l_q / A_f) the fields need
 //   K2_q = int G f_q,  K3_q = int grad'G div'f_q,  K4_q = int grad'G x f_q
-// (intK2, intK3, intK4 of srcint.f90 with no test face).  With
-// grad'G = (r - r') phi / (4 pi), phi = e^{ikR} (1/R^3 - ik/R^2), one
-// quadrature pass over the face gives the sums
-//   SG = sum w g,  SGr = sum w g r',  SPd = sum w phi (r - r')
-// and then  K2_q = c_q (SGr - p_q SG),  K3_q = div_q SPd,
-// K4_q = -c_q (r - p_q) x SPd   (all times A_f / (4 pi); SPd = sum w phi (r - r'),
-// using (r - r') x r' = -(r x (r - r'))).  Within three
-// average edge lengths of the face centroid the smoothed kernels are used and
-// the closed-form parts (1/(4 pi)) X_m1 - (k^2/(8 pi)) X_1 are added, as in
-// the reference.  The currents then give (c1 = i w mu0, c2 = 1/(i w eps0 n^2))
+// (intK2, intK3, intK4 of srcint.f90 with no test face), and with
+// c1 = i w mu0, c2 = 1/(i w eps0 n^2)
 //   E += x_J (c1 K2 + c2 K3) + x_M K4,   H += x_M (K2/c2 + K3/c1) - x_J K4.
+// The coefficients x go in first: the face's current is the affine field
+// (a r' + b) / A, so with D = r - r', grad'G = D phi / (4 pi),
+// phi = e^{ikR} (1/R^3 - ik/R^2), the sums
+//   g0 = sum w g,  g1 = sum w g D,  p1 = sum w phi D
+// give every source's sum_q x_q K2_q = (g0 X^ - a g1) A-free, K3 = 2 a p1 and
+// K4 = -X^ x p1 (all over 4 pi), X^ = a D0 + b about the centroid being the
+// current extended to r (D x D = 0).  Within three average edge lengths of the
+// face centroid the smoothed kernels are used and the closed-form parts
+// (1/(4 pi)) X_m1 - (k^2/(8 pi)) X_1 are added, as in the reference.
 
 namespace {
 
-constexpr int kNfThreads = 128;
-
-struct NfArgs {
-  int F, N;
-  const double *qabs;    // [F][NQ][3]
-  const double *cp;      // [F][3]
-  const double *area;    // [F]
-  const double *sl;      // [F][3]
-  const int *hpar;       // [F][3] global edge of local edge q
-  const FaceGeo *geo;    // [F]
-  const double *bn;      // [F][3][3] free vertex of local edge q
-  double thr2;           // (3 avelen)^2
-  double kr, ki;         // k = ri w / c0
-  Cd k2;                 // k^2
-  Cd c1, c2;             // i w mu0, 1 / (i w eps0 n^2)
-  const double2 *X;      // [nsrc][ldx]: J in 0..N-1, M in N..2N-1
-  int64_t ldx;
-  int nsrc;              // sources in this launch (<= NS)
-  const double *pts;     // [npts][3]
-  double2 *E, *H;        // [nsrc][npts][3] (the launch's first source at E)
-  int npts;
-};
-
 __device__ __forceinline__ Cd cadd(Cd a, Cd b) { return {a.re + b.re, a.im + b.im}; }
+__device__ __forceinline__ Cd csub(Cd a, Cd b) { return {a.re - b.re, a.im - b.im}; }
 __device__ __forceinline__ Cd csc(Cd a, double s) { return {a.re * s, a.im * s}; }
 __host__ __device__ __forceinline__ Cd cdivd(Cd a, Cd b) {
   const double d = b.re * b.re + b.im * b.im;
   return {(a.re * b.re + a.im * b.im) / d, (a.im * b.re - a.re * b.im) / d};
 }
+// acc + a b, acc - a b
+__device__ __forceinline__ Cd cfma(Cd a, Cd b, Cd acc) {
+  return {fma(a.re, b.re, fma(-a.im, b.im, acc.re)), fma(a.re, b.im, fma(a.im, b.re, acc.im))};
+}
+__device__ __forceinline__ Cd cfms(Cd a, Cd b, Cd acc) {
+  return {fma(-a.re, b.re, fma(a.im, b.im, acc.re)), fma(-a.re, b.im, fma(-a.im, b.re, acc.im))};
+}
+struct Cv {
+  Cd x, y, z;
+};
+__device__ __forceinline__ Cv cvcross(const Cv &a, const Cv &b) {
+  const Cd o = {0, 0};
+  return {cfms(a.z, b.y, cfma(a.y, b.z, o)), cfms(a.x, b.z, cfma(a.z, b.x, o)), cfms(a.y, b.x, cfma(a.x, b.y, o))};
+}
+__device__ __forceinline__ Cv cvadd(const Cv &a, const Cv &b) { return {cadd(a.x, b.x), cadd(a.y, b.y), cadd(a.z, b.z)}; }
+__device__ __forceinline__ Cv cvsub(const Cv &a, const Cv &b) { return {csub(a.x, b.x), csub(a.y, b.y), csub(a.z, b.z)}; }
+__device__ __forceinline__ Cv cvscale(Cd s, const Cv &a) { return {cmul(s, a.x), cmul(s, a.y), cmul(s, a.z)}; }
+// a D + b
+__device__ __forceinline__ Cv affine(Cd a, const double *D, const Cv &b) {
+  return {{fma(a.re, D[0], b.x.re), fma(a.im, D[0], b.x.im)},
+          {fma(a.re, D[1], b.y.re), fma(a.im, D[1], b.y.im)},
+          {fma(a.re, D[2], b.z.re), fma(a.im, D[2], b.z.im)}};
+}
+__device__ __forceinline__ Cd ld_c(const double2 *p) {
+  const double2 v = *p;
+  return {v.x, v.y};
+}
+__device__ __forceinline__ Cv ld_v(const double2 *p) { return {ld_c(p), ld_c(p + 1), ld_c(p + 2)}; }
 
-// One CTA per point; threads stride over the faces and reduce at the end.
-template <int NQ, int NS>
-__global__ void __launch_bounds__(kNfThreads) nfield_kernel(NfArgs a) {
-  const int ip = blockIdx.x;
-  const double r[3] = {a.pts[3 * ip], a.pts[3 * ip + 1], a.pts[3 * ip + 2]};
-  Cd e[NS][3], h[NS][3];
-#pragma unroll
-  for (int s = 0; s < NS; s++)
-#pragma unroll
-    for (int i = 0; i < 3; i++) e[s][i] = h[s][i] = Cd{0, 0};
-  const double k2r = a.k2.re, k2i = a.k2.im;
-  for (int f = threadIdx.x; f < a.F; f += blockDim.x) {
-    const double *cp = a.cp + 3 * f;
-    const double dc[3] = {r[0] - cp[0], r[1] - cp[1], r[2] - cp[2]};
-    const bool near = dc[0] * dc[0] + dc[1] * dc[1] + dc[2] * dc[2] < a.thr2;
-    Cd SG = {0, 0}, SGr[3] = {{0, 0}, {0, 0}, {0, 0}}, SPd[3] = {{0, 0}, {0, 0}, {0, 0}};
-    const double *q = a.qabs + (size_t)f * NQ * 3;
-#pragma unroll 1
-    for (int t = 0; t < NQ; t++) {
-      const double rp[3] = {q[3 * t], q[3 * t + 1], q[3 * t + 2]};
-      const double w = c_qw[t];
-      const double dx = r[0] - rp[0], dy = r[1] - rp[1], dz = r[2] - rp[2];
-      const double R2 = dx * dx + dy * dy + dz * dz;
-      Cd g, p;
-      if (R2 > 0) {
-        const double R = ::sqrt(R2), iR = 1.0 / R, iR2 = iR * iR, iR3 = iR2 * iR;
-        double sn, cs;
-        ::sincos(a.kr * R, &sn, &cs);
-        const double ea = ::exp(-a.ki * R);
-        const double er = ea * cs, ei = ea * sn;
-        const double qr = iR3 + a.ki * iR2, qi = -a.kr * iR2;  // 1/R^3 - i k / R^2
-        if (near) {  // green.f90 vGs / vgradGs: (e - 1)/R + k^2 R / 2, e q - 1/R^3 - k^2/(2R)
-          g = {(er - 1.0) * iR + 0.5 * k2r * R, ei * iR + 0.5 * k2i * R};
-          p = {er * qr - ei * qi - iR3 - 0.5 * k2r * iR, er * qi + ei * qr - 0.5 * k2i * iR};
-        } else {
-          g = {er * iR, ei * iR};
-          p = {er * qr - ei * qi, er * qi + ei * qr};
-        }
-      } else if (near) {  // R = 0: Gs = i k / (4 pi), grad Gs = 0
-        g = {-a.ki, a.kr};
-        p = {0, 0};
-      } else {
-        g = {0, 0};
-        p = {0, 0};
-      }
-      const double dd[3] = {dx, dy, dz};
-      SG = cadd(SG, csc(g, w));
-#pragma unroll
+// The affine currents of a face about its centroid: a = sum_p v_p sl_p / 2,
+// b = -sum_p v_p sl_p mu_p / 2, for the J and M halves of vector v + s ldv,
+// s = blockIdx.y: coef[s][F][8] = aJ, bJ[3], aM, bM[3].
+__global__ void face_current_kernel(int F, int N, const int *hpar, const double *sl, const double *mu,
+                                    const double2 *v, int64_t ldv, double2 *coef) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= F) return;
+  v += (size_t)blockIdx.y * ldv;
+  for (int h = 0; h < 2; h++) {
+    Cd a = {0, 0}, b[3] = {{0, 0}, {0, 0}, {0, 0}};
+    for (int p = 0; p < 3; p++) {
+      const double2 c = v[hpar[3 * f + p] + (h ? N : 0)];
+      const double s = 0.5 * sl[3 * f + p];
+      a.re += s * c.x;
+      a.im += s * c.y;
       for (int i = 0; i < 3; i++) {
-        SGr[i] = cadd(SGr[i], csc(g, w * rp[i]));
-        SPd[i] = cadd(SPd[i], csc(p, w * dd[i]));
+        const double t = s * mu[9 * (size_t)f + 3 * p + i];
+        b[i].re -= t * c.x;
+        b[i].im -= t * c.y;
       }
     }
-    const double An = a.area[f], sc = An * kOofpi;
-    SG = csc(SG, sc);
-    Cd grad[3];  // int grad'G over the face (+ its closed-form part when near)
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      SGr[i] = csc(SGr[i], sc);
-      grad[i] = csc(SPd[i], sc);
-    }
-    PointStatic<double> ps;
-    const double f4 = 1.0 / (4.0 * kPi);
-    const Cd f8 = {k2r / (8.0 * kPi), k2i / (8.0 * kPi)};
-    if (near) {
-      // intK3singular (srcint.f90:227-260): (1/(4 pi)) K3m1 - (k^2/(8 pi)) K31
-      point_static(r, a.geo[f], ps);
-#pragma unroll
-      for (int i = 0; i < 3; i++) grad[i] = cadd(grad[i], {f4 * ps.K3m1[i] - f8.re * ps.K31[i], -f8.im * ps.K31[i]});
-    }
-#pragma unroll
-    for (int qe = 0; qe < 3; qe++) {
-      const double slq = a.sl[3 * f + qe];
-      const double cq = slq / (2.0 * An), dq = slq / An;
-      const double *pq = a.bn + 9 * f + 3 * qe;
-      const double rpq[3] = {r[0] - pq[0], r[1] - pq[1], r[2] - pq[2]};
-      Cd K2[3], K3[3], K4[3];
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        K2[i] = csc({SGr[i].re - pq[i] * SG.re, SGr[i].im - pq[i] * SG.im}, cq);
-        K3[i] = csc(grad[i], dq);
-      }
-      // K4 = -c_q (r - p_q) x grad (intK4singular, srcint.f90:330-366, has the same form)
-      K4[0] = csc({rpq[1] * grad[2].re - rpq[2] * grad[1].re, rpq[1] * grad[2].im - rpq[2] * grad[1].im}, -cq);
-      K4[1] = csc({rpq[2] * grad[0].re - rpq[0] * grad[2].re, rpq[2] * grad[0].im - rpq[0] * grad[2].im}, -cq);
-      K4[2] = csc({rpq[0] * grad[1].re - rpq[1] * grad[0].re, rpq[0] * grad[1].im - rpq[1] * grad[0].im}, -cq);
-      if (near) {
-        // intK2singular (srcint.f90:121-154)
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          const double k2m1 = cq * (ps.mL1[i] + (ps.rho[i] - pq[i]) * ps.Sm1);
-          const double k21 = cq * (1.0 / 3.0 * ps.mL3[i] + (ps.rho[i] - pq[i]) * ps.S1);
-          K2[i] = cadd(K2[i], {f4 * k2m1 - f8.re * k21, -f8.im * k21});
-        }
-      }
-      const int idx = a.hpar[3 * f + qe];
-#pragma unroll
-      for (int s = 0; s < NS; s++) {
-        if (s >= a.nsrc) break;
-        const double2 xj2 = a.X[(size_t)s * a.ldx + idx], xm2 = a.X[(size_t)s * a.ldx + idx + a.N];
-        const Cd xj = {xj2.x, xj2.y}, xm = {xm2.x, xm2.y};
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          const Cd ee = cadd(cadd(cmul(a.c1, K2[i]), cmul(a.c2, K3[i])), Cd{0, 0});
-          e[s][i] = cadd(e[s][i], cadd(cmul(xj, ee), cmul(xm, K4[i])));
-          const Cd hh = cadd(cdivd(K2[i], a.c2), cdivd(K3[i], a.c1));
-          const Cd hx = cmul(xm, hh), hj = cmul(xj, K4[i]);
-          h[s][i] = cadd(h[s][i], {hx.re - hj.re, hx.im - hj.im});
-        }
-      }
-    }
-  }
-  // CTA reduction: warp shuffles, then one value per warp through shared memory
-  __shared__ double red[kNfThreads / 32][NS * 12];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int s = 0; s < NS; s++)
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      double v[4] = {e[s][i].re, e[s][i].im, h[s][i].re, h[s][i].im};
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_down_sync(0xffffffffu, v[c], o);
-        if (lane == 0) red[wid][s * 12 + i * 4 + c] = v[c];
-      }
-    }
-  __syncthreads();
-  for (int j = threadIdx.x; j < NS * 12; j += blockDim.x) {
-    const int s = j / 12, i = (j % 12) / 4, c = j % 4;
-    if (s >= a.nsrc) continue;
-    double t = 0;
-    for (int w = 0; w < kNfThreads / 32; w++) t += red[w][j];
-    double2 *dst = (c < 2 ? a.E : a.H) + ((size_t)s * a.npts + ip) * 3 + i;
-    if (c % 2 == 0) dst->x = t;
-    else dst->y = t;
+    double2 *o = coef + 8 * ((size_t)blockIdx.y * F + f) + 4 * h;
+    o[0] = make_double2(a.re, a.im);
+    for (int i = 0; i < 3; i++) o[1 + i] = make_double2(b[i].re, b[i].im);
   }
 }
 
+constexpr int kNfThreads = 128;
+constexpr int kNfTile = 8;  // faces staged at a time
+
+struct NfArgs {
+  int F;
+  const double *qrel;    // [F][NQ][3] minus the centroid
+  const double *cp;      // [F][3]
+  const double *area;    // [F]
+  const FaceGeo *geo;    // [F]
+  const double2 *coef;   // [sources][F][8] (the launch's first source)
+  double thr2;           // (3 avelen)^2
+  double kr, ki;         // k = ri w / c0
+  Cd k2;                 // k^2
+  Cd c1, c2, ic1, ic2;   // i w mu0, 1 / (i w eps0 n^2), and their reciprocals
+  int nsrc;              // sources in this launch (<= NS)
+  const double *pts;     // [npts][3]
+  int npts, per_split;   // faces per split (blockIdx.y)
+  double2 *part;         // [split][nsrc][npts][6]: E, H
+};
+
+// The closed-form parts of face n at r for one source's currents, added to
+// E, H (times 4 pi: the caller scales the sums).
+__device__ __noinline__ void nfield_static(const NfArgs &a, const double *r, const double *D0, int n, int ns, Cv *E,
+                                           Cv *H) {
+  PointStatic<double> ps;
+  point_static(r, a.geo[n], ps);
+  const double iA = 1.0 / a.area[n];
+  const double f4 = 1.0 / (4.0 * kPi) / kOofpi;
+  const Cd f8 = {a.k2.re / (8.0 * kPi) / kOofpi, a.k2.im / (8.0 * kPi) / kOofpi};
+  const Cd y0 = {f4 * ps.Sm1 - f8.re * ps.S1, -f8.im * ps.S1};
+  Cd gr[3], l[3];
+  double rc[3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    gr[i] = {iA * (f4 * ps.K3m1[i] - f8.re * ps.K31[i]), -iA * f8.im * ps.K31[i]};
+    l[i] = {f4 * ps.mL1[i] - f8.re * ps.mL3[i] / 3.0, -f8.im * ps.mL3[i] / 3.0};
+    rc[i] = ps.rho[i] - a.cp[3 * n + i];
+  }
+  const Cv P = {gr[0], gr[1], gr[2]}, Lv = {l[0], l[1], l[2]};
+#pragma unroll 1
+  for (int s = 0; s < ns; s++) {
+    const double2 *c = a.coef + ((size_t)s * a.F + n) * 8;
+    const Cd aJ = ld_c(c), aM = ld_c(c + 4), z = {iA, 0};
+    const Cv bJ = ld_v(c + 1), bM = ld_v(c + 5);
+    // int (a r' + b) / A over R and R: a (mL + rho S) + b S
+    const Cv yJ = cvscale(z, cvadd(cvscale(aJ, Lv), cvscale(y0, affine(aJ, rc, bJ))));
+    const Cv yM = cvscale(z, cvadd(cvscale(aM, Lv), cvscale(y0, affine(aM, rc, bM))));
+    E[s] = cvadd(E[s], cvsub(cvadd(cvscale(a.c1, yJ), cvscale(csc(cmul(a.c2, aJ), 2.0), P)),
+                             cvcross(affine(aM, D0, bM), P)));
+    H[s] = cvadd(H[s], cvadd(cvadd(cvscale(a.ic2, yM), cvscale(csc(cmul(a.ic1, aM), 2.0), P)),
+                             cvcross(affine(aJ, D0, bJ), P)));
+  }
+}
+
+// One thread per point over the faces of its split, staged in shared memory
+// in tiles (broadcast reads; neighbouring points share their near faces, so
+// warps seldom diverge).  FP64-pipe bound, about 90 instructions per point and
+// quadrature point; a 101 x 101 plane over 1,280 faces with one CTA per point
+// and the three RWG functions of a face apart took 3.7 ms.
+template <int NQ, int NS, bool LOSSLESS>
+__global__ void __launch_bounds__(kNfThreads) nfield_kernel(NfArgs a) {
+  constexpr int kCoef = 16 * NS, kFace = (kCoef + 3 + 3 * NQ + 1) / 2 * 2;
+  __shared__ __align__(16) double s_face[kNfTile][kFace];
+  const int ip = blockIdx.x * kNfThreads + threadIdx.x;
+  const bool valid = ip < a.npts;
+  double r[3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) r[i] = valid ? a.pts[3 * (size_t)ip + i] : 0.0;
+  Cv E[NS], H[NS];
+  const Cd z0 = {0, 0};
+#pragma unroll
+  for (int s = 0; s < NS; s++) E[s] = H[s] = Cv{z0, z0, z0};
+  const int n0 = blockIdx.y * a.per_split, n1 = min(a.F, n0 + a.per_split);
+  for (int base = n0; base < n1; base += kNfTile) {
+    const int cnt = min(kNfTile, n1 - base);
+    __syncthreads();
+    for (int e = threadIdx.x; e < cnt * (kCoef + 3 + 3 * NQ); e += kNfThreads) {
+      const int f = e / (kCoef + 3 + 3 * NQ), k = e % (kCoef + 3 + 3 * NQ), n = base + f;
+      double v;
+      if (k < kCoef)
+        v = k / 16 < a.nsrc ? reinterpret_cast<const double *>(a.coef + ((size_t)(k / 16) * a.F + n) * 8)[k % 16] : 0.0;
+      else if (k < kCoef + 3) v = a.cp[3 * n + k - kCoef];
+      else v = a.qrel[(size_t)n * NQ * 3 + k - kCoef - 3];
+      s_face[f][k] = v;
+    }
+    __syncthreads();
+    if (!valid) continue;
+#pragma unroll 1
+    for (int f = 0; f < cnt; f++) {
+      const double *fc = s_face[f], *fcp = fc + kCoef, *fq = fcp + 3;
+      const double D0[3] = {r[0] - fcp[0], r[1] - fcp[1], r[2] - fcp[2]};
+      const bool near = D0[0] * D0[0] + D0[1] * D0[1] + D0[2] * D0[2] < a.thr2;
+      Cd g0 = z0, g1[3] = {z0, z0, z0}, p1[3] = {z0, z0, z0};
+#pragma unroll 1
+      for (int j = 0; j < NQ; j++) {
+        const double D[3] = {D0[0] - fq[3 * j], D0[1] - fq[3 * j + 1], D0[2] - fq[3 * j + 2]};
+        const double R2 = D[0] * D[0] + D[1] * D[1] + D[2] * D[2], w = c_qw[j];
+        Cd g, p;
+        if (R2 > 0) {
+          const double iR = ::rsqrt(R2), R = R2 * iR;
+          double sn, cs;
+          ::sincos(a.kr * R, &sn, &cs);
+          const double ea = LOSSLESS ? 1.0 : ::exp(-a.ki * R);
+          const double er = ea * cs, ei = ea * sn, iR2 = iR * iR, iR3 = iR2 * iR;
+          const double qr = iR3 + a.ki * iR2, qi = -a.kr * iR2;  // 1/R^3 - i k / R^2
+          g = {er * iR, ei * iR};
+          p = {er * qr - ei * qi, er * qi + ei * qr};
+          if (near) {  // green.f90 vGs / vgradGs: (e - 1)/R + k^2 R / 2, e q - 1/R^3 - k^2/(2R)
+            g = {(er - 1.0) * iR + 0.5 * a.k2.re * R, ei * iR + 0.5 * a.k2.im * R};
+            p = {p.re - iR3 - 0.5 * a.k2.re * iR, p.im - 0.5 * a.k2.im * iR};
+          }
+        } else {  // R = 0: Gs = i k / (4 pi), grad Gs = 0
+          g = near ? Cd{-a.ki, a.kr} : z0;
+          p = z0;
+        }
+        g = csc(g, w);
+        p = csc(p, w);
+        g0 = cadd(g0, g);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          g1[i] = {fma(g.re, D[i], g1[i].re), fma(g.im, D[i], g1[i].im)};
+          p1[i] = {fma(p.re, D[i], p1[i].re), fma(p.im, D[i], p1[i].im)};
+        }
+      }
+      const Cv G1 = {g1[0], g1[1], g1[2]}, P1 = {p1[0], p1[1], p1[2]};
+#pragma unroll
+      for (int s = 0; s < NS; s++) {
+        const double2 *c = reinterpret_cast<const double2 *>(fc + 16 * s);
+        const Cd aJ = ld_c(c), aM = ld_c(c + 4);
+        const Cv XJ = affine(aJ, D0, ld_v(c + 1)), XM = affine(aM, D0, ld_v(c + 5));
+        const Cv uj = cvsub(cvscale(g0, XJ), cvscale(aJ, G1)), um = cvsub(cvscale(g0, XM), cvscale(aM, G1));
+        E[s] = cvadd(E[s], cvsub(cvadd(cvscale(a.c1, uj), cvscale(csc(cmul(a.c2, aJ), 2.0), P1)), cvcross(XM, P1)));
+        H[s] = cvadd(H[s], cvadd(cvadd(cvscale(a.ic2, um), cvscale(csc(cmul(a.ic1, aM), 2.0), P1)), cvcross(XJ, P1)));
+      }
+      if (near) nfield_static(a, r, D0, base + f, min(NS, a.nsrc), E, H);
+    }
+  }
+  if (!valid) return;
+#pragma unroll
+  for (int s = 0; s < NS; s++) {
+    if (s >= a.nsrc) break;
+    double2 *o = a.part + (((size_t)blockIdx.y * a.nsrc + s) * a.npts + ip) * 6;
+    const Cd v[6] = {E[s].x, E[s].y, E[s].z, H[s].x, H[s].y, H[s].z};
+#pragma unroll
+    for (int i = 0; i < 6; i++) o[i] = make_double2(kOofpi * v[i].re, kOofpi * v[i].im);
+  }
+}
+
+// E, H [nsrc][npts][3]: the splits' parts in split order.
+__global__ void nfield_sum_kernel(int npts, int nsrc, int splits, const double2 *part, double2 *E, double2 *H) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t per = (int64_t)nsrc * npts * 6;
+  if (e >= per) return;
+  double2 v = make_double2(0, 0);
+  for (int s = 0; s < splits; s++) {
+    const double2 p = part[s * per + e];
+    v.x += p.x;
+    v.y += p.y;
+  }
+  const int64_t at = e / 6;
+  const int i = (int)(e % 6);
+  (i < 3 ? E : H)[at * 3 + i % 3] = v;
+}
+
+template <int NQ, bool LOSSLESS>
+void launch_nfield_k(int ns, const dim3 &grid, cudaStream_t st, const NfArgs &a) {
+  if (ns == 1) nfield_kernel<NQ, 1, LOSSLESS><<<grid, kNfThreads, 0, st>>>(a);
+  else if (ns == 2) nfield_kernel<NQ, 2, LOSSLESS><<<grid, kNfThreads, 0, st>>>(a);
+  else nfield_kernel<NQ, 4, LOSSLESS><<<grid, kNfThreads, 0, st>>>(a);
+}
 template <int NQ>
-void launch_nfield(int ns, int npts, cudaStream_t st, const NfArgs &a) {
-  if (ns == 1) nfield_kernel<NQ, 1><<<npts, kNfThreads, 0, st>>>(a);
-  else if (ns == 2) nfield_kernel<NQ, 2><<<npts, kNfThreads, 0, st>>>(a);
-  else nfield_kernel<NQ, 4><<<npts, kNfThreads, 0, st>>>(a);
+void launch_nfield(int ns, const dim3 &grid, cudaStream_t st, const NfArgs &a) {
+  if (a.ki == 0.0) launch_nfield_k<NQ, true>(ns, grid, st, a);
+  else launch_nfield_k<NQ, false>(ns, grid, st, a);
 }
 
 }  // namespace
@@ -232,17 +297,24 @@ int scat_fields(Ctx *c, int d, double omega, const double *ri, int nsrc, const d
   if (d < 0 || d >= c->ndom) return fail(c, MOM_ERR_ARG, "domain index out of range");
   DomDev &D = c->dom[d];
   MOM_TRY(nfield_geometry(c, D));
+  const int F = D.F;
+  // faces per split: eight CTAs per SM in all, at least one tile of faces each
+  const int blocks = (npts + kNfThreads - 1) / kNfThreads;
+  const int want = std::max(1, std::min((F + kNfTile - 1) / kNfTile, 8 * c->nsm / blocks));
+  const int per = ((F + want - 1) / want + kNfTile - 1) / kNfTile * kNfTile, splits = (F + per - 1) / per;
+  const size_t b_coef = sizeof(double2) * 8 * (size_t)F * nsrc;
+  const size_t b_part = sizeof(double2) * 6 * (size_t)npts * std::min(nsrc, 4) * splits;
+  MOM_TRY(ensure_buffer(c, &c->adj_part, &c->adj_part_bytes, b_coef + b_part));
+  double2 *coef = (double2 *)c->adj_part;
+  face_current_kernel<<<dim3((F + 127) / 128, nsrc), 128, 0, c->stream>>>(F, c->N, D.hpar, D.sl, D.mu, X, ldx, coef);
+  c->launches++;
   const double k0 = omega / kC0;
   NfArgs a;
-  a.F = D.F;
-  a.N = c->N;
-  a.qabs = D.qabs;
+  a.F = F;
+  a.qrel = D.qrel;
   a.cp = D.cp;
   a.area = D.area;
-  a.sl = D.sl;
-  a.hpar = D.hpar;
   a.geo = reinterpret_cast<const FaceGeo *>(D.nf_geo);
-  a.bn = D.nf_bn;
   a.thr2 = (D.avelen * 3) * (D.avelen * 3);
   a.kr = ri[0] * k0;
   a.ki = ri[1] * k0;
@@ -251,25 +323,30 @@ int scat_fields(Ctx *c, int d, double omega, const double *ri, int nsrc, const d
   const Cd n2 = {ri[0] * ri[0] - ri[1] * ri[1], 2 * ri[0] * ri[1]};
   const Cd den = {-omega * kEps0 * n2.im, omega * kEps0 * n2.re};  // i w eps0 n^2
   a.c2 = cdivd({1.0, 0.0}, den);
-  a.ldx = ldx;
+  a.ic1 = cdivd({1.0, 0.0}, a.c1);
+  a.ic2 = den;
   a.pts = pts;
   a.npts = npts;
+  a.per_split = per;
+  a.part = (double2 *)((char *)c->adj_part + b_coef);
   for (int s0 = 0; s0 < nsrc; s0 += 4) {
     const int ns = std::min(4, nsrc - s0);
     a.nsrc = ns;
-    a.X = X + (size_t)s0 * ldx;
-    a.E = E + (size_t)s0 * npts * 3;
-    a.H = H + (size_t)s0 * npts * 3;
+    a.coef = coef + 8 * (size_t)F * s0;
     const int nl = ns == 1 ? 1 : (ns == 2 ? 2 : 4);
+    const dim3 grid(blocks, splits);
     switch (c->nq) {
-      case 1: launch_nfield<1>(nl, npts, c->stream, a); break;
-      case 3: launch_nfield<3>(nl, npts, c->stream, a); break;
-      case 4: launch_nfield<4>(nl, npts, c->stream, a); break;
-      case 7: launch_nfield<7>(nl, npts, c->stream, a); break;
-      case 13: launch_nfield<13>(nl, npts, c->stream, a); break;
+      case 1: launch_nfield<1>(nl, grid, c->stream, a); break;
+      case 3: launch_nfield<3>(nl, grid, c->stream, a); break;
+      case 4: launch_nfield<4>(nl, grid, c->stream, a); break;
+      case 7: launch_nfield<7>(nl, grid, c->stream, a); break;
+      case 13: launch_nfield<13>(nl, grid, c->stream, a); break;
       default: return fail(c, MOM_ERR_ARG, "unsupported number of quadrature points");
     }
-    c->launches++;
+    const int64_t vals = (int64_t)ns * npts * 6;
+    nfield_sum_kernel<<<(unsigned)((vals + 255) / 256), 256, 0, c->stream>>>(
+        npts, ns, splits, a.part, E + (size_t)s0 * npts * 3, H + (size_t)s0 * npts * 3);
+    c->launches += 2;
     MOM_CUDA(c, cudaGetLastError());
   }
   return MOM_OK;
