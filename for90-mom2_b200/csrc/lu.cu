@@ -10,8 +10,8 @@
 //   laswp_kernel   the panel's row interchanges on the other columns;
 //   diag_inv       inverses of the unit-lower and upper diagonal blocks;
 //   TRSM as GEMM   U12 = inv(L11) A12, then A22 -= L21 U12 (plain library
-//                  GEMMs: cuBLAS ZGEMM for FP64, CGEMM on TF32 tensor cores
-//                  for the mixed path).
+//                  GEMMs: cuBLAS ZGEMM for FP64, CGEMM for the narrow steps
+//                  of the mixed path, whose trailing updates run in tc_gemm.cu).
 // The mixed path factors an FP32 copy and refines in FP64 against the FP64
 // matrix (iterative refinement; residual GEMV kernel below).
 #include <cuda_runtime.h>
@@ -1343,7 +1343,7 @@ int lu_enqueue(Ctx *c, T *A, int precision, const LuWork &w) {
     return MOM_OK;
   };
   // C(m x ncol) -= L(m x nb) U(nb x ncol): the rank-64 updates; on the
-  // tensor cores (3xTF32) in the mixed path, as the trailing update
+  // tensor cores in the mixed path, as the trailing update
   auto update64 = [&](int64_t m, int64_t ncol, const T *Lm, const T *Um, T *Cm) -> int {
     if (m <= 0 || ncol <= 0) return MOM_OK;
     if (mixed && c->small_tc)
@@ -1407,7 +1407,7 @@ int lu_enqueue(Ctx *c, T *A, int precision, const LuWork &w) {
         MOM_TRY(update64(below, nc, A + (j0 + nb) + j0 * lda, A + j0 + t0 * lda, A + (j0 + nb) + t0 * lda));
       }
       if (mixed) {
-        // the large update on the tensor cores (3xTF32, FP32-accurate)
+        // the large update on the tensor cores (FP32-accurate)
         MOM_TRY(tc_cgemm_update(c, reinterpret_cast<float2 *>(A + t0 + t0 * lda), lda,
                                 reinterpret_cast<const float2 *>(A + t0 + J0 * lda), lda,
                                 reinterpret_cast<const float2 *>(A + J0 + t0 * lda), lda, (int)(n - t0), (int)nc,
@@ -2047,7 +2047,7 @@ int getrs_multi(Ctx *c, const T *F, double2 *X, int nrhs, int trans) {
   const int nb = c->nb, nblk = (int)(n / nb);
   const bool f32 = sizeof(T) == sizeof(float2);
   // FP32 factors and many right-hand sides: 256-row blocks whose updates run
-  // on the tensor cores (3xTF32, FP32-accurate like the rest of the solve)
+  // on the tensor cores (FP32-accurate like the rest of the solve)
   const bool tc = f32 && nrhs >= kMultiTc;
   const int64_t NBt = 4 * (int64_t)nb;
   const size_t ybytes = sizeof(T) * (size_t)n * nrhs, tbytes = sizeof(T) * (size_t)nb * nrhs;

@@ -383,7 +383,7 @@ int panel_reg(Ctx *c, float2 *A, int64_t lda, int64_t n, int64_t j0, int *ipiv, 
 int panel_reg(Ctx *c, double2 *A, int64_t lda, int64_t n, int64_t j0, int *ipiv, int *info, int *timeout,
               cudaStream_t st);
 
-// tc_gemm.cu: C -= L U (complex FP32) on the tensor cores, 3xTF32
+// tc_gemm.cu: C -= L U (complex FP32) on the tensor cores, FP32-accurate
 int tc_cgemm_update(Ctx *c, float2 *C, int64_t ldc, const float2 *L, int64_t ldl, const float2 *U, int64_t ldu, int m,
                     int nc, int k, float *work, int *err, int max_ctas = 0, bool reuse_a = false,
                     bool trans_l = false);

@@ -7,24 +7,39 @@
 //   Ahat[2i][2l] = Re L, Ahat[2i][2l+1] = -Im L, Ahat[2i+1][2l] = Im L,
 //   Ahat[2i+1][2l+1] = Re L
 // and U12 viewed as real 2k x nc (its own interleaved storage), C -= Ahat B.
-// Accuracy: each operand is split into a TF32 high part and an FP32 low
-// remainder, and the MMA accumulates hi*hi + hi*lo + lo*hi (three
-// kind::tf32 passes into one FP32 TMEM accumulator), which keeps the
-// factorisation close to FP32 accuracy so FP64 refinement converges in a
-// few steps.
+// Accuracy: each operand is split into two FP16 numbers, high part and
+// remainder, after a scaling by a power of two per row of L21 and per column
+// of U12 that puts its largest entry just below 2^15; the MMA accumulates
+// hi*hi + hi*lo + lo*hi (three kind::f16 passes into one FP32 TMEM
+// accumulator) and the epilogue undoes the scaling.  An entry keeps 22 bits, or
+// 2^-40 of its row's (column's) largest entry.  Three passes on TF32 parts keep
+// no more (the tensor core cuts the remainder to TF32) at half the rate and
+// twice the operand bytes.  Measured, relative Frobenius error of C - L U
+// against FP64, Gaussian operands (rows and columns scaled by any powers of
+// two alike), k = 16 / 48 / 64 / 128 / 256: 2.0e-7 / 4.3e-7 / 5.3e-7 / 9.8e-7 /
+// 1.9e-6, with TF32 parts 3.0e-7 / 7.5e-7 / 9.6e-7 / 1.9e-6 / 3.7e-6.
 //
 // Kernel: persistent, one CTA per SM, 128 x 256 output tiles, K blocks of
-// 32 floats (one 128-byte swizzle atom) staged by TMA in a 2-deep ring.
-//   warp 0   TMA producer (one elected lane)
-//   warp 1   MMA issuer (one elected lane; tcgen05.mma cta_group::1)
-//   warp 2   TMEM allocator (512 columns = two 128 x 256 accumulators)
-//   warps 4-7 epilogue: tcgen05.ld the accumulator, C -= acc (coalesced)
+// 32 halves (one 64-byte swizzle row) staged by TMA in a 4-deep ring (three
+// stages can be under way while one is consumed).
+//   warp 0    TMA producer (one elected lane)
+//   warp 1    MMA issuer (one elected lane; tcgen05.mma cta_group::1)
+//   warp 2    TMEM allocator (512 columns = two 128 x 256 accumulators)
+//   warps 4-11 epilogue: tcgen05.ld the accumulator, C -= acc (coalesced);
+//             two warps per 32 rows, so that enough of C is in flight to keep
+//             up with the MMAs of a K = 512 tile
+// Bound: with n = 15,360 and K = 512 a tile's MMAs take 6.6 us, its operands
+// 786 KB through L2 and its part of C 262 KB of HBM traffic; the 59 trailing
+// updates of the factorisation take 27.7 ms (43.3 ms with TF32 parts, two
+// stages and four epilogue warps; 18.3 ms at the bf16 rate).
 // Every mbarrier wait is bounded; on timeout the kernel records the error,
 // stops issuing work, waits (bounded) for its own copies and for the MMAs
 // already issued, frees TMEM and exits.
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 
@@ -33,11 +48,12 @@
 namespace mom {
 namespace {
 
-constexpr int kBM = 128, kBN = 256, kBK = 32, kStages = 2;
-constexpr int kTileA = kBM * kBK * 4;  // bytes of one A tile (hi or lo)
-constexpr int kTileB = kBN * kBK * 4;  // bytes of one B tile
+constexpr int kBM = 128, kBN = 256, kBK = 32, kStages = 4;
+constexpr int kTileA = kBM * kBK * 2;  // bytes of one A tile (hi or lo)
+constexpr int kTileB = kBN * kBK * 2;  // bytes of one B tile
 constexpr int kStageBytes = 2 * kTileA + 2 * kTileB;
-constexpr int kTcThreads = 256;
+constexpr int kEpiWarps = 8, kTcThreads = 128 + 32 * kEpiWarps;
+constexpr int kEpiCols = 32;  // columns of C an epilogue warp has in flight
 constexpr long long kDrainPolls = 1LL << 22;  // bound of the waits for work already issued
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -83,27 +99,26 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, u
       : "memory");
 }
 
-// K-major, 128-byte swizzled operand tile: rows of 128 bytes, 8-row atoms of
-// 1024 bytes (SBO), LBO unused (1), descriptor version 1, layout SWIZZLE_128B.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
+// K-major, 64-byte swizzled operand tile: rows of 64 bytes, 8-row atoms of
+// 512 bytes (SBO), LBO unused (1), descriptor version 1, layout SWIZZLE_64B.
+__device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;            // LBO (16-byte units)
-  d |= (uint64_t)(1024 >> 4) << 32;  // SBO
-  d |= (uint64_t)1 << 46;            // version
-  d |= (uint64_t)2 << 61;            // SWIZZLE_128B
+  d |= (uint64_t)1 << 16;           // LBO (16-byte units)
+  d |= (uint64_t)(512 >> 4) << 32;  // SBO
+  d |= (uint64_t)1 << 46;           // version
+  d |= (uint64_t)4 << 61;           // SWIZZLE_64B
   return d;
 }
 
-// kind::tf32 instruction descriptor: D f32, A/B tf32, both K-major, M=128, N=256.
-constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(kBN >> 3) << 17) |
-                            ((uint32_t)(kBM >> 4) << 24);
+// kind::f16 instruction descriptor: D f32, A/B f16, both K-major, M=128, N=256.
+constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 
-__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
       : "memory");
 }
@@ -115,7 +130,8 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
 struct TcArgs {
   float *C;        // real view of the complex FP32 C block
   int64_t ldc;     // in floats
-  int Mr, Nc, Kr;  // real rows of C, columns, real K
+  int Mr, Nc, Kp;  // real rows of C, columns, real K padded to kBK
+  const float *rinv, *cinv;  // undo the scaling: per complex row, per column
   int *err;        // device error word (timeout)
   long long spin;  // polls before an mbarrier wait is declared timed out
 };
@@ -124,13 +140,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap mAhi, const __grid_constant__ CUtensorMap mAlo,
                    const __grid_constant__ CUtensorMap mBhi, const __grid_constant__ CUtensorMap mBlo, TcArgs a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  // 1024-byte aligned stage buffers (SWIZZLE_128B atoms need it)
+  // 1024-byte aligned stage buffers (swizzle atoms need 512)
   unsigned char *smem = reinterpret_cast<unsigned char *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2], drain;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int numM = a.Mr / kBM, numN = (a.Nc + kBN - 1) / kBN, ntiles = numM * numN, nk = a.Kr / kBK;
+  const int numM = a.Mr / kBM, numN = (a.Nc + kBN - 1) / kBN, ntiles = numM * numN, nk = a.Kp / kBK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; s++) {
@@ -139,7 +155,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], 4);  // one arrival per epilogue warp
+      mbar_init(&acc_empty[b], kEpiWarps);  // one arrival per epilogue warp
     }
     mbar_init(&drain, 1);
     abort_flag = 0;
@@ -212,11 +228,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           const uint32_t base = smem_u32(smem + (size_t)s * kStageBytes);
           const uint32_t ahi = base, alo = base + kTileA, bhi = base + 2 * kTileA, blo = base + 2 * kTileA + kTileB;
 #pragma unroll
-          for (int k = 0; k < kBK / 8; k++) {
-            const uint32_t off = (uint32_t)k * 32;  // 8 tf32 = 32 bytes along K inside the swizzle atom
-            mma_tf32(d, sw128_desc(ahi + off), sw128_desc(bhi + off), (kb | k) != 0);
-            mma_tf32(d, sw128_desc(ahi + off), sw128_desc(blo + off), 1);
-            mma_tf32(d, sw128_desc(alo + off), sw128_desc(bhi + off), 1);
+          for (int k = 0; k < kBK / 16; k++) {
+            const uint32_t off = (uint32_t)k * 32;  // 16 halves = 32 bytes along K inside the swizzle atom
+            mma_f16(d, sw64_desc(ahi + off), sw64_desc(bhi + off), (kb | k) != 0);
+            mma_f16(d, sw64_desc(ahi + off), sw64_desc(blo + off), 1);
+            mma_f16(d, sw64_desc(alo + off), sw64_desc(bhi + off), 1);
           }
           mma_commit(&empty[s]);  // frees the stage when these MMAs complete
           if (++s == kStages) {
@@ -237,39 +253,52 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
   } else if (warp >= 4) {
     // ---------------- epilogue ----------------
-    const int ew = warp - 4;  // TMEM lanes 32*ew .. 32*ew+31
+    const int ew = warp % 4;            // TMEM lanes 32*ew .. 32*ew+31
+    const int half = (warp - 4) / 4;    // columns half * 128 .. of the tile
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, it++) {
       const int acc = it & 1;
       const unsigned acc_ph = (it >> 1) & 1;
-      int ok = 1;
-      if (lane == 0) ok = mbar_wait(&acc_full[acc], acc_ph, abort, a.spin) ? 1 : 0;
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int tm = t % numM, tn = t / numM;
       const int64_t row = (int64_t)tm * kBM + ew * 32 + lane;
       float *crow = a.C + row;
+      const float rs = a.rinv[row >> 1];
+      int ok = 1;
 #pragma unroll 1
-      for (int c0 = 0; c0 < kBN; c0 += 16) {
-        uint32_t v[16];
+      for (int c0 = half * (kBN / 2); c0 < (half + 1) * (kBN / 2); c0 += kEpiCols) {
+        const int col0 = tn * kBN + c0;
+        // the loads of C in flight before the accumulator is waited for and
+        // before the stores (which the compiler must assume to alias them)
+        float cv[kEpiCols];
+#pragma unroll
+        for (int j = 0; j < kEpiCols; j++)
+          cv[j] = (col0 + j < a.Nc) ? __ldcs(crow + (int64_t)(col0 + j) * a.ldc) : 0.0f;
+        if (c0 == half * (kBN / 2)) {
+          if (lane == 0) ok = mbar_wait(&acc_full[acc], acc_ph, abort, a.spin) ? 1 : 0;
+          ok = __shfl_sync(0xffffffffu, ok, 0);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
+        const float sc = col0 + lane < a.Nc ? a.cinv[col0 + lane] : 0.0f;
+        uint32_t v[kEpiCols];
         const uint32_t taddr = tmem + ((uint32_t)(ew * 32) << 16) + (uint32_t)(acc * kBN + c0);
         asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-            "%14, %15}, [%16];"
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+            "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+              "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+              "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
             : "r"(taddr));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const int col0 = tn * kBN + c0;
-        // all 16 loads in flight before the stores (the stores could alias them otherwise)
-        float cv[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++) cv[j] = (col0 + j < a.Nc) ? __ldcs(crow + (int64_t)(col0 + j) * a.ldc) : 0.0f;
-#pragma unroll
-        for (int j = 0; j < 16; j++)
-          if (col0 + j < a.Nc) __stcs(crow + (int64_t)(col0 + j) * a.ldc, cv[j] - __uint_as_float(v[j]));
+        for (int j = 0; j < kEpiCols; j++) {
+          const float cs = __shfl_sync(0xffffffffu, sc, j);
+          if (col0 + j < a.Nc)
+            __stcs(crow + (int64_t)(col0 + j) * a.ldc, fmaf(-(__uint_as_float(v[j]) * rs), cs, cv[j]));
+        }
       }
+      if (!ok) break;
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
@@ -283,61 +312,100 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   }
 }
 
-// Ahat_hi / Ahat_lo (Mr x Kr, row-major) from the complex block L (m x k, ld),
-// or (tr) from the transpose of a k x m block: L(i, l) = P[l + i ld].  In
-// 32 x 32 tiles through shared memory: the complex block is read along its
-// contiguous direction and the expanded rows are written as FP32 pairs
-// (block 32 x 8 threads).
-__global__ void __launch_bounds__(256) expand_a_tiled_kernel(const float2 *L, int64_t ld, int m, int k, float *hi,
-                                                             float *lo, bool tr) {
+// Power of two that puts a magnitude with these float bits into [2^14, 2^15),
+// and its reciprocal.
+__device__ __forceinline__ float scale_of(unsigned bits, float *inv) {
+  const int e = (int)(bits >> 23);                  // biased exponent, 0 for zero
+  const int s = bits == 0u ? 0 : min(126, max(-126, 141 - e));
+  *inv = __uint_as_float((unsigned)(127 - s) << 23);
+  return __uint_as_float((unsigned)(127 + s) << 23);
+}
+__device__ __forceinline__ unsigned mag_bits(float2 z) {
+  return max(__float_as_uint(fabsf(z.x)), __float_as_uint(fabsf(z.y)));
+}
+// v = hi + lo up to FP16 rounding of the remainder
+__device__ __forceinline__ void split_half(float v, __half *hi, __half *lo) {
+  *hi = __float2half_rn(v);
+  *lo = __float2half_rn(v - __half2float(*hi));
+}
+
+// Ahat_hi / Ahat_lo (2m x Kp halves, row-major) from the complex block L
+// (m x k, ld), or (tr) from the transpose of a k x m block: L(i, l) = P[l + i
+// ld], and the rows' inverse scales.  One CTA (32 x 8 threads) per 32 rows:
+// their largest entries first, then 32 x 32 tiles through shared memory, the
+// complex block read along its contiguous direction both times (the second
+// time from L2) and the expanded rows written as pairs of halves.
+__global__ void __launch_bounds__(256) expand_a_kernel(const float2 *L, int64_t ld, int m, int k, int Kp, __half *hi,
+                                                       __half *lo, float *rinv, bool tr) {
   __shared__ float2 t[32][33];  // [l][i] of the tile
-  const int i0 = blockIdx.y * 32, l0 = blockIdx.x * 32, tx = threadIdx.x;
-  for (int r = threadIdx.y; r < 32; r += 8) {
-    if (!tr) {
-      const int i = i0 + tx, l = l0 + r;
-      t[r][tx] = (i < m && l < k) ? L[i + (int64_t)l * ld] : make_float2(0.f, 0.f);
-    } else {
-      const int l = l0 + tx, i = i0 + r;
-      t[tx][r] = (i < m && l < k) ? L[l + (int64_t)i * ld] : make_float2(0.f, 0.f);
+  __shared__ unsigned s_max[32];
+  const int i0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
+  if (ty == 0) s_max[tx] = 0u;
+  __syncthreads();
+  if (!tr) {
+    unsigned b = 0u;
+    if (i0 + tx < m)
+      for (int l = ty; l < k; l += 8) b = max(b, mag_bits(L[i0 + tx + (int64_t)l * ld]));
+    atomicMax(&s_max[tx], b);
+  } else {
+    for (int r = ty; r < 32; r += 8) {
+      unsigned b = 0u;
+      if (i0 + r < m)
+        for (int l = tx; l < k; l += 32) b = max(b, mag_bits(L[l + (int64_t)(i0 + r) * ld]));
+      b = __reduce_max_sync(0xffffffffu, b);
+      if (tx == 0) s_max[r] = b;
     }
   }
-  __syncthreads();
-  const int64_t Kr = 2 * (int64_t)k;
-  for (int r = threadIdx.y; r < 32; r += 8) {
-    const int i = i0 + r, l = l0 + tx;
-    if (i >= m || l >= k) continue;
-    const float2 z = t[tx][r];
-    const float v[4] = {z.x, -z.y, z.y, z.x};  // rows 2i and 2i + 1, columns 2l and 2l + 1
-    float h[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      uint32_t u;
-      asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(v[q]));
-      h[q] = __uint_as_float(u);
+  for (int l0 = 0; l0 < Kp / 2; l0 += 32) {
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8) {
+      if (!tr) {
+        const int i = i0 + tx, l = l0 + r;
+        t[r][tx] = (i < m && l < k) ? L[i + (int64_t)l * ld] : make_float2(0.f, 0.f);
+      } else {
+        const int l = l0 + tx, i = i0 + r;
+        t[tx][r] = (i < m && l < k) ? L[l + (int64_t)i * ld] : make_float2(0.f, 0.f);
+      }
     }
-    const int64_t p0 = (2 * (int64_t)i) * Kr + 2 * l, p1 = p0 + Kr;
-    *reinterpret_cast<float2 *>(hi + p0) = make_float2(h[0], h[1]);
-    *reinterpret_cast<float2 *>(hi + p1) = make_float2(h[2], h[3]);
-    *reinterpret_cast<float2 *>(lo + p0) = make_float2(v[0] - h[0], v[1] - h[1]);
-    *reinterpret_cast<float2 *>(lo + p1) = make_float2(v[2] - h[2], v[3] - h[3]);
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8) {
+      const int i = i0 + r, l = l0 + tx;
+      if (i >= m || 2 * l >= Kp) continue;
+      float inv;
+      const float sc = scale_of(s_max[r], &inv);
+      const float2 z = t[tx][r];
+      if (l == 0) rinv[i] = inv;
+      __half2 h, g;  // (re, im): rows 2i and 2i + 1 hold (re, -im) and (im, re)
+      split_half(z.x * sc, &h.x, &g.x);
+      split_half(z.y * sc, &h.y, &g.y);
+      const int64_t p0 = (2 * (int64_t)i) * Kp + 2 * l, p1 = p0 + Kp;
+      *reinterpret_cast<__half2 *>(hi + p0) = __halves2half2(h.x, __hneg(h.y));
+      *reinterpret_cast<__half2 *>(hi + p1) = __halves2half2(h.y, h.x);
+      *reinterpret_cast<__half2 *>(lo + p0) = __halves2half2(g.x, __hneg(g.y));
+      *reinterpret_cast<__half2 *>(lo + p1) = __halves2half2(g.y, g.x);
+    }
   }
 }
 
-// B_hi / B_lo (Nc x Kr, K contiguous) from the complex block U (k x nc, ld).
-__global__ void split_b_kernel(const float2 *U, int64_t ld, int k, int nc, float *hi, float *lo) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)k * nc) return;
-  const int l = (int)(idx % k), j = (int)(idx / k);
-  const float2 z = U[l + (int64_t)j * ld];
-  const int64_t base = (int64_t)j * 2 * k + 2 * l;
-  const float vals[2] = {z.x, z.y};
-#pragma unroll
-  for (int q = 0; q < 2; q++) {
-    uint32_t h;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(vals[q]));
-    const float hf = __uint_as_float(h);
-    hi[base + q] = hf;
-    lo[base + q] = vals[q] - hf;
+// B_hi / B_lo (nc x Kp halves, K contiguous) from the complex block U (k x nc,
+// ld) and the columns' inverse scales: one warp per column.
+__global__ void __launch_bounds__(256) split_b_kernel(const float2 *U, int64_t ld, int k, int nc, int Kp, __half *hi,
+                                                      __half *lo, float *cinv) {
+  const int lane = threadIdx.x & 31, j = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (j >= nc) return;
+  const float2 *u = U + (int64_t)j * ld;
+  unsigned b = 0u;
+  for (int l = lane; l < k; l += 32) b = max(b, mag_bits(u[l]));
+  float inv;
+  const float sc = scale_of(__reduce_max_sync(0xffffffffu, b), &inv);
+  if (lane == 0) cinv[j] = inv;
+  for (int l = lane; l < Kp / 2; l += 32) {
+    const float2 z = l < k ? u[l] : make_float2(0.f, 0.f);
+    __half2 h, g;
+    split_half(z.x * sc, &h.x, &g.x);
+    split_half(z.y * sc, &h.y, &g.y);
+    reinterpret_cast<__half2 *>(hi + (int64_t)j * Kp)[l] = h;
+    reinterpret_cast<__half2 *>(lo + (int64_t)j * Kp)[l] = g;
   }
 }
 
@@ -357,54 +425,69 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// 2-D FP32 tensor map over a row-major rows x cols matrix (cols contiguous),
-// box = 32 columns (128 bytes) x box_rows rows, 128-byte swizzle.
-int make_map(Ctx *c, CUtensorMap *m, const float *base, int64_t rows, int64_t cols, int box_rows) {
+// 2-D FP16 tensor map over a row-major rows x cols matrix (cols contiguous),
+// box = 32 columns (64 bytes) x box_rows rows, 64-byte swizzle.
+int make_map(Ctx *c, CUtensorMap *m, const __half *base, int64_t rows, int64_t cols, int box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(c, MOM_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)(cols * sizeof(float))};
+  cuuint64_t strides[1] = {(cuuint64_t)(cols * sizeof(__half))};
   cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(c, MOM_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
   return MOM_OK;
 }
 
+// Real K of the expanded operands: 2 k padded with zeros to whole K blocks.
+int padded_k(int k) { return (2 * k + kBK - 1) / kBK * kBK; }
+size_t up256(size_t b) { return (b + 255) / 256 * 256; }
+
 }  // namespace
 
-// C (m x nc complex FP32, ldc) -= L (m x k, ldl) * U (k x nc, ldu) with the
-// 3xTF32 tensor-core kernel.  m must be a multiple of 64, k of 16.
-// work: >= (4 m k + 4 k nc) * 4 bytes of device scratch.  max_ctas > 0
-// caps the persistent grid.  reuse_a: work already holds the expansion of
-// this L (the previous call on the same stream had the same L, m and k).
-// trans_l: L is given as its k x m transpose at L (ld ldl).
+// C (m x nc complex FP32, ldc) -= L (m x k, ldl) * U (k x nc, ldu) on the
+// tensor cores (two FP16 parts per operand, FP32-accurate).  m must be a
+// multiple of 64, k of 16.  work: tc_cgemm_work_bytes(m, nc, k) of device
+// scratch.  max_ctas > 0 caps the persistent grid.  reuse_a: work already holds
+// the expansion of this L (the previous call on the same stream had the same L,
+// m and k).  trans_l: L is given as its k x m transpose at L (ld ldl).
 int tc_cgemm_update(Ctx *c, float2 *C, int64_t ldc, const float2 *L, int64_t ldl, const float2 *U, int64_t ldu, int m,
                     int nc, int k, float *work, int *err, int max_ctas, bool reuse_a, bool trans_l) {
   if (m <= 0 || nc <= 0 || k <= 0) return MOM_OK;
-  if ((2 * m) % kBM != 0 || (2 * k) % kBK != 0) return fail(c, MOM_ERR_ARG, "tc_cgemm_update: unsupported shape");
-  const int Mr = 2 * m, Kr = 2 * k;
-  float *ahi = work, *alo = ahi + (size_t)Mr * Kr, *bhi = alo + (size_t)Mr * Kr, *blo = bhi + (size_t)nc * Kr;
+  if ((2 * m) % kBM != 0 || (2 * k) % 32 != 0) return fail(c, MOM_ERR_ARG, "tc_cgemm_update: unsupported shape");
+  const int Mr = 2 * m, Kp = padded_k(k);
+  char *w = reinterpret_cast<char *>(work);
+  auto take = [&](size_t bytes) {
+    char *p = w;
+    w += up256(bytes);
+    return p;
+  };
+  // the expansion of L first: its place must not depend on nc (reuse_a)
+  __half *ahi = (__half *)take(sizeof(__half) * (size_t)Mr * Kp), *alo = (__half *)take(sizeof(__half) * (size_t)Mr * Kp);
+  float *rinv = (float *)take(sizeof(float) * m);
+  __half *bhi = (__half *)take(sizeof(__half) * (size_t)nc * Kp), *blo = (__half *)take(sizeof(__half) * (size_t)nc * Kp);
+  float *cinv = (float *)take(sizeof(float) * nc);
   if (!reuse_a) {
-    expand_a_tiled_kernel<<<dim3((unsigned)((k + 31) / 32), (unsigned)((m + 31) / 32)), dim3(32, 8), 0, c->stream>>>(
-        L, ldl, m, k, ahi, alo, trans_l);
+    expand_a_kernel<<<(unsigned)((m + 31) / 32), dim3(32, 8), 0, c->stream>>>(L, ldl, m, k, Kp, ahi, alo, rinv, trans_l);
     c->launches++;
   }
-  split_b_kernel<<<(unsigned)(((int64_t)k * nc + 255) / 256), 256, 0, c->stream>>>(U, ldu, k, nc, bhi, blo);
+  split_b_kernel<<<(unsigned)((nc + 7) / 8), 256, 0, c->stream>>>(U, ldu, k, nc, Kp, bhi, blo, cinv);
   c->launches++;
   CUtensorMap mAhi, mAlo, mBhi, mBlo;
-  MOM_TRY(make_map(c, &mAhi, ahi, Mr, Kr, kBM));
-  MOM_TRY(make_map(c, &mAlo, alo, Mr, Kr, kBM));
-  MOM_TRY(make_map(c, &mBhi, bhi, nc, Kr, kBN));
-  MOM_TRY(make_map(c, &mBlo, blo, nc, Kr, kBN));
+  MOM_TRY(make_map(c, &mAhi, ahi, Mr, Kp, kBM));
+  MOM_TRY(make_map(c, &mAlo, alo, Mr, Kp, kBM));
+  MOM_TRY(make_map(c, &mBhi, bhi, nc, Kp, kBN));
+  MOM_TRY(make_map(c, &mBlo, blo, nc, Kp, kBN));
   TcArgs ta;
   ta.C = reinterpret_cast<float *>(C);
   ta.ldc = 2 * ldc;
   ta.Mr = Mr;
   ta.Nc = nc;
-  ta.Kr = Kr;
+  ta.Kp = Kp;
+  ta.rinv = rinv;
+  ta.cinv = cinv;
   ta.err = err;
   ta.spin = wait_polls(c, 1);
   const int ntiles = (Mr / kBM) * ((nc + kBN - 1) / kBN);
@@ -418,7 +501,7 @@ int tc_cgemm_update(Ctx *c, float2 *C, int64_t ldc, const float2 *L, int64_t ldl
     tc_gemm_kernel<<<grid, kTcThreads, smem, c->stream>>>(mAhi, mAlo, mBhi, mBlo, ta);
   }
   c->launches++;
-  c->tc_flops += 6.0 * Mr * (double)nc * Kr;  // three TF32 passes, 2 FLOP per real MAC
+  c->tc_flops += 6.0 * Mr * (double)nc * 2 * k;  // three passes, 2 FLOP per real MAC
   MOM_CUDA(c, cudaGetLastError());
   return MOM_OK;
 }
@@ -429,7 +512,11 @@ int tc_init_kernels(Ctx *c) {
   return MOM_OK;
 }
 
-size_t tc_cgemm_work_bytes(int m, int nc, int k) { return ((size_t)8 * m * k + (size_t)4 * k * nc) * sizeof(float); }
+size_t tc_cgemm_work_bytes(int m, int nc, int k) {
+  const size_t Kp = padded_k(k);
+  return 2 * up256(sizeof(__half) * 2 * (size_t)m * Kp) + up256(sizeof(float) * m) +
+         2 * up256(sizeof(__half) * (size_t)nc * Kp) + up256(sizeof(float) * nc);
+}
 
 }  // namespace mom
 

@@ -36,8 +36,9 @@ extern "C" {
 
 /* Arithmetic of sysmat / solve. */
 #define MOM_PREC_FP64 0  /* FP64 assembly and FP64 LU (the reference's arithmetic) */
-#define MOM_PREC_MIXED 1 /* FP32 far pairs + FP64 near pairs; FP32 LU with TF32
-                            tensor-core trailing updates; FP64 refinement */
+#define MOM_PREC_MIXED 1 /* FP32 far pairs + FP64 near pairs; FP32 LU with
+                            FP32-accurate tensor-core trailing updates; FP64
+                            refinement */
 
 /* Boundary types of mesh edges (mesh.f90:16-25): the symmetry planes. */
 #define MOM_BND_NONE 1
