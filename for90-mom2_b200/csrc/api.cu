@@ -407,9 +407,11 @@ int mom_gpu_create(int32_t device, mom_ctx **out) {
   }
   // A fixed cuBLAS workspace (no allocation inside the captured LU graph);
   // the look-ahead stream has its own handle and workspace.
-  bool ok = cudaMalloc(&c->blas_ws, kBlasWorkspace) == cudaSuccess &&
+  int low = 0, high = 0;  // the look-ahead panels go before the updates beside them
+  bool ok = cudaDeviceGetStreamPriorityRange(&low, &high) == cudaSuccess &&
+            cudaMalloc(&c->blas_ws, kBlasWorkspace) == cudaSuccess &&
             cublasSetWorkspace(c->blas, c->blas_ws, kBlasWorkspace) == CUBLAS_STATUS_SUCCESS &&
-            cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking) == cudaSuccess &&
+            cudaStreamCreateWithPriority(&c->stream2, cudaStreamNonBlocking, high) == cudaSuccess &&
             cublasCreate(&c->blas2) == CUBLAS_STATUS_SUCCESS &&
             cublasSetStream(c->blas2, c->stream2) == CUBLAS_STATUS_SUCCESS &&
             cudaMalloc(&c->blas_ws2, kBlasWorkspace) == cudaSuccess &&
@@ -432,8 +434,6 @@ int mom_gpu_create(int32_t device, mom_ctx **out) {
   c->use_graph = !(eg && eg[0] == '0');
   const char *ea = std::getenv("MOM_AUTOTUNE");
   c->autotune = !(ea && ea[0] == '0');
-  const char *et = std::getenv("MOM_SMALL_TC");
-  if (et) c->small_tc = et[0] != '0';
   const char *eo = std::getenv("MOM_LU_OUTER");
   if (eo) c->outer_panels = std::max(1, std::min(16, std::atoi(eo)));
   const char *ep = std::getenv("MOM_PANEL_CTAS");
@@ -454,8 +454,6 @@ int mom_gpu_create(int32_t device, mom_ctx **out) {
   if (ae) c->adj_eps_plain = std::atoi(ae) != 0;
   const char *av = std::getenv("MOM_ADJ_VERTEX_PLAIN");
   if (av) c->adj_vertex_reverse = std::atoi(av) != 0;
-  const char *ft = std::getenv("MOM_FUSED_TRSM");
-  if (ft) c->fused_trsm = std::max(0, std::min(2, std::atoi(ft)));
   *out = c;
   return MOM_OK;
 }
@@ -637,17 +635,7 @@ int mom_gpu_solve(mom_ctx *c, int32_t precision, double tol, int32_t maxit, doub
   MOM_CUDA(c, cudaSetDevice(c->device));
   // one factorisation and solve per representation (solve_systems, solver.f90:325-357)
   int it = 0;
-  if (c->factored != precision) {
-    for (int r = 0; r < c->nga; r++) {
-      select_rep(c, r);
-      const int rc = lu_factor(c, precision);
-      if (rc != MOM_OK) {
-        select_rep(c, 0);
-        c->factored = -1;
-        return rc;
-      }
-    }
-  }
+  if (c->factored != precision) MOM_TRY(lu_factor_reps(c, precision));
   for (int r = 0; r < c->nga; r++) {
     select_rep(c, r);
     int itr = 0;

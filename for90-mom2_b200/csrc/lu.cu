@@ -541,11 +541,15 @@ __device__ __forceinline__ void join_level(int t, const double2 *D, double2 *XL,
 // CTA b inverts the diagonal block kb = kb0 + b (rows and columns 64 kb ..)
 // of the factors in A: inv(L11) into invd[kb][0] (and FP32 into
 // invL32[kb]), inv(U11) into invd[kb][1], for the triangles TRI selects.
+// blockIdx.y selects one of several matrices, batch_A and batch_inv apart.
 template <typename T, int TRI>
 __global__ void __launch_bounds__(kDiagThreads) diag_inv_kernel(const T *A, int64_t lda, int kb0, double2 *invd,
-                                                                float2 *invL32) {
+                                                                float2 *invL32, int64_t batch_A = 0,
+                                                                int64_t batch_inv = 0) {
   extern __shared__ double2 sm[];
   constexpr int nb = kDiagNb, nn = kDiagNb * kDiagNb;
+  A += blockIdx.y * batch_A;
+  invd += blockIdx.y * batch_inv;
   const int kb = kb0 + blockIdx.x;
   const int64_t j0 = (int64_t)kb * nb;
   double2 *invL = invd + (size_t)kb * 2 * nn, *invU = invL + nn;
@@ -1106,83 +1110,9 @@ __global__ void axpy_kernel(double2 *X, const double2 *D, int64_t count) {
   }
 }
 
-// U12 of an outer block in one launch: B <- inv(L11) B for the np panels'
-// rows [J0, J0 + np nb) and the columns [c0, c0 + ncol), L11 unit lower
-// triangular.  Per panel p: X_p = inv(L_pp) B_p with the diagonal block's
-// inverse (diag_inv_kernel), then B_q -= L_qp X_p for every panel q below.
-// One CTA per kBtCols columns keeps its np nb x kBtCols tile in shared
-// memory; the 64 x 64 factor blocks are staged one at a time.  FP32 complex
-// products with FP32 accumulation, as the library CGEMM it replaces.
-constexpr int kBtCols = 32;
-constexpr int kBtThreads = 256;
-constexpr int kBtMaxPanels = 4;
-constexpr int kBtLd = 65;             // padded row stride of the staged factor block
-constexpr int kBtLdB = kBtCols + 1;   // padded row stride of the column tile
-constexpr size_t kBtSmem = sizeof(float2) * ((size_t)kBtMaxPanels * 64 * kBtLdB + 64 * kBtLd);
-
-__global__ void __launch_bounds__(kBtThreads) block_trsm_kernel(float2 *A, int64_t lda, int64_t J0, int np,
-                                                                int64_t c0, int ncol, const float2 *invL) {
-  extern __shared__ float2 bt_smem[];
-  float2 *Bs = bt_smem;                                  // [np * 64][kBtLdB]
-  float2 *Ms = bt_smem + (size_t)kBtMaxPanels * 64 * kBtLdB;  // [64][kBtLd], row-major
-  const int t = threadIdx.x, j = t % kBtCols, rg = t / kBtCols;  // 8 rows per thread
-  const int jc = blockIdx.x * kBtCols;
-  const int rows = np * 64;
-  for (int idx = t; idx < rows * kBtCols; idx += kBtThreads) {
-    const int r = idx % rows, cc = idx / rows;
-    Bs[r * kBtLdB + cc] = (jc + cc < ncol) ? A[(J0 + r) + (c0 + jc + cc) * lda] : make_float2(0.f, 0.f);
-  }
-  for (int p = 0; p < np; p++) {
-    // X_p = inv(L_pp) B_p
-    __syncthreads();
-    const float2 *inv = invL + (size_t)p * 64 * 64;  // column-major 64 x 64
-    for (int idx = t; idx < 64 * 64; idx += kBtThreads) Ms[(idx % 64) * kBtLd + idx / 64] = inv[idx];
-    __syncthreads();
-    float2 acc[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) acc[r] = make_float2(0.f, 0.f);
-    for (int k = 0; k < 64; k++) {
-      const float2 b = Bs[(p * 64 + k) * kBtLdB + j];
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        const float2 m = Ms[(rg * 8 + r) * kBtLd + k];
-        acc[r].x = fmaf(m.x, b.x, fmaf(-m.y, b.y, acc[r].x));
-        acc[r].y = fmaf(m.x, b.y, fmaf(m.y, b.x, acc[r].y));
-      }
-    }
-    __syncthreads();  // every read of B_p done
-#pragma unroll
-    for (int r = 0; r < 8; r++) Bs[(p * 64 + rg * 8 + r) * kBtLdB + j] = acc[r];
-    // B_q -= L_qp X_p
-    for (int q = p + 1; q < np; q++) {
-      __syncthreads();
-      const float2 *L = A + (J0 + q * 64) + (J0 + p * 64) * lda;
-      for (int idx = t; idx < 64 * 64; idx += kBtThreads) Ms[(idx % 64) * kBtLd + idx / 64] = L[(idx % 64) + (idx / 64) * lda];
-      __syncthreads();
-#pragma unroll
-      for (int r = 0; r < 8; r++) acc[r] = make_float2(0.f, 0.f);
-      for (int k = 0; k < 64; k++) {
-        const float2 x = Bs[(p * 64 + k) * kBtLdB + j];
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-          const float2 m = Ms[(rg * 8 + r) * kBtLd + k];
-          acc[r].x = fmaf(m.x, x.x, fmaf(-m.y, x.y, acc[r].x));
-          acc[r].y = fmaf(m.x, x.y, fmaf(m.y, x.x, acc[r].y));
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        float2 &v = Bs[(q * 64 + rg * 8 + r) * kBtLdB + j];
-        v.x -= acc[r].x;
-        v.y -= acc[r].y;
-      }
-    }
-  }
-  __syncthreads();
-  for (int idx = t; idx < rows * kBtCols; idx += kBtThreads) {
-    const int r = idx % rows, cc = idx / rows;
-    if (jc + cc < ncol) A[(J0 + r) + (c0 + jc + cc) * lda] = Bs[r * kBtLdB + cc];
-  }
+__global__ void iota_kernel(int *p, int n, int count) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < count) p[i] = i % n;
 }
 
 struct LuWork {
@@ -1194,6 +1124,7 @@ struct LuWork {
   float *tcw;      // tensor-core GEMM operands (mixed path)
   int *pmap;       // [257]: composed panel permutation (dst[128], src[128], count)
   int *pmb;        // [2][16][260]: the composed permutations of every panel of an outer block, double-buffered
+  int *map;        // [2][kMaxGroup][256]: row moves of the cluster panels, double-buffered
   void *W2;        // nb x 16 nb workspace of the look-ahead stream's block TRSM
 };
 
@@ -1223,6 +1154,7 @@ int lu_workspace(Ctx *c, int precision, LuWork &w, int slot = -1) {
   const size_t o_i32 = take(sizeof(float2) * (size_t)nb * c->n);
   const size_t o_pm = take(sizeof(int) * 260);
   const size_t o_pmb = take(sizeof(int) * 260 * 2 * 16);
+  const size_t o_map = take(sizeof(int) * 256 * 2 * kMaxGroup);
   const size_t o_w2 = take(esz * (size_t)nb * 16 * nb);
   const size_t o_tc =
       take(precision == MOM_PREC_MIXED ? tc_cgemm_work_bytes((int)c->n, (int)c->n, c->outer_panels * nb) : 0);
@@ -1239,6 +1171,7 @@ int lu_workspace(Ctx *c, int precision, LuWork &w, int slot = -1) {
   w.tcw = (float *)(b + o_tc);
   w.pmap = (int *)(b + o_pm);
   w.pmb = (int *)(b + o_pmb);
+  w.map = (int *)(b + o_map);
   w.W2 = (void *)(b + o_w2);
   return MOM_OK;
 }
@@ -1286,7 +1219,10 @@ int launch_panel(Ctx *c, T *A, int64_t lda, int64_t n, int64_t j0, int P, int *i
   if (!st) st = c->stream;
   const int nb = c->nb;
   const int64_t m = n - j0;
-  if (on_cluster<T>(c, m)) return panel_reg(c, A, lda, n, j0, ipiv, info, w.timeout, st);
+  if (on_cluster<T>(c, m)) {
+    const PanelCall<T> p = {A, lda, n, j0, ipiv, info, w.timeout, nullptr, st, 1, 0, 0, 0};
+    return panel_reg<T>(c, p, false);
+  }
   const int rpc = (int)((m + P - 1) / P);
   P = (int)((m + rpc - 1) / rpc);
   const size_t smem = sizeof(typename SlabOf<T>::type) * (size_t)nb * rpc;
@@ -1342,13 +1278,8 @@ int lu_enqueue(Ctx *c, T *A, int precision, const LuWork &w) {
     }
     return MOM_OK;
   };
-  // C(m x ncol) -= L(m x nb) U(nb x ncol): the rank-64 updates; on the
-  // tensor cores in the mixed path, as the trailing update
+  // C(m x ncol) -= L(m x nb) U(nb x ncol): the rank-64 updates
   auto update64 = [&](int64_t m, int64_t ncol, const T *Lm, const T *Um, T *Cm) -> int {
-    if (m <= 0 || ncol <= 0) return MOM_OK;
-    if (mixed && c->small_tc)
-      return tc_cgemm_update(c, reinterpret_cast<float2 *>(Cm), lda, reinterpret_cast<const float2 *>(Lm), lda,
-                             reinterpret_cast<const float2 *>(Um), lda, (int)m, (int)ncol, nb, w.tcw, c->dinfo + 2);
     return gemm(m, ncol, nb, -1.0, Lm, lda, Um, lda, 1.0, Cm, lda);
   };
   // B(nb x ncol, at A + j0 + col*lda) <- inv(L_jj) B, through the workspace
@@ -1447,9 +1378,11 @@ int lu_enqueue(Ctx *c, T *A, int precision, const LuWork &w) {
 //             TRSM and update of J on the next block's columns (L), then
 //             record eL; the same on the rest (R), its tensor-core GEMM on
 //             fewer SMs; then wait for eF;
-//   stream 2: wait eL; factor block J+1 (panels, interchanges inside the
-//             block only, diagonal inverses, in-block TRSM and updates on its
-//             own cuBLAS handle); record eF.
+//   stream 2: wait eL; factor block J+1 (panels, interchanges, TRSM and updates
+//             inside the block only, on its own cuBLAS handle); record eF.
+// The panels run on one cluster where they all fit (lu_panel.cu, with the
+// interchanges and TRSMs of swap_trsm), else on CTAs that exchange through
+// global memory, with TRSMs by the inverses of the diagonal blocks.
 // Interchanges commute with the row-wise trailing update, so applying a
 // block's interchanges to the columns outside it after its factorisation
 // (instead of panel by panel) gives the same factors; the columns left of
@@ -1488,44 +1421,48 @@ int lu_enqueue_la(Ctx *c, T *A, const LuWork &w) {
     return MOM_OK;
   };
   // factor the outer block at J0 on stream st (panel CTAs capped at pcap > 0)
+  const bool cl = on_cluster<T>(c, n);
+  auto call = [&](int64_t j0, cudaStream_t st, bool swaps) {
+    return PanelCall<T>{A, lda, n, j0, c->ipiv, w.info, w.timeout, swaps ? w.map + 256 * ((j0 / nb) & 1) : nullptr, st, 1,
+                        0, 0, 0};
+  };
   auto factor_block = [&](int64_t J0, cudaStream_t st, cublasHandle_t h, int *pm, int pcap) -> int {
     const int64_t NBc = std::min<int64_t>(NB, n - J0);
     for (int64_t j0 = J0; j0 < J0 + NBc; j0 += nb) {
       const int p = (int)((j0 - J0) / nb), kb = (int)(j0 / nb);
-      const int64_t m = n - j0;
-      int P = panel_ctas(c, m, kPanelMaxRows<T>);
-      if (pcap > 0) P = (int)std::max<int64_t>(std::min(P, pcap), (m + kPanelMaxRows<T> - 1) / kPanelMaxRows<T>);
-      {
-        ProfScope ps(c, kProfPanel, st);
-        MOM_TRY(launch_panel<T>(c, A, lda, n, j0, P, c->ipiv, w.info, w, st));
-      }
-      {
+      const int64_t m = n - j0, rest = J0 + NBc - (j0 + nb);
+      int *mp = pm + 260 * p;
+      if (cl) {
+        {
+          ProfScope ps(c, kProfPanel, st);
+          MOM_TRY(panel_reg<T>(c, call(j0, st, true), pcap > 0));
+        }
         ProfScope pz(c, kProfPivotAux, st);
-        int *mp = pm + 260 * p;
-        pivot_map_kernel<<<1, 32, 0, st>>>(c->ipiv, j0, nb, mp, mp + 128, mp + 256);
-        if (NBc > nb)
-          laswp_range_kernel<T><<<(unsigned)((NBc * 32 + 255) / 256), 256, 0, st>>>(A, lda, J0, NBc, j0, nb, mp,
-                                                                                      mp + 128, mp + 256);
-        c->launches += NBc > nb ? 2 : 1;
-      }
-      {
+        MOM_TRY(swap_trsm<T>(c, call(j0, st, true), j0 + nb, j0 + nb + rest, J0, j0, c->perm, mp));
+      } else {
+        int P = panel_ctas(c, m, kPanelMaxRows<T>);
+        if (pcap > 0) P = (int)std::max<int64_t>(std::min(P, pcap), (m + kPanelMaxRows<T> - 1) / kPanelMaxRows<T>);
+        {
+          ProfScope ps(c, kProfPanel, st);
+          MOM_TRY(launch_panel<T>(c, A, lda, n, j0, P, c->ipiv, w.info, w, st));
+        }
+        {
+          ProfScope pz(c, kProfPivotAux, st);
+          pivot_map_kernel<<<1, 32, 0, st>>>(c->ipiv, j0, nb, mp, mp + 128, mp + 256);
+          if (NBc > nb)
+            laswp_range_kernel<T><<<(unsigned)((NBc * 32 + 255) / 256), 256, 0, st>>>(A, lda, J0, NBc, j0, nb, mp,
+                                                                                        mp + 128, mp + 256);
+          c->launches += NBc > nb ? 2 : 1;
+        }
         ProfScope pd(c, kProfDiagInv, st);
         diag_inv_kernel<T, 0><<<1, kDiagThreads, sizeof(double2) * (3 * nb * nb + nb), st>>>(A, lda, kb, c->invd,
                                                                                               w.invL32);
         c->launches++;
         MOM_CUDA(c, cudaGetLastError());
+        if (rest > 0) MOM_TRY(trsm_l(h, st, (T *)w.W2, j0, j0 + nb, rest));
       }
-      const int64_t rest = J0 + NBc - (j0 + nb);
       if (rest > 0) {
         ProfScope pg(c, kProfGemm, st);
-        if (c->fused_trsm != 0 && nb == 64) {
-          block_trsm_kernel<<<(unsigned)((rest + kBtCols - 1) / kBtCols), kBtThreads, kBtSmem, st>>>(
-              reinterpret_cast<float2 *>(A), lda, j0, 1, j0 + nb, (int)rest, w.invL32 + (size_t)kb * nb * nb);
-          c->launches++;
-          MOM_CUDA(c, cudaGetLastError());
-        } else {
-          MOM_TRY(trsm_l(h, st, (T *)w.W2, j0, j0 + nb, rest));
-        }
         MOM_TRY(gemm(h, n - j0 - nb, rest, nb, -1.0f, A + (j0 + nb) + j0 * lda, lda, A + j0 + (j0 + nb) * lda, lda,
                      1.0f, A + (j0 + nb) + (j0 + nb) * lda, lda));
       }
@@ -1539,19 +1476,12 @@ int lu_enqueue_la(Ctx *c, T *A, const LuWork &w) {
     if (ncol <= 0) return MOM_OK;
     const int64_t NBc = std::min<int64_t>(NB, n - J0), t0 = J0 + NBc;
     ProfScope pg(c, kProfGemm);
-    if ((c->fused_trsm == 1 || (c->fused_trsm == 2 && ncol <= NB)) && NBc <= (int64_t)kBtMaxPanels * nb &&
-        nb == 64) {
-      block_trsm_kernel<<<(unsigned)((ncol + kBtCols - 1) / kBtCols), kBtThreads, kBtSmem, sa>>>(
-          reinterpret_cast<float2 *>(A), lda, J0, (int)(NBc / nb), c0, (int)ncol, w.invL32 + (size_t)(J0 / nb) * nb * nb);
-      c->launches++;
-      MOM_CUDA(c, cudaGetLastError());
-    } else {
-      for (int64_t j0 = J0; j0 < t0; j0 += nb) {
-        MOM_TRY(trsm_l(c->blas, sa, (T *)w.W, j0, c0, ncol));
-        const int64_t below = t0 - (j0 + nb);
-        MOM_TRY(gemm(c->blas, below, ncol, nb, -1.0f, A + (j0 + nb) + j0 * lda, lda, A + j0 + c0 * lda, lda, 1.0f,
-                     A + (j0 + nb) + c0 * lda, lda));
-      }
+    for (int64_t j0 = J0; j0 < t0; j0 += nb) {
+      if (cl) MOM_TRY(swap_trsm<T>(c, call(j0, sa, false), c0, c0 + ncol, 0, 0, nullptr));
+      else MOM_TRY(trsm_l(c->blas, sa, (T *)w.W, j0, c0, ncol));
+      const int64_t below = t0 - (j0 + nb);
+      MOM_TRY(gemm(c->blas, below, ncol, nb, -1.0f, A + (j0 + nb) + j0 * lda, lda, A + j0 + c0 * lda, lda, 1.0f,
+                   A + (j0 + nb) + c0 * lda, lda));
     }
     MOM_TRY(tc_cgemm_update(c, reinterpret_cast<float2 *>(A + t0 + c0 * lda), lda,
                             reinterpret_cast<const float2 *>(A + t0 + J0 * lda), lda,
@@ -1559,6 +1489,10 @@ int lu_enqueue_la(Ctx *c, T *A, const LuWork &w) {
                             (int)NBc, w.tcw, c->dinfo + 2, gemm_ctas, reuse_a));
     return MOM_OK;
   };
+  if (cl) {
+    iota_kernel<<<(unsigned)((n + 255) / 256), 256, 0, sa>>>(c->perm, (int)n, (int)n);
+    c->launches++;
+  }
   // stream 2 joins the stream (and any capture open on it)
   MOM_CUDA(c, cudaEventRecord(c->la_ev[0], sa));
   MOM_CUDA(c, cudaStreamWaitEvent(sb, c->la_ev[0], 0));
@@ -1614,6 +1548,11 @@ int lu_enqueue_la(Ctx *c, T *A, const LuWork &w) {
   MOM_CUDA(c, cudaStreamWaitEvent(sa, c->la_ev[2], 0));
   {
     ProfScope pd(c, kProfDiagInv);
+    if (cl) {
+      diag_inv_kernel<T, 0><<<(unsigned)(n / nb), kDiagThreads, sizeof(double2) * (3 * nb * nb + nb), sa>>>(
+          A, lda, 0, c->invd, nullptr);
+      c->launches++;
+    }
     diag_inv_kernel<T, 1><<<(unsigned)(n / nb), kDiagThreads, sizeof(double2) * (3 * nb * nb + nb), sa>>>(
         A, lda, 0, c->invd, nullptr);
     c->launches++;
@@ -1622,28 +1561,156 @@ int lu_enqueue_la(Ctx *c, T *A, const LuWork &w) {
     c->launches++;
     MOM_CUDA(c, cudaGetLastError());
   }
-  compose_pivots_kernel<<<1, 256, sizeof(int) * n, sa>>>(c->ipiv, (int)n, c->perm);
-  c->launches++;
+  if (!cl) {
+    compose_pivots_kernel<<<1, 256, sizeof(int) * n, sa>>>(c->ipiv, (int)n, c->perm);
+    c->launches++;
+  }
   MOM_CUDA(c, cudaGetLastError());
   return MOM_OK;
 }
 
+// From this order on the FP32 trailing updates run on the tensor cores (whole
+// mixed calls, tensor cores against library FP32 GEMMs: 2,160 unknowns 4.96 and
+// 5.05 ms, 2,940 6.8 and 7.1 ms, 4,860 12.6 and 16.2 ms; no difference below).
+constexpr int64_t kTcFromOrder = 2048;
+// From this order on the FP32 factorisation goes by outer blocks of 256 columns
+// (lu_enqueue_la): its updates read and write the trailing matrix four times
+// less, which the 64-column updates are bound by.  Whole calls, 256 against 64
+// columns: 7,260 unknowns 25.4 and 24.3 ms, 8,640 33.0 and 33.7 ms, 11,760 56.9
+// and 67.3 ms.
+constexpr int64_t kOuterFromOrder = 8192;
+
+// The factorisation when every panel fits one thread-block cluster: right
+// looking by 64-column panels with look-ahead, for `batch` matrices of the same
+// order (the representations of a symmetry group) at once.
+//   stream 1: panel J's interchanges and U12 on the next panel's 64 columns and
+//             their update; then the same on the columns right of them (and
+//             the interchanges left of J) and the large update, beside
+//   stream 2: panel J+1, one launch on one cluster, so that it keeps its SMs.
+// A panel is a serial chain of 64 pivot decisions on 16 SMs (64-126 us); the
+// large update takes the other SMs, so whichever is longer hides the other.
+template <typename T>
+int lu_enqueue_cluster(Ctx *c, T *A, const LuWork &w, int batch) {
+  const int64_t n = c->n, lda = c->lda, mat = lda * n;
+  const int nb = c->nb;
+  constexpr bool f32 = sizeof(T) == sizeof(float2);
+  cudaStream_t sa = c->stream, sb = c->stream2;
+  MOM_CUDA(c, cudaMemsetAsync(c->dinfo, 0, sizeof(int) * 4, sa));
+  MOM_BLAS(c, cublasSetMathMode(c->blas, CUBLAS_DEFAULT_MATH));
+  iota_kernel<<<(unsigned)((n * batch + 255) / 256), 256, 0, sa>>>(c->perm, (int)n, (int)(n * batch));
+  c->launches++;
+  auto call = [&](int64_t j0, cudaStream_t st) {
+    return PanelCall<T>{A, lda, n, j0, c->ipiv, w.info, w.timeout, w.map + 256 * kMaxGroup * ((j0 / nb) & 1), st, batch,
+                        mat, n, 256};
+  };
+  auto panel = [&](int64_t j0, cudaStream_t st, bool beside) -> int {
+    ProfScope ps(c, kProfPanel, st);
+    return panel_reg<T>(c, call(j0, st), beside);
+  };
+  auto swaps = [&](int64_t j0, int64_t r0, int64_t r1, int64_t l1, int *perm) -> int {
+    ProfScope ps(c, kProfPivotAux);
+    return swap_trsm<T>(c, call(j0, sa), r0, r1, 0, l1, perm);
+  };
+  // A22 -= L21 U12 on the columns [c0, c1) right of panel j0
+  auto update = [&](int64_t j0, int64_t c0, int64_t c1, int ctas, bool reuse) -> int {
+    const int64_t r0 = j0 + nb, m = n - r0, nc = c1 - c0;
+    if (m <= 0 || nc <= 0) return MOM_OK;
+    ProfScope ps(c, kProfGemm);
+    T *Lm = A + r0 + j0 * lda, *Um = A + j0 + c0 * lda, *Cm = A + r0 + c0 * lda;
+    if constexpr (f32) {
+      if (batch == 1 && n >= kTcFromOrder && nc > nb)
+        return tc_cgemm_update(c, Cm, lda, Lm, lda, Um, lda, (int)m, (int)nc, nb, w.tcw, c->dinfo + 2, ctas, reuse);
+      c->blas_calls++;
+      const cuComplex al = make_cuComplex(-1.0f, 0), be = make_cuComplex(1.0f, 0);
+      MOM_BLAS(c, cublasCgemmStridedBatched(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)m, (int)nc, nb, &al,
+                                            (const cuComplex *)Lm, (int)lda, mat, (const cuComplex *)Um, (int)lda, mat,
+                                            &be, (cuComplex *)Cm, (int)lda, mat, batch));
+    } else {
+      c->blas_calls++;
+      const cuDoubleComplex al = make_cuDoubleComplex(-1.0, 0), be = make_cuDoubleComplex(1.0, 0);
+      MOM_BLAS(c, cublasZgemmStridedBatched(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)m, (int)nc, nb, &al,
+                                            (const cuDoubleComplex *)Lm, (int)lda, mat, (const cuDoubleComplex *)Um,
+                                            (int)lda, mat, &be, (cuDoubleComplex *)Cm, (int)lda, mat, batch));
+    }
+    return MOM_OK;
+  };
+  // stream 2 joins the stream (and any capture open on it)
+  MOM_CUDA(c, cudaEventRecord(c->la_ev[0], sa));
+  MOM_CUDA(c, cudaStreamWaitEvent(sb, c->la_ev[0], 0));
+  MOM_TRY(panel(0, sa, false));
+  for (int64_t j0 = 0; j0 < n; j0 += nb) {
+    const int64_t t0 = j0 + nb;
+    if (t0 >= n) {
+      MOM_TRY(swaps(j0, 0, 0, j0, c->perm));
+      break;
+    }
+    if (c->lookahead && t0 + nb < n) {
+      MOM_TRY(swaps(j0, t0, t0 + nb, 0, nullptr));
+      MOM_TRY(update(j0, t0, t0 + nb, 0, false));
+      MOM_CUDA(c, cudaEventRecord(c->la_ev[1], sa));
+      MOM_CUDA(c, cudaStreamWaitEvent(sb, c->la_ev[1], 0));
+      MOM_TRY(panel(t0, sb, true));
+      MOM_CUDA(c, cudaEventRecord(c->la_ev[2], sb));
+      MOM_TRY(swaps(j0, t0 + nb, n, j0, c->perm));
+      MOM_TRY(update(j0, t0 + nb, n, std::max(8, c->nsm - c->panel_cluster), false));
+      MOM_CUDA(c, cudaStreamWaitEvent(sa, c->la_ev[2], 0));
+    } else {
+      MOM_TRY(swaps(j0, t0, n, j0, c->perm));
+      MOM_TRY(update(j0, t0, n, 0, false));
+      MOM_TRY(panel(t0, sa, false));
+    }
+  }
+  // stream 2 rejoins stream 1 (closes any capture branch it holds)
+  MOM_CUDA(c, cudaEventRecord(c->la_ev[2], sb));
+  MOM_CUDA(c, cudaStreamWaitEvent(sa, c->la_ev[2], 0));
+  {
+    // the inverses of every diagonal block, which the solves need
+    ProfScope pd(c, kProfDiagInv);
+    const dim3 grid((unsigned)(n / nb), batch);
+    const size_t smem = sizeof(double2) * (3 * nb * nb + nb);
+    const int64_t binv = 2 * (int64_t)nb * n;
+    diag_inv_kernel<T, 0><<<grid, kDiagThreads, smem, sa>>>(A, lda, 0, c->invd, nullptr, mat, binv);
+    diag_inv_kernel<T, 1><<<grid, kDiagThreads, smem, sa>>>(A, lda, 0, c->invd, nullptr, mat, binv);
+    c->launches += 2;
+    if (f32) {
+      inv_to_fp32_kernel<<<c->nsm * 4, 256, 0, sa>>>(c->invd, c->inv32, binv * batch);
+      c->launches++;
+    }
+    MOM_CUDA(c, cudaGetLastError());
+  }
+  return MOM_OK;
+}
+
+// The schedule in use: by the cluster panels when all of them fit one cluster.
+template <typename T>
+int lu_issue(Ctx *c, T *A, int precision, const LuWork &w, int batch);
+
 // The look-ahead schedule serves the mixed path (tensor-core trailing
 // updates) with at least two outer blocks.
 bool use_lookahead(const Ctx *c, int precision) {
-  return c->lookahead && precision == MOM_PREC_MIXED && !c->small_tc && c->outer_panels <= 16 &&
+  return c->lookahead && precision == MOM_PREC_MIXED && c->outer_panels <= 16 &&
          c->n > 2 * (int64_t)c->outer_panels * c->nb;
 }
 
 // Captures the factorisation of this precision into g (replacing what g held).
 template <typename T>
-int lu_capture(Ctx *c, T *A, int precision, const LuWork &w, Ctx::LuGraph &g, const std::vector<uintptr_t> &key) {
+int lu_issue(Ctx *c, T *A, int precision, const LuWork &w, int batch) {
+  // (with several matrices at once the 64-column updates fill the GPU)
+  const bool outer = batch == 1 && use_lookahead(c, precision) && c->n >= kOuterFromOrder;
+  if (on_cluster<T>(c, c->n) && !outer) return lu_enqueue_cluster<T>(c, A, w, batch);
+  if (batch != 1) return fail(c, MOM_ERR_ARG, "one matrix at a time without cluster panels");
+  return use_lookahead(c, precision) ? lu_enqueue_la<T>(c, A, w) : lu_enqueue<T>(c, A, precision, w);
+}
+
+template <typename T>
+int lu_capture(Ctx *c, T *A, int precision, const LuWork &w, int batch, Ctx::LuGraph &g,
+               const std::vector<uintptr_t> &key) {
   g.reset();
   const int64_t l0 = c->launches, b0 = c->blas_calls;
   const double f0 = c->tc_flops;
   MOM_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   c->capturing = true;
-  const int st = use_lookahead(c, precision) ? lu_enqueue_la<T>(c, A, w) : lu_enqueue<T>(c, A, precision, w);
+  const int st = lu_issue<T>(c, A, precision, w, batch);
   c->capturing = false;
   cudaGraph_t graph = nullptr;
   const cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
@@ -1673,7 +1740,7 @@ int lu_capture(Ctx *c, T *A, int precision, const LuWork &w, Ctx::LuGraph &g, co
 }
 
 template <typename T>
-int lu_factor_t(Ctx *c, T *A, int precision) {
+int lu_factor_t(Ctx *c, T *A, int precision, int batch) {
   const int64_t n = c->n;
   const int nb = c->nb;
   if (n % nb != 0) return fail(c, MOM_ERR_ARG, "matrix order must be a multiple of the panel width");
@@ -1694,8 +1761,9 @@ int lu_factor_t(Ctx *c, T *A, int precision) {
                                         (uintptr_t)c->dinfo,  (uintptr_t)c->nsm,   (uintptr_t)c->prof,
                                         (uintptr_t)tune_hash(c), (uintptr_t)c->outer_panels, (uintptr_t)c->inv32,
                                         (uintptr_t)wait_polls(c, 0), (uintptr_t)wait_polls(c, 1),
-                                        (uintptr_t)use_lookahead(c, precision), (uintptr_t)c->la_ctas,
-                                        (uintptr_t)(c->la_from * 1e6), (uintptr_t)c->fused_trsm};
+                                        (uintptr_t)use_lookahead(c, precision), (uintptr_t)c->lookahead,
+                                        (uintptr_t)batch,       (uintptr_t)c->panel_cluster, (uintptr_t)c->la_ctas,
+                                        (uintptr_t)(c->la_from * 1e6)};
     for (Ctx::LuGraph *h : c->lu_graphs)
       if (h->exec && h->key == key) g = h;
     if (!g) {
@@ -1707,7 +1775,7 @@ int lu_factor_t(Ctx *c, T *A, int precision) {
       }
       g = new Ctx::LuGraph();
       c->lu_graphs.push_back(g);
-      const int rc = lu_capture<T>(c, A, precision, w, *g, key);
+      const int rc = lu_capture<T>(c, A, precision, w, batch, *g, key);
       if (rc != MOM_OK) {
         delete g;
         c->lu_graphs.pop_back();
@@ -1719,7 +1787,7 @@ int lu_factor_t(Ctx *c, T *A, int precision) {
     c->blas_calls += g->blas_calls;
     c->tc_flops += g->tc_flops;
   } else {
-    MOM_TRY(use_lookahead(c, precision) ? lu_enqueue_la<T>(c, A, w) : lu_enqueue<T>(c, A, precision, w));
+    MOM_TRY(lu_issue<T>(c, A, precision, w, batch));
   }
   }
   int hinfo[3] = {0, 0, 0};
@@ -1834,6 +1902,7 @@ int lu_init_kernels(Ctx *c) {
   MOM_CUDA(c, set_smem(panel_kernel<double2>));
   MOM_CUDA(c, set_smem(panel_kernel<float2>));
   c->panel_cluster = panel_reg_max_cluster();
+  MOM_TRY(panel_init_kernels(c));
   const char *ec = std::getenv("MOM_PANEL_CLUSTER");
   if (ec) c->panel_cluster = std::max(0, std::min(c->panel_cluster, std::atoi(ec)));
   MOM_CUDA(c, set_smem(diag_inv_kernel<double2, 0>));
@@ -1841,7 +1910,6 @@ int lu_init_kernels(Ctx *c) {
   MOM_CUDA(c, set_smem(diag_inv_kernel<double2, 1>));
   MOM_CUDA(c, set_smem(diag_inv_kernel<float2, 1>));
   MOM_CUDA(c, set_smem(compose_pivots_kernel));
-  MOM_CUDA(c, cudaFuncSetAttribute(block_trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBtSmem));
   MOM_CUDA(c, set_smem(trsv_flow_kernel<double2, 1, false>));
   MOM_CUDA(c, set_smem(trsv_flow_kernel<double2, 2, false>));
   MOM_CUDA(c, set_smem(trsv_flow_kernel<double2, 4, false>));
@@ -1987,10 +2055,25 @@ int lu_autotune(Ctx *c, int precision) {
 
 }  // namespace
 
-int lu_factor(Ctx *c, int precision) {
+// The current representation's matrix, or `batch` of them from it on.
+static int lu_factor(Ctx *c, int precision, int batch) {
   MOM_TRY(lu_autotune(c, precision));
-  if (precision == MOM_PREC_MIXED) return lu_factor_t<float2>(c, c->A32, precision);
-  return lu_factor_t<double2>(c, c->A, precision);
+  if (precision == MOM_PREC_MIXED) return lu_factor_t<float2>(c, c->A32, precision, batch);
+  return lu_factor_t<double2>(c, c->A, precision, batch);
+}
+
+// Every representation's matrix: at once where the cluster panels serve the
+// order, else one after the other.
+int lu_factor_reps(Ctx *c, int precision) {
+  const bool at_once = precision == MOM_PREC_MIXED ? on_cluster<float2>(c, c->n) : on_cluster<double2>(c, c->n);
+  int rc = MOM_OK;
+  for (int r = 0; r < (at_once ? 1 : c->nga) && rc == MOM_OK; r++) {
+    select_rep(c, r);
+    rc = lu_factor(c, precision, at_once ? c->nga : 1);
+  }
+  select_rep(c, 0);
+  if (rc != MOM_OK) c->factored = -1;
+  return rc;
 }
 
 namespace {

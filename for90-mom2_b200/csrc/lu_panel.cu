@@ -45,13 +45,16 @@ constexpr int kPanelNb = 64;
 struct RegPanelArgs {
   void *A;
   int64_t lda;
-  int64_t c0;        // first column (and row) of the subpanel
-  int64_t j0;        // first column of the 64-column panel
-  int m;             // rows n - c0
-  int *ipiv;         // ipiv[c0 ..]: pivot rows (global, 0-based)
+  int64_t j0;        // first column (and row) of the 64-column panel
+  int m;             // rows n - j0
+  int s0, s1;        // subpanels [s0, s1) of W columns
+  int *ipiv;         // ipiv[j0 ..]: pivot rows (global, 0-based)
   int *info;         // first zero pivot (1-based), 0 if none
   int *timeout;      // set when a wait ran out
   long long spin;    // polls before a wait is declared timed out
+  int *map;          // [2][128] or null: the subpanels' row moves (from, to), rows from j0, 2 W per subpanel
+  // blockIdx.y selects one of several matrices of the same shape
+  int64_t batch_A, batch_piv, batch_map;
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -161,8 +164,13 @@ struct __align__(16) PanelMsg {
   alignas(16) E v[W];
 };
 
-// One cluster of gridDim.x CTAs of T threads; thread t of CTA b holds the rows
-// b T R + T r + t, r < R, of the subpanel (W columns each).
+// One cluster of gridDim.x CTAs of T threads per matrix.  Per subpanel thread t
+// of CTA b holds the rows b T R + T r + t, r < R, counted from the subpanel's
+// first row (W columns each).  With several subpanels in one launch the rows
+// of the next one, and the columns right of it, take the rank-W update of the
+// last one as they are loaded, so the cluster keeps its SMs for the whole panel
+// (beside a GEMM that would take them between launches).  What other CTAs of
+// the cluster wrote is read through L2 after a cluster barrier.
 template <typename E, int W, int R, int T>
 __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
   using Msg = PanelMsg<E, W>;
@@ -173,9 +181,9 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
   __shared__ unsigned s_wmag[2][kRegWarps];
   __shared__ __align__(8) unsigned long long s_bar[2];
   __shared__ E s_l11[W][W + 1];
+  __shared__ __align__(16) E s_u[kPanelNb - W][W];
   __shared__ int s_src[W], s_top[W];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, cta = blockIdx.x, CL = gridDim.x;
-  const int m = a.m;
   const unsigned bar0 = smem_u32(&s_bar[0]), bar1 = smem_u32(&s_bar[1]);
   const unsigned tx = (unsigned)(CL * sizeof(Msg));
   if (tid == 0) {
@@ -185,27 +193,15 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar0), "r"(tx) : "memory");
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar1), "r"(tx) : "memory");
   }
-  E *A = reinterpret_cast<E *>(a.A) + a.c0 + a.c0 * a.lda;
+  E *P = reinterpret_cast<E *>(a.A) + blockIdx.y * a.batch_A + a.j0 + a.j0 * a.lda;  // the panel's first entry
+  int *ipiv = a.ipiv + blockIdx.y * a.batch_piv + a.j0;
   E x[R][W];
   int pos[R];
   bool act[R];
-#pragma unroll
-  for (int r = 0; r < R; r++) {
-    pos[r] = cta * (T * R) + r * T + tid;
-    act[r] = pos[r] < m;
-  }
-#pragma unroll
-  for (int r = 0; r < R; r++)
-#pragma unroll
-    for (int j = 0; j < W; j++) {
-      x[r][j].x = 0;
-      x[r][j].y = 0;
-      if (act[r]) x[r][j] = A[pos[r] + j * a.lda];
-    }
+  int m = 0, top = 0, ph = 0;  // rows of the subpanel; ph: columns exchanged before it
+  bool dead = false;
   // every CTA's mbarriers are initialised before any message is sent
   cluster_barrier();
-  int top = lane;  // warp 0: the position of the row that began at position `lane`
-  bool dead = false;
   // where this thread's pieces of a message go (16 bytes each)
   constexpr int kSend = (kRegMaxCluster * kMsgChunks + T - 1) / T;
   unsigned to_msg[kSend], to_bar[kSend];
@@ -237,7 +233,7 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
     }
     const unsigned wm = __reduce_max_sync(0xffffffffu, bm);
     const int best = __ffs(__ballot_sync(0xffffffffu, bm == wm)) - 1;
-    const int par = c & 1;
+    const int par = (ph + c) & 1;
     const E brp = recip_of(bv);
     rest();
     if (lane == best) {
@@ -266,13 +262,13 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
   // columns follow, and the multipliers of the columns done since the window
   // began come last; so every column runs the same instructions (a fully
   // unrolled loop of 16 columns spent 40% of its time on instruction fetch).
-  auto columns = [&](auto win, int c0, int c1) {
+  auto columns = [&](auto win, int first, int c0, int c1) {
     constexpr int WIN = decltype(win)::value;
 #pragma unroll 1
     for (int c = c0; c < c1; c++) {
       // 1. the CTAs' messages of column c: the largest key wins
-      const int par = c & 1;
-      const unsigned bar = par ? bar1 : bar0, phase = (unsigned)(c >> 1) & 1u;
+      const int par = (ph + c) & 1;
+      const unsigned bar = par ? bar1 : bar0, phase = (unsigned)((ph + c) >> 1) & 1u;
       if (!dead) {
         long long it = 0;
         while (!mbar_poll(bar, phase)) {
@@ -334,8 +330,8 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
           if (lane == 0) {
             s_src[c] = none ? -1 : in->row;
             if (cta == 0) {
-              a.ipiv[a.c0 + c] = (int)a.c0 + p;
-              if (!live) atomicCAS(a.info, 0, (int)a.c0 + c + 1);
+              ipiv[first + c] = (int)a.j0 + first + p;
+              if (!live) atomicCAS(a.info, 0, (int)a.j0 + first + c + 1);
             }
           }
         }
@@ -352,53 +348,137 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
       else rest();
     }
   };
-  propose(0, []() {});
-  columns(std::integral_constant<int, W>{}, 0, W / 2);
-  columns(std::integral_constant<int, W / 2>{}, W / 2, W);
-  // no CTA leaves while messages to it can be under way (all have been
-  // waited for unless a wait ran out)
-  if (wid == 0 && lane < W) s_top[lane] = top;
-  const int stop = __syncthreads_or(dead ? 1 : 0);
-  if (!stop) {
+#pragma unroll 1
+  for (int s = a.s0; s < a.s1; s++) {
+    const int first = s * W;        // the subpanel's first column and row
+    const bool carry = s > a.s0;    // the last subpanel's update is still to do
+    E *A = P + first + first * a.lda;
+    m = a.m - first;
+    top = lane;  // warp 0: the position of the row that began at position `lane`
+    if (carry) {
+      // U12 of the last subpanel on the columns from here on
+      constexpr int kPer = ((kPanelNb - W) * W + T - 1) / T;
+      E v[kPer];  // every load in flight before the shared stores
 #pragma unroll
-    for (int r = 0; r < R; r++)
+      for (int u = 0; u < kPer; u++) {
+        const int i = tid + u * T;
+        v[u] = E{0, 0};
+        if (i < (kPanelNb - first) * W) v[u] = __ldcg(A - W + i % W + (i / W) * a.lda);
+      }
 #pragma unroll
-      for (int j = 0; j < W; j++)
-        if (cta * (T * R) + r * T + tid < m) A[pos[r] + ((j + W / 2) % W) * a.lda] = x[r][j];
-    // 6. the panel's other columns: the rows the interchanges move (lane i < W:
-    //    row i takes the i-th pivot row; lane W + i: the place that the old
-    //    row i ended at), and U12 = inv(L11) A12 on the columns to the right.
-    //    One warp per column.
-    int from = -1, to = -1;
-    if (lane < W) {
-      from = s_src[lane];
-      to = lane;
-      if (from < 0) from = lane;  // failed pivot: no interchange
-    } else if (lane < 2 * W && s_top[lane - W] >= W) {
-      from = lane - W;
-      to = s_top[lane - W];
+      for (int u = 0; u < kPer; u++) {
+        const int i = tid + u * T;
+        if (i < (kPanelNb - first) * W) s_u[i / W][i % W] = v[u];
+      }
+      __syncthreads();
     }
-    E *P = reinterpret_cast<E *>(a.A) + a.c0 + a.j0 * a.lda;  // column 0 of the panel, row c0
-    const int own = (int)(a.c0 - a.j0);
-    for (int col = cta * kRegWarps + wid; col < kPanelNb - W; col += CL * kRegWarps) {
-      const int cc = col < own ? col : col + W;
-      E *q = P + (int64_t)cc * a.lda;
-      E v = {0, 0};
-      if (from >= 0) v = q[from];
-      __syncwarp();
-      if (cc >= own + W) {
 #pragma unroll
-        for (int k = 0; k < W - 1; k++) {
-          E u;
-          u.x = __shfl_sync(0xffffffffu, v.x, k);
-          u.y = __shfl_sync(0xffffffffu, v.y, k);
-          if (lane > k && lane < W) v = nmac(v, s_l11[lane][k], u);
+    for (int r = 0; r < R; r++) {
+      pos[r] = cta * (T * R) + r * T + tid;
+      act[r] = pos[r] < m;
+#pragma unroll
+      for (int j = 0; j < W; j++) {
+        x[r][j] = E{0, 0};
+        if (act[r]) x[r][j] = __ldcg(A + pos[r] + j * a.lda);
+      }
+    }
+    if (carry) {
+#pragma unroll 1
+      for (int r0 = 0; r0 < R; r0++) {
+        // one row at a time (its multipliers take W registers); the rows
+        // rotate so that every access to x has a fixed index
+        const int row = cta * (T * R) + r0 * T + tid;
+        const bool on = row < m;
+        E l[W];
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+          l[k] = E{0, 0};
+          if (on) l[k] = __ldcg(A + row + (k - W) * a.lda);
+        }
+        E y[W];
+#pragma unroll
+        for (int j = 0; j < W; j++) y[j] = x[0][j];
+#pragma unroll
+        for (int j = 0; j < W; j++)
+#pragma unroll
+          for (int k = 0; k < W; k++) y[j] = nmac(y[j], l[k], s_u[j][k]);
+#pragma unroll
+        for (int r = 0; r + 1 < R; r++)
+#pragma unroll
+          for (int j = 0; j < W; j++) x[r][j] = x[r + 1][j];
+#pragma unroll
+        for (int j = 0; j < W; j++) x[R - 1][j] = y[j];
+        // the columns right of this subpanel, in place
+#pragma unroll 1
+        for (int j0 = W; j0 < kPanelNb - first; j0 += 8) {
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            y[j] = E{0, 0};
+            if (on) y[j] = __ldcg(A + row + (j0 + j) * a.lda);
+          }
+#pragma unroll
+          for (int j = 0; j < 8; j++)
+#pragma unroll
+            for (int k = 0; k < W; k++) y[j] = nmac(y[j], l[k], s_u[j0 + j][k]);
+#pragma unroll
+          for (int j = 0; j < 8; j++)
+            if (on) A[row + (j0 + j) * a.lda] = y[j];
         }
       }
-      if (to >= 0) q[to] = v;
     }
+    propose(0, []() {});
+    columns(std::integral_constant<int, W>{}, first, 0, W / 2);
+    columns(std::integral_constant<int, W / 2>{}, first, W / 2, W);
+    ph += W;
+    if (wid == 0 && lane < W) s_top[lane] = top;
+    // (a CTA whose wait ran out stores nothing more)
+    const int stop = __syncthreads_or(dead ? 1 : 0);
+    if (!stop) {
+#pragma unroll
+      for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int j = 0; j < W; j++)
+          if (cta * (T * R) + r * T + tid < m) A[pos[r] + ((j + W / 2) % W) * a.lda] = x[r][j];
+      // 4. the panel's other columns: the rows the interchanges move (lane i <
+      //    W: row i takes the i-th pivot row; lane W + i: the place that the
+      //    old row i ended at), and U12 = inv(L11) A12 on the columns to the
+      //    right.  One warp per column.
+      int from = -1, to = -1;
+      if (lane < W) {
+        from = s_src[lane];
+        to = lane;
+        if (from < 0) from = lane;  // failed pivot: no interchange
+      } else if (lane < 2 * W && s_top[lane - W] >= W) {
+        from = lane - W;
+        to = s_top[lane - W];
+      }
+      if (a.map && cta == 0 && wid == 0 && lane < 2 * W) {
+        int *map = a.map + blockIdx.y * a.batch_map + 2 * W * s + lane;
+        map[0] = from < 0 ? -1 : first + from;
+        map[128] = first + to;
+      }
+      for (int col = cta * kRegWarps + wid; col < kPanelNb - W; col += CL * kRegWarps) {
+        const int cc = col < first ? col : col + W;
+        E *q = P + first + (int64_t)cc * a.lda;
+        E v = {0, 0};
+        if (from >= 0) v = __ldcg(q + from);
+        __syncwarp();
+        if (cc >= first + W) {
+#pragma unroll
+          for (int k = 0; k < W - 1; k++) {
+            E u;
+            u.x = __shfl_sync(0xffffffffu, v.x, k);
+            u.y = __shfl_sync(0xffffffffu, v.y, k);
+            if (lane > k && lane < W) v = nmac(v, s_l11[lane][k], u);
+          }
+        }
+        if (to >= 0) q[to] = v;
+      }
+    }
+    // every column of the cluster is in place; and no CTA leaves while messages
+    // to it can be under way (all have been waited for unless a wait ran out)
+    cluster_barrier();
   }
-  cluster_barrier();
 }
 
 // C (m x nc) -= L (m x W) U (W x nc): the rows below a subpanel on the
@@ -408,7 +488,11 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
 constexpr int kRwThreads = 128;
 constexpr int kRwCols = 8;
 template <typename E, int W>
-__global__ void __launch_bounds__(kRwThreads) rank_w_kernel(const E *L, const E *U, E *C, int64_t lda, int m) {
+__global__ void __launch_bounds__(kRwThreads) rank_w_kernel(const E *L, const E *U, E *C, int64_t lda, int m,
+                                                            int64_t batch) {
+  L += blockIdx.z * batch;
+  U += blockIdx.z * batch;
+  C += blockIdx.z * batch;
   __shared__ __align__(16) E su[kRwCols][W];
   const int j0 = blockIdx.y * kRwCols;
   for (int i = threadIdx.x; i < kRwCols * W; i += kRwThreads) su[i / W][i % W] = U[i % W + (j0 + i / W) * lda];
@@ -440,12 +524,203 @@ __global__ void __launch_bounds__(kRwThreads) rank_w_kernel(const E *L, const E 
   }
 }
 
+// The interchanges of a panel, and U12 = inv(L11) A12, on columns outside it.
+// Four lanes share a column, eight columns per warp: lane g holds the rows 4 i +
+// g of the column's top 64.  The interchanges are gathers (each top row loads
+// its source; the old top rows that leave are stored where they end).  The
+// substitution with the unit lower L11 (staged in shared memory) goes four rows
+// at a time: the four rows among the four lanes by shuffles, then every row
+// below takes their four products.  The registers rotate by one row per step, so
+// the loop body is the same 15 guarded row updates.  Columns left of the panel
+// are only interchanged, and with them the vector that records the row order.
+// Bound by the latency of its chain (loads, map, sixteen steps): 17 us in FP64,
+// 13 us in FP32 under ncu, whatever the number of columns up to 3,840.  Before, a map kernel, an interchange
+// kernel, the inverse of L11, a GEMM with it and a copy took about 45 us.
+constexpr int kStThreads = 128, kStTile = kStThreads / 4;  // columns per CTA
+
+template <typename E>
+struct SwapTrsmArgs {
+  E *A;
+  int64_t lda, j0;
+  int entries;              // map entries per subpanel: 2 W
+  const int *map;           // [2][128], or null: no interchanges
+  int *moves;               // or null: the composed moves, dst[128], src[128], count
+  int64_t r0, r1;           // columns right of the panel: interchange and solve
+  int64_t l0, l1;           // columns left of it: interchange
+  int *perm;                // or null
+  int64_t batch_A, batch_piv, batch_map;
+};
+constexpr int kStLd = kPanelNb + 1;  // row stride of the staged L11
+template <typename E>
+constexpr size_t swap_trsm_smem() {
+  return sizeof(E) * kPanelNb * kStLd;
+}
+
+template <typename E>
+__global__ void __launch_bounds__(kStThreads) swap_trsm_kernel(SwapTrsmArgs<E> a) {
+  extern __shared__ __align__(16) unsigned char st_smem[];
+  E *s_l = reinterpret_cast<E *>(st_smem);  // [row][k]
+  __shared__ int2 s_map[128];               // (from, to) of the subpanels' moves
+  __shared__ int s_src[kPanelNb];           // source of each top row
+  __shared__ int2 s_out[128];               // old top rows that leave: (from, to)
+  __shared__ int s_nout;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  E *A = a.A + blockIdx.y * a.batch_A + a.j0;
+  const int64_t tr = (a.r1 - a.r0 + kStTile - 1) / kStTile;  // tiles of the right side come first
+  const bool right = (int64_t)blockIdx.x < tr;
+  if (right) {
+    // sixteen loads in flight per thread before the shared stores
+    for (int i0 = tid; i0 < kPanelNb * kPanelNb; i0 += 16 * kStThreads) {
+      E v[16];
+#pragma unroll
+      for (int u = 0; u < 16; u++) {
+        const int i = i0 + u * kStThreads;
+        v[u] = A[i % kPanelNb + (a.j0 + i / kPanelNb) * a.lda];
+      }
+#pragma unroll
+      for (int u = 0; u < 16; u++) {
+        const int i = i0 + u * kStThreads;
+        s_l[(i % kPanelNb) * kStLd + i / kPanelNb] = v[u];
+      }
+    }
+  }
+  if (tid < kPanelNb) s_src[tid] = tid;
+  if (tid == 0) s_nout = 0;
+  if (a.map) {
+    const int *map = a.map + blockIdx.y * a.batch_map;
+    s_map[tid] = make_int2(map[tid], map[128 + tid]);
+    __syncthreads();
+    // entry -> the row that its destination holds after every subpanel's
+    // moves: follow the moves backwards; the last subpanel that moves a row to
+    // a destination speaks for it
+    const int sub = tid / a.entries, to = s_map[tid].y;
+    int from = -1;
+    if (s_map[tid].x >= 0) {
+      from = to;
+      for (int s = 128 / a.entries - 1; s >= 0; s--) {
+        int hit = -1;
+#pragma unroll 8
+        for (int e = 0; e < a.entries; e++) {
+          const int2 v = s_map[s * a.entries + e];
+          if (v.x >= 0 && v.y == from) hit = v.x;
+        }
+        if (hit >= 0) {
+          if (s > sub && from == to) {
+            from = -1;
+            break;
+          }
+          from = hit;
+        }
+      }
+    }
+    if (from >= 0 && from != to) {
+      if (to < kPanelNb) s_src[to] = from;
+      else s_out[atomicAdd(&s_nout, 1)] = make_int2(from, to);
+    }
+  }
+  __syncthreads();
+  const int nout = s_nout;
+  if (blockIdx.x == gridDim.x - 1) {
+    // by the last CTA: the row order, and the composed moves
+    if (a.perm) {
+      int *perm = a.perm + blockIdx.y * a.batch_piv + a.j0;
+      int v = 0, o = 0;
+      if (tid < kPanelNb) v = perm[s_src[tid]];
+      if (tid < nout) o = perm[s_out[tid].x];
+      __syncthreads();
+      if (tid < kPanelNb) perm[tid] = v;
+      if (tid < nout) perm[s_out[tid].y] = o;
+    }
+    if (a.moves) {
+      const bool moved = tid < kPanelNb && s_src[tid] != tid;
+      if (tid < nout) {
+        a.moves[tid] = (int)a.j0 + s_out[tid].y;
+        a.moves[128 + tid] = (int)a.j0 + s_out[tid].x;
+      }
+      __shared__ int s_cnt;
+      if (tid == 0) s_cnt = nout;
+      __syncthreads();
+      if (moved) {
+        const int at = atomicAdd(&s_cnt, 1);
+        a.moves[at] = (int)a.j0 + tid;
+        a.moves[128 + at] = (int)a.j0 + s_src[tid];
+      }
+      __syncthreads();
+      if (tid == 0) a.moves[256] = s_cnt;
+    }
+  }
+  const int64_t tile = right ? blockIdx.x : (int64_t)blockIdx.x - tr;
+  const int64_t col = (right ? a.r0 : a.l0) + tile * kStTile + wid * 8 + lane / 4, end = right ? a.r1 : a.l1;
+  const int g = lane & 3;
+  const bool on = col < end;
+  E *q = A + (on ? col : 0) * a.lda;
+  E x[16];
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    x[i] = E{0, 0};
+    const int src = s_src[4 * i + g];
+    if (on && (right || src != 4 * i + g)) x[i] = q[src];
+  }
+  // the rows that leave: all loads of a column before its stores
+  for (int o0 = 0; o0 < nout; o0 += 64) {
+    E v[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const int e = o0 + 4 * i + g;
+      v[i] = E{0, 0};
+      if (on && e < nout) v[i] = q[s_out[e].x];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const int e = o0 + 4 * i + g;
+      if (on && e < nout) q[s_out[e].y] = v[i];
+    }
+  }
+  if (!right) {
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      if (on && s_src[4 * i + g] != 4 * i + g) q[4 * i + g] = x[i];
+    return;
+  }
+#pragma unroll 1
+  for (int b = 0; b < 16; b++) {
+    // rows 4 b .. 4 b + 3, x[0] of the four lanes
+    const E *l = s_l + (4 * b + g) * kStLd + 4 * b;
+    E u[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      u[k].x = __shfl_sync(0xffffffffu, x[0].x, (lane & ~3) + k);
+      u[k].y = __shfl_sync(0xffffffffu, x[0].y, (lane & ~3) + k);
+      if (k < 3 && g > k) x[0] = nmac(x[0], l[k], u[k]);
+    }
+    if (on) q[4 * b + g] = x[0];
+    // the rows below, five at a time (one by one under their own guards they
+    // would wait for each other); past the end a row reads the
+    // last row of L11 and is not used
+#pragma unroll
+    for (int h = 1; h < 16; h += 5)
+      if (h < 16 - b) {
+#pragma unroll
+        for (int i = h; i < h + 5; i++) {
+          const E *li = s_l + min(4 * (b + i) + g, kPanelNb - 1) * kStLd + 4 * b;
+          E y = x[i];
+#pragma unroll
+          for (int k = 0; k < 4; k++) y = nmac(y, li[k], u[k]);
+          x[i - 1] = y;
+        }
+      }
+  }
+}
+
 template <typename E, int W, int R, int T>
-int launch_reg(Ctx *c, const RegPanelArgs &a, cudaStream_t st) {
-  int CL = 1;
-  while ((int64_t)T * R * CL < a.m) CL *= 2;
+int launch_reg(Ctx *c, const RegPanelArgs &a, int batch, cudaStream_t st) {
+  // (CTAs without rows still share the work on the other columns: 64 rows on
+  // one CTA take 78 us per panel, on eight 64 us)
+  int CL = std::min(8, c->panel_cluster);
+  while ((int64_t)T * R * CL < a.m - a.s0 * W) CL *= 2;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(CL);
+  cfg.gridDim = dim3(CL, batch);
   cfg.blockDim = dim3(T);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
@@ -473,41 +748,53 @@ template <typename E> constexpr int kRows8 = 2 * kRows16<E>;
 // serve two rows each, which wins in FP32 (4,096 rows: 74 against 76 us), and
 // in FP64, bound by its arithmetic, 256 threads win (102 against 105 us).
 template <typename E>
-int launch_sub(Ctx *c, int W, const RegPanelArgs &a, cudaStream_t st) {
-  const int64_t rows = (a.m + c->panel_cluster - 1) / c->panel_cluster;  // per CTA of the largest cluster
+int launch_sub(Ctx *c, int W, const RegPanelArgs &a, int batch, cudaStream_t st) {
+  const int64_t rows = (a.m - a.s0 * W + c->panel_cluster - 1) / c->panel_cluster;  // per CTA of the largest cluster
   if constexpr (sizeof(E) == 8) {
-    if (W == 8) return launch_reg<E, 8, 8, 256>(c, a, st);
-    if (rows <= 128) return launch_reg<E, 16, 1, 128>(c, a, st);
-    if (rows <= 256) return launch_reg<E, 16, 2, 128>(c, a, st);
-    if (rows <= 512) return launch_reg<E, 16, 2, 256>(c, a, st);
-    return launch_reg<E, 16, 4, 256>(c, a, st);
+    if (W == 8) return launch_reg<E, 8, 8, 256>(c, a, batch, st);
+    if (rows <= 128) return launch_reg<E, 16, 1, 128>(c, a, batch, st);
+    if (rows <= 256) return launch_reg<E, 16, 2, 128>(c, a, batch, st);
+    if (rows <= 512) return launch_reg<E, 16, 2, 256>(c, a, batch, st);
+    return launch_reg<E, 16, 4, 256>(c, a, batch, st);
   } else {
-    if (W == 8) return launch_reg<E, 8, 4, 256>(c, a, st);
-    if (rows <= 128) return launch_reg<E, 16, 1, 128>(c, a, st);
-    if (rows <= 256) return launch_reg<E, 16, 1, 256>(c, a, st);
-    return launch_reg<E, 16, 2, 256>(c, a, st);
+    if (W == 8) return launch_reg<E, 8, 4, 256>(c, a, batch, st);
+    if (rows <= 128) return launch_reg<E, 16, 1, 128>(c, a, batch, st);
+    if (rows <= 256) return launch_reg<E, 16, 1, 256>(c, a, batch, st);
+    return launch_reg<E, 16, 2, 256>(c, a, batch, st);
   }
 }
 
 template <typename E, int W>
-int factor_panel(Ctx *c, E *A, int64_t lda, int64_t n, int64_t j0, int *ipiv, int *info, int *timeout,
-                 cudaStream_t st) {
-  for (int64_t c0 = j0; c0 < j0 + kPanelNb; c0 += W) {
-    RegPanelArgs a;
-    a.A = A;
-    a.lda = lda;
-    a.c0 = c0;
-    a.j0 = j0;
-    a.m = (int)(n - c0);
-    a.ipiv = ipiv;
-    a.info = info;
-    a.timeout = timeout;
-    a.spin = wait_polls(c, 0);
-    MOM_TRY(launch_sub<E>(c, W, a, st));
-    const int nc = (int)(j0 + kPanelNb - (c0 + W)), below = a.m - W;
+int factor_panel(Ctx *c, const PanelCall<E> &p, bool one_launch) {
+  RegPanelArgs a;
+  a.A = p.A;
+  a.lda = p.lda;
+  a.j0 = p.j0;
+  a.m = (int)(p.n - p.j0);
+  a.ipiv = p.ipiv;
+  a.info = p.info;
+  a.timeout = p.timeout;
+  a.spin = wait_polls(c, 0);
+  a.map = p.map;
+  a.batch_A = p.batch_A;
+  a.batch_piv = p.batch_piv;
+  a.batch_map = p.batch_map;
+  constexpr int kSub = kPanelNb / W;
+  if (one_launch) {
+    a.s0 = 0;
+    a.s1 = kSub;
+    return launch_sub<E>(c, W, a, p.batch, p.st);
+  }
+  for (int s = 0; s < kSub; s++) {
+    a.s0 = s;
+    a.s1 = s + 1;
+    MOM_TRY(launch_sub<E>(c, W, a, p.batch, p.st));
+    const int64_t c0 = p.j0 + s * W;
+    const int nc = kPanelNb - (s + 1) * W, below = (int)(p.n - c0) - W;
     if (nc > 0 && below > 0) {
-      rank_w_kernel<E, W><<<dim3((below + 2 * kRwThreads - 1) / (2 * kRwThreads), nc / kRwCols), kRwThreads, 0, st>>>(
-          A + (c0 + W) + c0 * lda, A + c0 + (c0 + W) * lda, A + (c0 + W) + (c0 + W) * lda, lda, below);
+      const dim3 grid((below + 2 * kRwThreads - 1) / (2 * kRwThreads), nc / kRwCols, p.batch);
+      E *L = p.A + (c0 + W) + c0 * p.lda, *U = p.A + c0 + (c0 + W) * p.lda, *C = U + W;
+      rank_w_kernel<E, W><<<grid, kRwThreads, 0, p.st>>>(L, U, C, p.lda, below, p.batch_A);
       c->launches++;
       MOM_CUDA(c, cudaGetLastError());
     }
@@ -558,18 +845,52 @@ int64_t panel_reg_rows(const Ctx *c, bool f32) {
   return (int64_t)(f32 ? kRows8<float2> : kRows8<double2>) * c->panel_cluster;
 }
 
-int panel_reg(Ctx *c, float2 *A, int64_t lda, int64_t n, int64_t j0, int *ipiv, int *info, int *timeout,
-              cudaStream_t st) {
-  if (n - j0 <= (int64_t)kRows16<float2> * c->panel_cluster)
-    return factor_panel<float2, 16>(c, A, lda, n, j0, ipiv, info, timeout, st);
-  return factor_panel<float2, 8>(c, A, lda, n, j0, ipiv, info, timeout, st);
+// 16 columns at a time while the rows fit.  One launch for the panel if
+// one_launch says so (the caller runs something else beside it).  Alone, four
+// launches with the rank-16 updates on every SM between them are faster on tall
+// panels (16,384 rows FP32: 110 against 147 us, 4,096 rows 73 against 93 us, FP64
+// 104 against 112 us; no difference up to 1,024 rows).
+template <typename E>
+int panel_reg(Ctx *c, const PanelCall<E> &p, bool one_launch) {
+  if (p.n - p.j0 <= (int64_t)kRows16<E> * c->panel_cluster) return factor_panel<E, 16>(c, p, one_launch);
+  return factor_panel<E, 8>(c, p, one_launch);
 }
+template int panel_reg<float2>(Ctx *, const PanelCall<float2> &, bool);
+template int panel_reg<double2>(Ctx *, const PanelCall<double2> &, bool);
 
-int panel_reg(Ctx *c, double2 *A, int64_t lda, int64_t n, int64_t j0, int *ipiv, int *info, int *timeout,
-              cudaStream_t st) {
-  if (n - j0 <= (int64_t)kRows16<double2> * c->panel_cluster)
-    return factor_panel<double2, 16>(c, A, lda, n, j0, ipiv, info, timeout, st);
-  return factor_panel<double2, 8>(c, A, lda, n, j0, ipiv, info, timeout, st);
+template <typename E>
+int swap_trsm(Ctx *c, const PanelCall<E> &p, int64_t r0, int64_t r1, int64_t l0, int64_t l1, int *perm, int *moves) {
+  SwapTrsmArgs<E> a;
+  a.A = p.A;
+  a.lda = p.lda;
+  a.j0 = p.j0;
+  a.entries = p.n - p.j0 <= (int64_t)kRows16<E> * c->panel_cluster ? 32 : 16;
+  a.map = p.map;
+  a.r0 = r0;
+  a.r1 = std::max(r0, r1);
+  a.l0 = l0;
+  a.l1 = std::max(l0, l1);
+  a.perm = perm;
+  a.moves = moves;
+  a.batch_A = p.batch_A;
+  a.batch_piv = p.batch_piv;
+  a.batch_map = p.batch_map;
+  const int64_t tiles = (a.r1 - a.r0 + kStTile - 1) / kStTile + (a.l1 - a.l0 + kStTile - 1) / kStTile;
+  if (tiles == 0 && !perm && !moves) return MOM_OK;
+  swap_trsm_kernel<E><<<dim3((unsigned)std::max<int64_t>(1, tiles), p.batch), kStThreads, swap_trsm_smem<E>(), p.st>>>(a);
+  c->launches++;
+  MOM_CUDA(c, cudaGetLastError());
+  return MOM_OK;
+}
+template int swap_trsm<float2>(Ctx *, const PanelCall<float2> &, int64_t, int64_t, int64_t, int64_t, int *, int *);
+template int swap_trsm<double2>(Ctx *, const PanelCall<double2> &, int64_t, int64_t, int64_t, int64_t, int *, int *);
+
+int panel_init_kernels(Ctx *c) {
+  MOM_CUDA(c, cudaFuncSetAttribute(swap_trsm_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)swap_trsm_smem<float2>()));
+  MOM_CUDA(c, cudaFuncSetAttribute(swap_trsm_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)swap_trsm_smem<double2>()));
+  return MOM_OK;
 }
 
 }  // namespace mom

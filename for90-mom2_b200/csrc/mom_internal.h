@@ -224,13 +224,6 @@ struct Ctx {
   // CTAs that exchange through global memory.
   int panel_cluster = 0;
   int outer_panels = 4;  // panels per outer block of the LU (MOM_LU_OUTER): trailing GEMMs have K = 64 * this
-  int small_tc = 0;      // mixed path: K = 64 updates on the tensor cores too (MOM_SMALL_TC=1), else library FP32 GEMM
-  // Look-ahead path: the block TRSMs of an outer block by block_trsm_kernel
-  // instead of library CGEMMs: MOM_FUSED_TRSM=1 everywhere (measured slower
-  // at 15,360 unknowns: 158.6 against 155.0 ms per solve), 2 only for the
-  // narrow updates on the panels' critical path (the next block's columns and
-  // the in-block updates), 0 (default) nowhere.
-  int fused_trsm = 0;
   // Permittivity gradients by adj_eps_kernel (FP64 geometry, dual numbers in
   // k only); MOM_ADJ_EPS_PLAIN=0 selects the all-dual adj_pair_kernel.
   int adj_eps_plain = 1;
@@ -361,7 +354,8 @@ int load_matrix(Ctx *c, const double *A_host, int64_t ldh, int precision);
 
 // lu.cu
 int lu_init_kernels(Ctx *c);
-int lu_factor(Ctx *c, int precision);
+// Every representation's matrix (leaves representation 0 selected).
+int lu_factor_reps(Ctx *c, int precision);
 int lu_solve(Ctx *c, int precision, double tol, int maxit, int *iters);
 int lu_solve_ex(Ctx *c, int precision, int trans, const double2 *B, double2 *X, int nrhs, double tol, int maxit,
                 int *iters);
@@ -374,14 +368,31 @@ int shg_solve(Ctx *c, double omega, const double *ri, const double *shri, const 
               double tol, int maxit, int *iters);
 void free_shg(DomDev &D);
 
-// lu_panel.cu: the 64-column panel at column j0 (rows j0 .. n) on one
-// thread-block cluster, for n - j0 <= panel_reg_rows().
+// lu_panel.cu: the 64-column panel at column j0 (rows j0 .. n) of `batch`
+// matrices (batch_A entries apart; their pivots batch_piv, their maps
+// batch_map), each on one thread-block cluster, for n - j0 <=
+// panel_reg_rows().  map (or null): the panel's row moves for swap_trsm.
+template <typename E>
+struct PanelCall {
+  E *A;
+  int64_t lda, n, j0;
+  int *ipiv, *info, *timeout, *map;
+  cudaStream_t st;
+  int batch;
+  int64_t batch_A, batch_piv, batch_map;
+};
 int panel_reg_max_cluster();
 int64_t panel_reg_rows(const Ctx *c, bool f32);
-int panel_reg(Ctx *c, float2 *A, int64_t lda, int64_t n, int64_t j0, int *ipiv, int *info, int *timeout,
-              cudaStream_t st);
-int panel_reg(Ctx *c, double2 *A, int64_t lda, int64_t n, int64_t j0, int *ipiv, int *info, int *timeout,
-              cudaStream_t st);
+template <typename E>
+int panel_reg(Ctx *c, const PanelCall<E> &p, bool one_launch);
+// The interchanges of that panel and U12 = inv(L11) A12 on the columns [r0, r1)
+// right of it, the interchanges alone on [l0, l1) left of it and on perm (or
+// null); a null p.map leaves the interchanges out.  moves (or null) receives the
+// panel's interchanges as dst[128], src[128], count.
+template <typename E>
+int swap_trsm(Ctx *c, const PanelCall<E> &p, int64_t r0, int64_t r1, int64_t l0, int64_t l1, int *perm,
+              int *moves = nullptr);
+int panel_init_kernels(Ctx *c);
 
 // tc_gemm.cu: C -= L U (complex FP32) on the tensor cores, FP32-accurate
 int tc_cgemm_update(Ctx *c, float2 *C, int64_t ldc, const float2 *L, int64_t ldl, const float2 *U, int64_t ldu, int m,

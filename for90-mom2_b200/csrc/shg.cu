@@ -772,14 +772,7 @@ int shg_solve(Ctx *c, double omega, const double *ri, const double *shri, const 
   // sides are zero (identity rows), one factorisation and solve each
   int it = 0;
   for (int r = 0; r < nga && nga > 1; r++) MOM_TRY(apply_bc_rhs(c, r, c->B + r * col_rep, nsrc));
-  for (int r = 0; r < nga; r++) {
-    select_rep(c, r);
-    const int rc = lu_factor(c, precision);
-    if (rc != MOM_OK) {
-      select_rep(c, 0);
-      return rc;
-    }
-  }
+  MOM_TRY(lu_factor_reps(c, precision));
   for (int r = 0; r < nga; r++) {
     select_rep(c, r);
     int itr = 0;
