@@ -1292,6 +1292,7 @@ int load_matrix(Ctx *c, const double *A_host, int64_t ldh, int precision) {
 
 #include "adjoint_impl.cuh"
 #include "nfields_impl.cuh"
+#include "adjoint_eps_impl.cuh"
 #include "adjoint_nodes_impl.cuh"
 
 namespace {
@@ -1413,50 +1414,67 @@ int adjoint_eps(Ctx *c, double omega, const double *ri, int d, int R, const doub
   a.xv = xv;
   a.W = W;
   const int nobj = R == 0 ? 1 : R;
-  const dim3 grid((D.F + kAdjThreads - 1) / kAdjThreads, D.F);
-  const size_t nvals = (size_t)grid.x * grid.y * nobj * 2;
-  MOM_TRY(ensure_buffer(c, &c->adj_part, &c->adj_part_bytes, sizeof(double) * nvals));
-  a.part = (double *)c->adj_part;
   if (c->adj_eps_plain) {
-    // the same sums with FP64 geometry and dual numbers only where k enters
-    MOM_TRY(nfield_geometry(c, D));
+    // one objective (or the dense W) per pair of launches
     AdjEpsArgs e;
     e.F = D.F;
     e.n = c->n;
     e.N = c->N;
     e.qrel = D.qrel;
-    e.qabs = D.qabs;
     e.cp = D.cp;
-    e.area = D.area;
     e.mu = D.mu;
     e.sl = D.sl;
-    e.bn = D.nf_bn;
-    e.geo = reinterpret_cast<const FaceGeo *>(D.nf_geo);
     e.hpar = D.hpar;
     e.near_bits = D.near_bits;
-    e.kr = a.kr;
-    e.ki = a.ki;
-    e.c1 = a.c1;
-    e.c2 = a.c2;
-    e.Zsi = a.Zsi;
-    e.R = R;
-    e.lam = lam;
-    e.xv = xv;
+    e.nnear = D.nnear;
+    e.near_m = D.near_m;
+    e.near_n = D.near_n;
+    e.near_static = D.near_static;
+    auto val = [](const Cx<Dual> &z) { return Cd{z.re.v, z.im.v}; };
+    auto der = [](const Cx<Dual> &z) { return Cd{z.re.d, z.im.d}; };
+    const Cx<Dual> k = {a.kr, a.ki};
+    e.k = val(k);
+    e.dk = der(k);
+    e.c1 = val(a.c1);
+    e.c2 = val(a.c2);
+    e.dc2 = der(a.c2);
+    e.Z = val(a.Zsi);
+    e.dZ = der(a.Zsi);
     e.W = W;
-    e.part = a.part;
-    switch (c->nq) {
-      case 1: launch_adj_eps<1>(grid, c->stream, e); break;
-      case 3: launch_adj_eps<3>(grid, c->stream, e); break;
-      case 4: launch_adj_eps<4>(grid, c->stream, e); break;
-      case 7: launch_adj_eps<7>(grid, c->stream, e); break;
-      case 13: launch_adj_eps<13>(grid, c->stream, e); break;
-      default: return fail(c, MOM_ERR_ARG, "unsupported number of quadrature points");
+    const dim3 far((D.F + kEpsThreads - 1) / kEpsThreads, (D.F + kEpsTests - 1) / kEpsTests);
+    const unsigned near = (unsigned)((D.nnear + kEpsThreads - 1) / kEpsThreads);
+    const size_t parts = (size_t)far.x * far.y + near;
+    MOM_TRY(ensure_buffer(c, &c->adj_part, &c->adj_part_bytes, sizeof(double2) * parts * nobj));
+    for (int o = 0; o < nobj; o++) {
+      e.lam = R ? lam + (size_t)o * c->n : nullptr;
+      e.xv = R ? xv + (size_t)o * c->n : nullptr;
+      e.part = (double2 *)c->adj_part + parts * o;
+      switch (c->nq) {
+        case 1: launch_adj_eps<1>(far, near, c->stream, e); break;
+        case 3: launch_adj_eps<3>(far, near, c->stream, e); break;
+        case 4: launch_adj_eps<4>(far, near, c->stream, e); break;
+        case 7: launch_adj_eps<7>(far, near, c->stream, e); break;
+        case 13: launch_adj_eps<13>(far, near, c->stream, e); break;
+        default: return fail(c, MOM_ERR_ARG, "unsupported number of quadrature points");
+      }
+      c->launches += near ? 2 : 1;
+      MOM_CUDA(c, cudaGetLastError());
     }
-    c->launches++;
-    MOM_CUDA(c, cudaGetLastError());
-  } else {
-    MOM_TRY(adj_launch_pair(c, grid, a));
+    std::vector<double> h(2 * parts * nobj);
+    MOM_CUDA(c, cudaMemcpyAsync(h.data(), c->adj_part, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream));
+    MOM_CUDA(c, cudaStreamSynchronize(c->stream));
+    for (int o = 0; o < nobj; o++) {
+      out[2 * o] = out[2 * o + 1] = 0;
+      for (size_t b = 0; b < parts; b++)
+        for (int i = 0; i < 2; i++) out[2 * o + i] += h[2 * (parts * o + b) + i];
+    }
+    return MOM_OK;
   }
+  const dim3 grid((D.F + kAdjThreads - 1) / kAdjThreads, D.F);
+  const size_t nvals = (size_t)grid.x * grid.y * nobj * 2;
+  MOM_TRY(ensure_buffer(c, &c->adj_part, &c->adj_part_bytes, sizeof(double) * nvals));
+  a.part = (double *)c->adj_part;
+  MOM_TRY(adj_launch_pair(c, grid, a));
   std::vector<double> h(nvals);
   MOM_CUDA(c, cudaMemcpyAsync(h.data(), a.part, sizeof(double) * nvals, cudaMemcpyDeviceToHost, c->stream));
   MOM_CUDA(c, cudaStreamSynchronize(c->stream));

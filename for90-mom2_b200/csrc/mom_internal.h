@@ -224,8 +224,8 @@ struct Ctx {
   // CTAs that exchange through global memory.
   int panel_cluster = 0;
   int outer_panels = 4;  // panels per outer block of the LU (MOM_LU_OUTER): trailing GEMMs have K = 64 * this
-  // Permittivity gradients by adj_eps_kernel (FP64 geometry, dual numbers in
-  // k only); MOM_ADJ_EPS_PLAIN=0 selects the all-dual adj_pair_kernel.
+  // Permittivity gradients by the point-pair forms of adjoint_eps_impl.cuh;
+  // MOM_ADJ_EPS_PLAIN=0 selects the all-dual adj_pair_kernel.
   int adj_eps_plain = 1;
   // Vertex gradients in reverse mode (adjoint_nodes_impl.cuh);
   // MOM_ADJ_VERTEX_PLAIN=0 selects the forward-mode adj_pair_kernel.
