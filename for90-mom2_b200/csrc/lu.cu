@@ -1898,6 +1898,7 @@ cudaError_t set_smem(T *fn) {
 
 // Shared-memory opt-in of the LU kernels, once per context (outside any
 // stream capture and off the factorisation's critical path).
+static int multi_init_kernels(Ctx *c);
 int lu_init_kernels(Ctx *c) {
   MOM_CUDA(c, set_smem(panel_kernel<double2>));
   MOM_CUDA(c, set_smem(panel_kernel<float2>));
@@ -1926,7 +1927,7 @@ int lu_init_kernels(Ctx *c) {
   MOM_CUDA(c, set_smem(trsv_flow_kernel<float2, 2, true>));
   MOM_CUDA(c, set_smem(trsv_flow_kernel<float2, 4, true>));
   MOM_CUDA(c, set_smem(trsv_flow_kernel<float2, 8, true>));
-  return MOM_OK;
+  return multi_init_kernels(c);
 }
 
 namespace {
@@ -2119,26 +2120,111 @@ int blas_gemm<float2>(Ctx *c, cublasOperation_t ta, int m, int nn, int k, double
   return MOM_OK;
 }
 
-// Many right-hand sides: blocked substitution with the diagonal-block
-// inverses, every step a library GEMM (64-row blocks; the updates of the
-// rows below / above are tall GEMMs with K = 64).  X (n x nrhs, ld n) is
-// overwritten with A^{-1} X (trans: A^{-T} X).  T = float2 works on the FP32
-// factors in FP32 (no TF32), T = double2 on the FP64 factors.
+// One block of at most kTriRows rows of the many-right-hand-side substitution:
+// Y(block) <- M^{-1} Y(block), M the block's triangle of L (lower) or U, TR of
+// their transposes U^T (lower) and L^T.  A CTA keeps kTriCols columns in shared
+// memory and takes the triangle's 64 x 64 tiles in order, row by row (y_k -=
+// M_kj y_j, then y_k <- inv_k y_k), each prefetched with cp.async; a thread has
+// one row, all the columns and a quarter of the tile's columns.  The tiles are
+// read by every CTA (L2) and the rows are a serial chain, so it is bound by
+// latency: few columns per CTA, so that 500 of them fill the chip.  FP32, 500
+// columns, 256 rows: 15 us (55 with the triangle read from L2 by each thread as
+// it went; the 11 library calls this takes the place of, 80).
+constexpr int kTriRows = 256, kTriCols = 4, kTriThreads = 256;
+template <typename T>
+constexpr int kTriStages = sizeof(T) == sizeof(float2) ? 3 : 2;
+constexpr int kTriTile = 64 * 65;  // a row (TR) is padded by one element
+template <typename T>
+constexpr size_t kTriSmem = sizeof(T) * (kTriStages<T> * kTriTile + kTriRows * kTriCols + 4 * 64 * kTriCols);
+
+template <typename T, bool TR>
+__global__ void __launch_bounds__(kTriThreads)
+    tri_block_kernel(const T *__restrict__ F, int64_t lda, const T *__restrict__ inv, int64_t K0, int rows, T *Y,
+                     int64_t n, int nrhs, bool lower) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int S = kTriStages<T>;
+  T *tiles = reinterpret_cast<T *>(smem_raw);
+  T *y = tiles + S * kTriTile;                // [row][column]
+  T *red = y + kTriRows * kTriCols;           // [quarter][column][row of the tile]
+  const int c0 = blockIdx.x * kTriCols, tid = threadIdx.x, r = tid % 64, part = tid / 64;
+  const int nb = rows / 64, nt = nb * (nb + 1) / 2;
+  // tile t: column step u of row step s, u == s the diagonal's inverse
+  auto row_of = [](int t) { return t >= 6 ? 3 : t >= 3 ? 2 : t >= 1 ? 1 : 0; };
+  auto blk = [&](int s) { return lower ? s : nb - 1 - s; };
+  auto issue = [&](int t) {
+    if (t < nt) {
+      const int s = row_of(t), u = t - s * (s + 1) / 2;
+      const int64_t i = K0 + 64 * blk(s), j = K0 + 64 * blk(u);
+      // the inverses of L, then of U; the transposed pass applies the other's transpose
+      const T *src = u == s ? inv + ((size_t)(K0 / 64 + blk(s)) * 2 + (lower != TR ? 0 : 1)) * 64 * 64
+                            : (TR ? F + j + i * lda : F + i + j * lda);
+      const int64_t ld = u == s ? 64 : lda;
+      T *dst = tiles + (t % S) * kTriTile;
+      constexpr int kVec = TR ? 1 : 16 / (int)sizeof(T);  // elements per copy
+      for (int x = tid; x < 64 * 64 / kVec; x += kTriThreads) {
+        const int e = x * kVec % 64, l = x * kVec / 64;
+        cp_async(dst + l * (TR ? 65 : 64) + e, src + e + l * ld, kVec * sizeof(T) == 16);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int t = 0; t < S - 1; t++) issue(t);
+  for (int i = tid; i < rows * kTriCols; i += kTriThreads) {
+    const int l = i % rows, c = i / rows;
+    y[l * kTriCols + c] = c0 + c < nrhs ? Y[(size_t)(c0 + c) * n + K0 + l] : T{0, 0};
+  }
+  T acc[kTriCols];
+#pragma unroll
+  for (int c = 0; c < kTriCols; c++) acc[c] = T{0, 0};
+  for (int t = 0; t < nt; t++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+    __syncthreads();  // tile t is there, tile t - 1 and the sums are read
+    issue(t + S - 1);
+    const int s = row_of(t), u = t - s * (s + 1) / 2;
+    const T *m = tiles + (t % S) * kTriTile, *yu = y + 64 * blk(u) * kTriCols;
+#pragma unroll 4
+    for (int j = part * 16; j < part * 16 + 16; j++) {
+      const T e = m[TR ? r * 65 + j : j * 64 + r];
+#pragma unroll
+      for (int c = 0; c < kTriCols; c++) cmac(acc[c], e, yu[j * kTriCols + c]);
+    }
+    if (u < s - 1) continue;  // the row's last tile, then its inverse
+#pragma unroll
+    for (int c = 0; c < kTriCols; c++) {
+      red[(part * kTriCols + c) * 64 + r] = acc[c];
+      acc[c] = T{0, 0};
+    }
+    __syncthreads();
+    T v = red[part * 64 + r];  // column `part`
+#pragma unroll
+    for (int p = 1; p < 4; p++) v = cadd(v, red[(p * kTriCols + part) * 64 + r]);
+    T *o = y + (64 * blk(s) + r) * kTriCols + part;
+    if (u < s) v = T{o->x - v.x, o->y - v.y};
+    *o = v;
+  }
+  __syncthreads();
+  for (int i = tid; i < rows * kTriCols; i += kTriThreads) {
+    const int l = i % rows, c = i / rows;
+    if (c0 + c < nrhs) Y[(size_t)(c0 + c) * n + K0 + l] = y[l * kTriCols + c];
+  }
+}
+
+// Many right-hand sides: blocked substitution, kTriRows rows at a time with
+// tri_block_kernel, then the update of the rows below (above): with FP32
+// factors and kMultiTc right-hand sides or more on the tensor cores
+// (FP32-accurate like the rest of the solve), else by the library GEMM.
+// X (n x nrhs, ld n) is overwritten with A^{-1} X (trans: A^{-T} X).  T =
+// float2 works on the FP32 factors in FP32 (no TF32), T = double2 on the FP64
+// factors.
 template <typename T>
 int getrs_multi(Ctx *c, const T *F, double2 *X, int nrhs, int trans) {
   const int64_t n = c->n, lda = c->lda;
-  const int nb = c->nb, nblk = (int)(n / nb);
   const bool f32 = sizeof(T) == sizeof(float2);
-  // FP32 factors and many right-hand sides: 256-row blocks whose updates run
-  // on the tensor cores (FP32-accurate like the rest of the solve)
   const bool tc = f32 && nrhs >= kMultiTc;
-  const int64_t NBt = 4 * (int64_t)nb;
-  const size_t ybytes = sizeof(T) * (size_t)n * nrhs, tbytes = sizeof(T) * (size_t)nb * nrhs;
-  const size_t o_t = ((ybytes + 255) / 256) * 256, o_w = o_t + ((tbytes + 255) / 256) * 256;
-  const size_t wbytes = tc ? tc_cgemm_work_bytes((int)n, nrhs, (int)NBt) : 0;
+  const size_t ybytes = sizeof(T) * (size_t)n * nrhs, o_w = ((ybytes + 255) / 256) * 256;
+  const size_t wbytes = tc ? tc_cgemm_work_bytes((int)n, nrhs, kTriRows) : 0;
   MOM_TRY(ensure_buffer(c, &c->ws2, &c->ws2_bytes, o_w + wbytes + 1024));
   T *Y = (T *)c->ws2;
-  T *Tm = (T *)((char *)c->ws2 + o_t);
   float *tw = (float *)((char *)c->ws2 + o_w);
   const T *inv = f32 ? (const T *)c->inv32 : (const T *)c->invd;
   ProfScope ps(c, kProfTrsv);
@@ -2147,75 +2233,25 @@ int getrs_multi(Ctx *c, const T *F, double2 *X, int nrhs, int trans) {
   c->launches++;
   MOM_CUDA(c, cudaGetLastError());
   MOM_BLAS(c, cublasSetMathMode(c->blas, CUBLAS_DEFAULT_MATH));
-  const cublasOperation_t op = trans ? CUBLAS_OP_T : CUBLAS_OP_N;
-  // block k of the pass: y_k <- inv_k y_k (through Tm), then the update
-  auto diag = [&](int kb, int which) -> int {
-    const int64_t k0 = (int64_t)kb * nb;
-    MOM_TRY(blas_gemm<T>(c, op, nb, nrhs, nb, 1.0, inv + ((size_t)kb * 2 + which) * nb * nb, nb, Y + k0, n, 0.0, Tm,
-                         nb));
-    MOM_CUDA(c, cudaMemcpy2DAsync(Y + k0, sizeof(T) * n, Tm, sizeof(T) * nb, sizeof(T) * nb, nrhs,
-                                  cudaMemcpyDeviceToDevice, c->stream));
-    return MOM_OK;
-  };
-  if (tc) {
-    // forward: L (unit lower), or U^T; 64-row blocks inside a 256-row block
-    // with the library GEMM, the rows below the 256-row block on the tensor cores
-    for (int64_t K0 = 0; K0 < n; K0 += NBt) {
-      const int64_t K1 = std::min<int64_t>(K0 + NBt, n);
-      for (int64_t k0 = K0; k0 < K1; k0 += nb) {
-        MOM_TRY(diag((int)(k0 / nb), trans ? 1 : 0));
-        const int64_t mi = K1 - k0 - nb;
-        if (mi > 0) {
-          const T *Ab = trans ? F + k0 + (k0 + nb) * lda : F + (k0 + nb) + k0 * lda;
-          MOM_TRY(blas_gemm<T>(c, op, (int)mi, nrhs, nb, -1.0, Ab, lda, Tm, nb, 1.0, Y + k0 + nb, n));
-        }
-      }
-      if (K1 < n) {
-        const T *Ab = trans ? F + K0 + K1 * lda : F + K1 + K0 * lda;
-        MOM_TRY(tc_cgemm_update(c, reinterpret_cast<float2 *>(Y + K1), n, reinterpret_cast<const float2 *>(Ab), lda,
-                                reinterpret_cast<const float2 *>(Y + K0), n, (int)(n - K1), nrhs, (int)(K1 - K0), tw,
-                                c->dinfo + 2, 0, false, trans != 0));
-      }
-    }
-    // backward: U, or L^T (unit upper)
-    for (int64_t K0 = ((n - 1) / NBt) * NBt; K0 >= 0; K0 -= NBt) {
-      const int64_t K1 = std::min<int64_t>(K0 + NBt, n);
-      for (int64_t k0 = K1 - nb; k0 >= K0; k0 -= nb) {
-        MOM_TRY(diag((int)(k0 / nb), trans ? 0 : 1));
-        if (k0 > K0) {
-          const T *Ab = trans ? F + k0 + K0 * lda : F + K0 + k0 * lda;
-          MOM_TRY(blas_gemm<T>(c, op, (int)(k0 - K0), nrhs, nb, -1.0, Ab, lda, Tm, nb, 1.0, Y + K0, n));
-        }
-      }
-      if (K0 > 0) {
-        const T *Ab = trans ? F + K0 : F + K0 * lda;
-        MOM_TRY(tc_cgemm_update(c, reinterpret_cast<float2 *>(Y), n, reinterpret_cast<const float2 *>(Ab), lda,
-                                reinterpret_cast<const float2 *>(Y + K0), n, (int)K0, nrhs, (int)(K1 - K0), tw,
-                                c->dinfo + 2, 0, false, trans != 0));
-      }
-    }
-    permute_rows_kernel<T, double2><<<pg, 256, 0, c->stream>>>(Y, n, X, n, n, c->perm, trans ? 2 : 1);
+  // the block of rows K0 on, and the update of rows [i0, i1) from it
+  auto step = [&](int64_t K0, bool lower, int64_t i0, int64_t i1) -> int {
+    const int rows = (int)std::min<int64_t>(kTriRows, n - K0), m = (int)(i1 - i0);
+    const unsigned ctas = (unsigned)((nrhs + kTriCols - 1) / kTriCols);
+    auto *kern = trans ? tri_block_kernel<T, true> : tri_block_kernel<T, false>;
+    kern<<<ctas, kTriThreads, kTriSmem<T>, c->stream>>>(F, lda, inv, K0, rows, Y, n, nrhs, lower);
     c->launches++;
     MOM_CUDA(c, cudaGetLastError());
-    return MOM_OK;
-  }
+    if (m <= 0) return MOM_OK;
+    const T *Ab = trans ? F + K0 + i0 * lda : F + i0 + K0 * lda;
+    if (tc)
+      return tc_cgemm_update(c, reinterpret_cast<float2 *>(Y + i0), n, reinterpret_cast<const float2 *>(Ab), lda,
+                             reinterpret_cast<const float2 *>(Y + K0), n, m, nrhs, rows, tw, c->dinfo + 2, 0, false,
+                             trans != 0);
+    return blas_gemm<T>(c, trans ? CUBLAS_OP_T : CUBLAS_OP_N, m, nrhs, rows, -1.0, Ab, lda, Y + K0, n, 1.0, Y + i0, n);
+  };
   // forward: L (unit lower), or U^T; backward: U, or L^T (unit upper)
-  for (int kb = 0; kb < nblk; kb++) {
-    const int64_t k0 = (int64_t)kb * nb, m = n - k0 - nb;
-    MOM_TRY(diag(kb, trans ? 1 : 0));
-    if (m > 0) {
-      const T *Ab = trans ? F + k0 + (k0 + nb) * lda : F + (k0 + nb) + k0 * lda;
-      MOM_TRY(blas_gemm<T>(c, op, (int)m, nrhs, nb, -1.0, Ab, lda, Tm, nb, 1.0, Y + k0 + nb, n));
-    }
-  }
-  for (int kb = nblk - 1; kb >= 0; kb--) {
-    const int64_t k0 = (int64_t)kb * nb;
-    MOM_TRY(diag(kb, trans ? 0 : 1));
-    if (k0 > 0) {
-      const T *Ab = trans ? F + k0 : F + k0 * lda;
-      MOM_TRY(blas_gemm<T>(c, op, (int)k0, nrhs, nb, -1.0, Ab, lda, Tm, nb, 1.0, Y, n));
-    }
-  }
+  for (int64_t K0 = 0; K0 < n; K0 += kTriRows) MOM_TRY(step(K0, true, std::min<int64_t>(K0 + kTriRows, n), n));
+  for (int64_t K0 = (n - 1) / kTriRows * kTriRows; K0 >= 0; K0 -= kTriRows) MOM_TRY(step(K0, false, 0, K0));
   permute_rows_kernel<T, double2><<<pg, 256, 0, c->stream>>>(Y, n, X, n, n, c->perm, trans ? 2 : 1);
   c->launches++;
   MOM_CUDA(c, cudaGetLastError());
@@ -2223,6 +2259,14 @@ int getrs_multi(Ctx *c, const T *F, double2 *X, int nrhs, int trans) {
 }
 
 }  // namespace
+
+static int multi_init_kernels(Ctx *c) {
+  MOM_CUDA(c, set_smem(tri_block_kernel<double2, false>));
+  MOM_CUDA(c, set_smem(tri_block_kernel<double2, true>));
+  MOM_CUDA(c, set_smem(tri_block_kernel<float2, false>));
+  MOM_CUDA(c, set_smem(tri_block_kernel<float2, true>));
+  return MOM_OK;
+}
 
 // Solve A X = B (trans: A^T X = B) for nrhs columns (ld n) with the factors
 // of `precision` in place.  FP64: one triangular solve.  Mixed: x = 0,
