@@ -163,6 +163,28 @@ int alloc_representations(Ctx *c, int nga) {
   return MOM_OK;
 }
 
+// Room for the face-pair blocks of several group actions at once (the gather
+// adds them to the matrices in one pass) where it leaves the FP32 copies and
+// 4 GiB free; otherwise of fewer, down to what there is.
+void grow_blocks(Ctx *c, int nga) {
+  size_t one = 0;
+  for (const auto &D : c->dom) one = std::max(one, sizeof(double2) * 18 * (size_t)D.F * D.F);
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return;
+  const size_t keep = c->A_bytes / 2 + (size_t(4) << 30);
+  for (; nga > 1 && one * nga > c->blk_bytes; nga /= 2) {
+    double2 *b = nullptr;
+    if (fr < one * nga + keep) continue;
+    if (cudaMalloc(&b, one * nga) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    cudaFree(c->blk);
+    c->blk = b;
+    c->blk_bytes = one * nga;
+  }
+}
+
 }  // namespace mom
 
 using namespace mom;
@@ -247,6 +269,7 @@ int mom_gpu_set_symmetry(mom_ctx *c, int32_t nnames, const char *const *names, c
     }
   }
   MOM_TRY(alloc_representations(c, n));
+  grow_blocks(c, n);
   return MOM_OK;
 }
 

@@ -164,7 +164,7 @@ struct Ctx {
   float2 *A32 = nullptr;   // FP32 copy (LU in place in mixed mode)
   size_t A_bytes = 0, A32_bytes = 0;
   double2 *blk = nullptr;  // face-pair blocks [source F][test F][9][2] of the largest domain
-  size_t blk_bytes = 0;    //   or, when blk_fused, of every domain at blk + blk_off[d]
+  size_t blk_bytes = 0;    //   (for several group actions) or, when blk_fused, of every domain at blk + blk_off[d]
   bool blk_fused = false;
   std::vector<size_t> blk_off;  // [ndom], in double2
   int *dmap = nullptr;     // [ndom][N]: domain edge of each global edge, -1 if none
