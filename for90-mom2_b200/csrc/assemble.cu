@@ -105,9 +105,10 @@ __device__ __forceinline__ void zero(Cx<T> &a) {
 // points, GS for the source points, GD for the centroid offset; the adjoint
 // runs T = dual numbers on plain FP64 geometry (permittivity) or on one dual
 // and one plain face (vertex coordinates).
-template <typename T, int NQ, bool SMOOTH, bool LOSSLESS = false, typename G = T, typename GS = G, typename GD = G>
+template <typename T, int NQ, bool SMOOTH, bool LOSSLESS = false, int LANES = 1, typename G = T, typename GS = G,
+          typename GD = G>
 __device__ __forceinline__ void pair_moments(const G *rho_t, const GS *rho_s, int sstride, const GD d[3], T kr, T ki,
-                                             Moments<T> &M) {
+                                             Moments<T> &M, int lane = 0) {
   zero(M.TA);
   zero(M.TD);
   zero(M.KG);
@@ -122,7 +123,7 @@ __device__ __forceinline__ void pair_moments(const G *rho_t, const GS *rho_s, in
   // k^2 for the smoothed kernels
   const T k2r = kr * kr - ki * ki, k2i = 2 * kr * ki;
 #pragma unroll 1
-  for (int t = 0; t < NQ; t++) {
+  for (int t = LANES > 1 ? lane : 0; t < NQ; t += LANES) {
     const G rx = rho_t[3 * t], ry = rho_t[3 * t + 1], rz = rho_t[3 * t + 2];
     const G wt = (G)c_qw[t];
     const auto ax = d[0] + rx, ay = d[1] + ry, az = d[2] + rz;
@@ -627,11 +628,15 @@ struct NearArgs {
 };
 
 // Per wavelength, FP64: smoothed-G quadrature of each near pair (one thread
-// per pair) plus the closed-form terms; overwrites the pair's block.
-template <int NQ>
+// per pair, or LANES with every LANES-th test point each) plus the closed-form
+// terms; overwrites the pair's block.  Bound by the latency of a pair's serial
+// chain (169 point pairs and 9 edge pairs, 72 us).
+template <int NQ, int LANES>
 __global__ void __launch_bounds__(128) near_kernel(NearArgs a) {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= a.nnear) return;
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = (int)(idx % LANES);
+  const bool live = idx / LANES < a.nnear;  // the lanes of a pair agree
+  const int64_t j = live ? idx / LANES : 0;
   const int m = a.near_m[j], n = a.near_n[j];
   double d[3], mu[3][3], nu[3][3], slp[3], slq[3];
 #pragma unroll
@@ -646,7 +651,16 @@ __global__ void __launch_bounds__(128) near_kernel(NearArgs a) {
     }
   }
   Moments<double> Mt;
-  pair_moments<double, NQ, true>(a.tqrel + (size_t)m * NQ * 3, a.qrel + (size_t)n * NQ * 3, 1, d, a.kr, a.ki, Mt);
+  pair_moments<double, NQ, true, false, LANES>(a.tqrel + (size_t)m * NQ * 3, a.qrel + (size_t)n * NQ * 3, 1, d, a.kr,
+                                               a.ki, Mt, lane);
+  if (LANES > 1) {
+    double *mv = reinterpret_cast<double *>(&Mt);
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(Mt) / sizeof(double)); i++)
+#pragma unroll
+      for (int w = 1; w < LANES; w *= 2) mv[i] += __shfl_xor_sync(0xffffffffu, mv[i], w);
+  }
+  if (!live) return;
   double2 out[18];
   const Cd fD = {a.c1.re * kOofpi / 4.0, a.c1.im * kOofpi / 4.0};
   const Cd fH = {a.c2.re * kOofpi, a.c2.im * kOofpi};
@@ -658,6 +672,7 @@ __global__ void __launch_bounds__(128) near_kernel(NearArgs a) {
   double2 *dst = a.blk + ((size_t)n * a.F + m) * 18;
 #pragma unroll
   for (int i = 0; i < 9; i++) {
+    if (LANES > 1 && i % LANES != lane) continue;
     Cd dterm = {f4 * st[i] - f8.re * st[9 + i], -f8.im * st[9 + i]};
     Cd hterm = {f4 * st[18 + i] - f8.re * st[27 + i], -f8.im * st[27 + i]};
     Cd kterm = {f4 * st[36 + i] - f8.re * st[45 + i], -f8.im * st[45 + i]};
@@ -1105,6 +1120,20 @@ MediumConsts medium_consts(double omega, const double *ri, int d) {
   return m;
 }
 
+template <int LANES>
+int launch_near(Ctx *c, const NearArgs &na) {
+  const unsigned blocks = (unsigned)((na.nnear * LANES + 127) / 128);
+  switch (c->nq) {
+    case 1: near_kernel<1, LANES><<<blocks, 128, 0, c->stream>>>(na); break;
+    case 3: near_kernel<3, LANES><<<blocks, 128, 0, c->stream>>>(na); break;
+    case 4: near_kernel<4, LANES><<<blocks, 128, 0, c->stream>>>(na); break;
+    case 7: near_kernel<7, LANES><<<blocks, 128, 0, c->stream>>>(na); break;
+    case 13: near_kernel<13, LANES><<<blocks, 128, 0, c->stream>>>(na); break;
+    default: return fail(c, MOM_ERR_ARG, "unsupported number of quadrature points");
+  }
+  return MOM_OK;
+}
+
 // The face-pair blocks of domain d under group action g (pair_kernel for
 // every pair, then near_kernel over the near pairs) into blk.
 int domain_blocks(Ctx *c, int d, int g, double omega, const double *ri, int precision, double2 *blk) {
@@ -1177,16 +1206,13 @@ int domain_blocks(Ctx *c, int d, int g, double omega, const double *ri, int prec
         na.c2 = c2;
         na.k2 = {kr * kr - ki * ki, 2 * kr * ki};
         na.blk = blk;
-        const unsigned blocks = (unsigned)((nnear + 127) / 128);
         ProfScope ps(c, kProfNear);
-        switch (c->nq) {
-          case 1: near_kernel<1><<<blocks, 128, 0, c->stream>>>(na); break;
-          case 3: near_kernel<3><<<blocks, 128, 0, c->stream>>>(na); break;
-          case 4: near_kernel<4><<<blocks, 128, 0, c->stream>>>(na); break;
-          case 7: near_kernel<7><<<blocks, 128, 0, c->stream>>>(na); break;
-          case 13: near_kernel<13><<<blocks, 128, 0, c->stream>>>(na); break;
-          default: return fail(c, MOM_ERR_ARG, "unsupported number of quadrature points");
-        }
+        // Four lanes a pair while one would leave SMs without a CTA: two
+        // domains of 80 and 180 faces take 66 and 112 us instead of 156 and
+        // 161; beyond (320 faces, 167 against 173; 720, 318 against 312) the
+        // lanes only repeat the pair's last part.
+        if (nnear < 128 * (int64_t)c->nsm) MOM_TRY(launch_near<4>(c, na));
+        else MOM_TRY(launch_near<1>(c, na));
         c->launches++;
         MOM_CUDA(c, cudaGetLastError());
       }
