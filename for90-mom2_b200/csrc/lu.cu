@@ -656,7 +656,7 @@ struct TrsvArgs {
   int nb, P, rpc, ns;
   const void *inv;   // [nblk][2][nb][nb] (T): inv(L_kk), inv(U_kk)
   const int *perm;
-  double2 *X, *Y, *Z;  // [ns][n]: right-hand sides in X (solution returned there); the solved
+  double2 *X, *Y, *Z;  // [ns][n] (Y, Z of the kernel's NS >= ns columns): right-hand sides in X (solution returned there); the solved
                        // blocks of the forward pass are published in Y, of the backward pass in Z
                        // (both zeroed before the launch; published words carry a mark bit)
   int *timeout;
@@ -693,12 +693,12 @@ __device__ __forceinline__ T group_sum(T v, int g) {
   return v;
 }
 
-// ys = Inv * xs for an nb x nb block (column-major, element type T) and NS
-// vectors xs[sv * nb + j] (type T); `parts` adjacent lanes share one output
-// and reduce with shuffles.  The result goes to ys (FP64) and ysc (T).
+// Inv * xs for an nb x nb block (columns of inv ld apart, element type T) and
+// NS vectors xs[sv * nb + j] (type T); `parts` adjacent lanes share one output
+// and reduce with shuffles, one of them hands it to out(index sv * nb + r, sum).
 // tr: apply the transpose.  Requires nb a multiple of 64.
-template <typename T, int NS>
-__device__ void block_apply(const T *inv, int nb, const T *xs, double2 *ys, T *ysc, bool tr) {
+template <typename T, int NS, typename Out>
+__device__ __forceinline__ void block_apply(const T *inv, int nb, int ld, const T *xs, bool tr, Out out) {
   const int O = nb * NS;
   int parts = 1;
   while (parts * 2 * O <= (int)blockDim.x && parts < 16) parts *= 2;
@@ -710,8 +710,8 @@ __device__ void block_apply(const T *inv, int nb, const T *xs, double2 *ys, T *y
     T a0 = {0, 0}, a1 = {0, 0}, a2 = {0, 0}, a3 = {0, 0};
     if (valid) {
       for (int j = part; j < nb; j += 4 * parts) {
-        const T *i0 = tr ? inv + j + (size_t)r * nb : inv + r + (size_t)j * nb;
-        const size_t st = tr ? (size_t)parts : (size_t)parts * nb;
+        const T *i0 = tr ? inv + j + (size_t)r * ld : inv + r + (size_t)j * ld;
+        const size_t st = tr ? (size_t)parts : (size_t)parts * ld;
         cmac(a0, i0[0], xs[sv * nb + j]);
         cmac(a1, i0[st], xs[sv * nb + j + parts]);
         cmac(a2, i0[2 * st], xs[sv * nb + j + 2 * parts]);
@@ -719,12 +719,8 @@ __device__ void block_apply(const T *inv, int nb, const T *xs, double2 *ys, T *y
       }
     }
     const T acc = group_sum(cadd(cadd(a0, a1), cadd(a2, a3)), parts);
-    if (valid && part == 0) {
-      ys[o] = make_double2(acc.x, acc.y);
-      ysc[o] = acc;
-    }
+    if (valid && part == 0) out(o, acc);
   }
-  __syncthreads();
 }
 
 __device__ __forceinline__ void cp_async(void *smem, const void *gmem, int bytes_is_16) {
@@ -772,36 +768,45 @@ __device__ __forceinline__ bool read_word2(const double2 *p, double2 *v) {
 // block's rows first, solves and publishes it, and only then updates the
 // rest, so the critical path per block is one flag hand-off, one L2 read of
 // y_k, a 64-row update and one 64 x 64 apply; between consecutive blocks of
-// one CTA there is no hand-off at all.  The steps of both passes form one
+// one CTA there is no hand-off at all.  That path is a serial chain of 2 n / 64
+// steps; per step, FP64 at 3,840 unknowns, 3.7 us (4.2 with the inverses
+// unpadded in shared memory, four-way bank conflicts, and with three more
+// barriers between the update, the apply and the publication).  The steps of both passes
+// form one
 // sequence t = 0 .. 2 nblk - 1 (pass 0 block t, then pass 1 block
 // 2 nblk - 1 - t); the last block of pass 0 is the first of pass 1 and
 // stays with its owner.  TR solves A^T x = b: forward with U^T, backward
 // with L^T (unit), x = P^T z; its tile is the block row of U (L) right
 // (left) of the diagonal, row by row with a padded stride.
+template <typename T, bool TR>
+__host__ __device__ constexpr int trsv_pad() {
+  return TR ? 4 : 32 / (int)sizeof(T);
+}
 template <typename T, int NS, bool TR>
 __global__ void __launch_bounds__(256, 1) trsv_flow_kernel(TrsvArgs a) {
-  __shared__ double2 ysb[2][NS * 64];  // y of the current / next block (FP64)
-  __shared__ T ysc[2][NS * 64];        // the same in the factor's precision
+  __shared__ T ysc[2][NS * 64];        // y of the current / next block, in the factor's precision
   __shared__ T xsc[NS * 64];           // the block being solved, in the factor's precision
-  __shared__ int s_ok;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const T *M = reinterpret_cast<const T *>(a.M);
   const T *inv = reinterpret_cast<const T *>(a.inv);
   const int64_t n = a.n, lda = a.lda;
   const int nb = a.nb, nblk = (int)(n / nb), rpc = a.rpc, S = a.stages;
-  const int nsteps = 2 * nblk;
+  const int nsteps = 2 * nblk, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int kVec = 16 / (int)sizeof(T);  // elements per copy
   const int64_t r0 = (int64_t)blockIdx.x * rpc;
   const int64_t r1 = min(n, r0 + rpc);
-  // shared memory: own rows [NS][rpc] (double2) | inverses [S][nb][nb] | tiles [S]
+  // shared memory: own rows [NS][rpc] (double2) | inverses [S][nb][ci] | tiles [S]
   double2 *xo = reinterpret_cast<double2 *>(smem_raw);
   T *sinv = reinterpret_cast<T *>(smem_raw + sizeof(double2) * (size_t)NS * rpc);
   // tile element (row i, column j of the block): TR i * (nb + 1) + j, else
-  // j * cs + i with the column stride cs padded by 64 bytes, so that the
-  // lanes of a warp reading 4 columns of 8 rows hit distinct banks
-  const int cs = rpc + 64 / (int)sizeof(T);
+  // j * cs + i with the column stride cs padded by 32 bytes, so that the lanes
+  // of a quarter (FP32: half) warp reading 4 columns of 2 (4) rows hit distinct
+  // banks; the inverses' columns likewise (TR: 2 (4) columns of 4 rows)
+  const int cs = rpc + 32 / (int)sizeof(T);
+  const int ci = nb + trsv_pad<T, TR>();
   const size_t tile_elems = TR ? (size_t)rpc * (nb + 1) : (size_t)nb * cs;
   const size_t tile_stride = ((sizeof(T) * tile_elems + 15) / 16) * 16 / sizeof(T);
-  T *tiles = sinv + (size_t)S * nb * nb;
+  T *tiles = sinv + (size_t)S * nb * ci;
   auto blk_of = [&](int t) { return t < nblk ? t : nsteps - 1 - t; };
   auto pass_of = [&](int t) { return t < nblk ? 0 : 1; };
   auto owns = [&](int kb) { return (int64_t)kb * nb >= r0 && (int64_t)kb * nb < r1; };
@@ -816,15 +821,13 @@ __global__ void __launch_bounds__(256, 1) trsv_flow_kernel(TrsvArgs a) {
       const int cnt = hi <= lo ? 0 : (int)(hi - lo);
       T *tile = tiles + (size_t)(t % S) * tile_stride;
       if (TR) {
-        for (int idx = threadIdx.x; idx < cnt * nb; idx += blockDim.x) {
-          const int j = idx % nb, i = idx / nb;
-          cp_async(tile + (size_t)i * (nb + 1) + j, M + (k0 + j) + (lo + i) * lda, sizeof(T) == 16);
-        }
+        for (int i = warp; i < cnt; i += 8)
+          for (int j = lane; j < nb; j += 32)
+            cp_async(tile + (size_t)i * (nb + 1) + j, M + (k0 + j) + (lo + i) * lda, sizeof(T) == 16);
       } else {
-        for (int idx = threadIdx.x; idx < cnt * nb; idx += blockDim.x) {
-          const int i = idx % cnt, j = idx / cnt;
-          cp_async(tile + (size_t)j * cs + i, M + (lo + i) + (k0 + j) * lda, sizeof(T) == 16);
-        }
+        for (int j = warp; j < nb; j += 8)
+          for (int i = lane * kVec; i < cnt; i += 32 * kVec)
+            cp_async(tile + (size_t)j * cs + i, M + (lo + i) + (k0 + j) * lda, 1);
       }
     }
     const int u = t + 1;
@@ -832,8 +835,9 @@ __global__ void __launch_bounds__(256, 1) trsv_flow_kernel(TrsvArgs a) {
       // pass 0 applies inv(L) (or inv(U)^T), pass 1 inv(U) (or inv(L)^T)
       const int pu = pass_of(u);
       const T *ib = inv + ((size_t)blk_of(u) * 2 + (TR ? 1 - pu : pu)) * nb * nb;
-      T *dst = sinv + (size_t)(u % S) * nb * nb;
-      for (int idx = threadIdx.x; idx < nb * nb; idx += blockDim.x) cp_async(dst + idx, ib + idx, sizeof(T) == 16);
+      T *dst = sinv + (size_t)(u % S) * nb * ci;
+      for (int j = warp; j < nb; j += 8)
+        for (int i = lane * kVec; i < nb; i += 32 * kVec) cp_async(dst + j * ci + i, ib + j * nb + i, 1);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -845,10 +849,11 @@ __global__ void __launch_bounds__(256, 1) trsv_flow_kernel(TrsvArgs a) {
   // the tile rows from tlo.  G adjacent lanes share a row when there are few
   // rows (shuffle reduction); products and the 64-term sums in the factor's
   // precision, the running vector in FP64.  No barrier inside.
-  auto update = [&](int64_t k0, int64_t lo, int64_t hi, int64_t tlo, const T *tl, const T *y) {
+  // next: those rows are the block to solve, whose values go to xsc as well.
+  auto update = [&](int64_t k0, int64_t lo, int64_t hi, int64_t tlo, const T *tl, const T *y, bool next) {
     const int rows = hi > lo ? (int)(hi - lo) : 0;
     if (rows == 0) return;  // uniform over the CTA
-    const int G = NS > 2 ? 1 : (rows <= 64 ? 4 : (rows <= 128 ? 2 : 1));
+    const int G = NS > 2 || rows > 128 ? 1 : 4;
     const int part = threadIdx.x % G, rpr = (int)blockDim.x / G;
     const int64_t mstride = TR ? 1 : (a.direct ? lda : cs);
     for (int base = 0; base < rows; base += rpr) {
@@ -880,28 +885,30 @@ __global__ void __launch_bounds__(256, 1) trsv_flow_kernel(TrsvArgs a) {
           v.x -= (double)acc.x;
           v.y -= (double)acc.y;
           xo[(size_t)sv * rpc + li] = v;
+          if (next) st2(xsc + sv * nb + ri, v);
         }
       }
     }
   };
-  // solve the own block of step u from xo and publish it
-  auto solve_publish = [&](int u) {
+  // solve the own block of step u from xsc (staged: it is there; else from xo)
+  // and publish it
+  auto solve_publish = [&](int u, bool staged) {
     const int kb = blk_of(u), pu = pass_of(u);
     const int64_t l0 = (int64_t)kb * nb - r0;
-    for (int idx = threadIdx.x; idx < nb * NS; idx += blockDim.x) {
+    for (int idx = threadIdx.x; idx < nb * NS && !staged; idx += blockDim.x) {
       const int j = idx % nb, sv = idx / nb;
       st2(xsc + sv * nb + j, xo[(size_t)sv * rpc + l0 + j]);
     }
     __syncthreads();
-    double2 *y = ysb[u & 1];
-    block_apply<T, NS>(sinv + (size_t)(u % S) * nb * nb, nb, xsc, y, ysc[u & 1], TR);
+    T *yn = ysc[u & 1];
     double2 *E = pu == 0 ? a.Y : a.Z;
-    for (int idx = threadIdx.x; idx < nb * NS; idx += blockDim.x) {
-      const int j = idx % nb, sv = idx / nb;
-      const double2 v = y[sv * nb + j];
-      xo[(size_t)sv * rpc + l0 + j] = v;
+    block_apply<T, NS>(sinv + (size_t)(u % S) * nb * ci, nb, ci, xsc, TR, [&](int o, T acc) {
+      const int j = o % nb, sv = o / nb;
+      const double2 v = make_double2(acc.x, acc.y);
       publish_word2(E + (size_t)sv * n + (int64_t)kb * nb + j, v);
-    }
+      yn[o] = acc;
+      xo[(size_t)sv * rpc + l0 + j] = v;
+    });
     __syncthreads();
   };
   // own rows of P X (TR: X)
@@ -909,12 +916,12 @@ __global__ void __launch_bounds__(256, 1) trsv_flow_kernel(TrsvArgs a) {
   for (int idx = threadIdx.x; idx < NS * nrow; idx += blockDim.x) {
     const int li = idx % nrow, sv = idx / nrow;
     const int64_t i = r0 + li;
-    xo[(size_t)sv * rpc + li] = a.X[(size_t)sv * n + (TR ? i : a.perm[i])];
+    xo[(size_t)sv * rpc + li] = sv < a.ns ? a.X[(size_t)sv * n + (TR ? i : a.perm[i])] : make_double2(0, 0);
   }
   for (int t = -1; t <= S - 2; t++) issue(t);
   wait_stage();
   __syncthreads();
-  if (owns(blk_of(0))) solve_publish(0);
+  if (owns(blk_of(0))) solve_publish(0, false);
   __syncthreads();
   issue(S - 1);
   for (int t = 0; t < nsteps; t++) {
@@ -924,60 +931,43 @@ __global__ void __launch_bounds__(256, 1) trsv_flow_kernel(TrsvArgs a) {
     upd_range(pass, k0, nb, r0, r1, &lo, &hi);
     const int u = t + 1;
     const bool own_next = u < nsteps && owns(blk_of(u));
+    wait_stage();
+    bool ok = true;
     if ((hi > lo || own_next) && !owns(kb)) {
       // poll the published words of block kb until all are marked (bounded)
       const double2 *E = pass == 0 ? a.Y : a.Z;
-      long long it = 0;
-      while (true) {
-        int ok = 1;
-        for (int idx = threadIdx.x; idx < nb * NS; idx += blockDim.x) {
-          const int j = idx % nb, sv = idx / nb;
-          double2 v;
-          if (read_word2(E + (size_t)sv * n + k0 + j, &v)) {
-            st2(&ysc[t & 1][sv * nb + j], v);
-          } else {
-            ok = 0;
-          }
+      for (int idx = threadIdx.x; idx < nb * NS && ok; idx += blockDim.x) {
+        const int j = idx % nb, sv = idx / nb;
+        double2 v;
+        long long it = 0;
+        while (!read_word2(E + (size_t)sv * n + k0 + j, &v)) {
+          if ((++it & 255) != 0 && it <= a.spin) continue;
+          if (it > a.spin) atomicExch(a.timeout, 1);
+          ok = it <= a.spin && *(volatile int *)a.timeout == 0;
+          if (!ok) break;
         }
-        if (__syncthreads_and(ok)) break;
-        if ((++it & 255) == 0 || it > a.spin) {
-          if (threadIdx.x == 0) {
-            int go = 1;
-            if (*(volatile int *)a.timeout) go = 0;
-            else if (it > a.spin) {
-              atomicExch(a.timeout, 1);
-              go = 0;
-            }
-            s_ok = go;
-          }
-          __syncthreads();
-          if (!s_ok) {
-            cp_async_wait_all();
-            return;
-          }
-        }
+        st2(&ysc[t & 1][sv * nb + j], v);
       }
     }
-    wait_stage();
-    __syncthreads();
+    if (!__syncthreads_and(ok)) {  // a wait ran out, here or in another CTA
+      cp_async_wait_all();
+      return;
+    }
     const T *tl = tiles + (size_t)(t % S) * tile_stride;
     const T *yc = ysc[t & 1];
     if (own_next) {
       const int64_t a0 = (int64_t)blk_of(u) * nb;
       const bool same = pass_of(u) == pass;
+      if (same) update(k0, a0, a0 + nb, lo, tl, yc, true);
+      solve_publish(u, same);
       if (same) {
-        update(k0, a0, a0 + nb, lo, tl, yc);
-        __syncthreads();
-      }
-      solve_publish(u);
-      if (same) {
-        update(k0, lo, a0, lo, tl, yc);
-        update(k0, a0 + nb, hi, lo, tl, yc);
+        update(k0, lo, a0, lo, tl, yc, false);
+        update(k0, a0 + nb, hi, lo, tl, yc, false);
       } else {
-        update(k0, lo, hi, lo, tl, yc);
+        update(k0, lo, hi, lo, tl, yc, false);
       }
     } else {
-      update(k0, lo, hi, lo, tl, yc);
+      update(k0, lo, hi, lo, tl, yc, false);
     }
     __syncthreads();
     issue(t + S);
@@ -987,24 +977,35 @@ __global__ void __launch_bounds__(256, 1) trsv_flow_kernel(TrsvArgs a) {
   for (int idx = threadIdx.x; idx < NS * nrow; idx += blockDim.x) {
     const int li = idx % nrow, sv = idx / nrow;
     const int64_t i = r0 + li;
-    a.X[(size_t)sv * n + (TR ? a.perm[i] : i)] = xo[(size_t)sv * rpc + li];
+    if (sv < a.ns) a.X[(size_t)sv * n + (TR ? a.perm[i] : i)] = xo[(size_t)sv * rpc + li];
   }
 }
 
 constexpr int kGemvRows = 256;
 constexpr int kGemvCols = 256;
 
-// partial[chunk][s][i] = sum_{j in chunk} A[i, j] x_s[j]  (FP64 matrix)
+// Columns per chunk: kGemvCols, or fewer so that small matrices still give each
+// SM four CTAs (2,160 unknowns: 306 CTAs instead of 81, 60 us instead of 103).
+inline int gemv_cols(const Ctx *c, int64_t n) {
+  const int64_t rblocks = (n + kGemvRows - 1) / kGemvRows;
+  int cols = kGemvCols;
+  while (cols > 32 && rblocks * ((n + cols - 1) / cols) < 4 * c->nsm) cols /= 2;
+  return cols;
+}
+
+// partial[chunk][s][i] = sum_{j in chunk} A[i, j] x_s[j]  (FP64 matrix),
+// gridDim.y chunks of `cols` columns
 template <int NS>
 __global__ void __launch_bounds__(kGemvRows) gemv_partial_kernel(const double2 *A, int64_t lda, int64_t n,
-                                                                 const double2 *X, int64_t ldx, double2 *partial) {
+                                                                 const double2 *X, int64_t ldx, int nv, int cols,
+                                                                 double2 *partial) {
   __shared__ double2 xs[NS][kGemvCols];
   const int64_t i = (int64_t)blockIdx.x * kGemvRows + threadIdx.x;
-  const int64_t j0 = (int64_t)blockIdx.y * kGemvCols;
-  const int cnt = (n - j0) < kGemvCols ? (int)(n - j0) : kGemvCols;
+  const int64_t j0 = (int64_t)blockIdx.y * cols;
+  const int cnt = (n - j0) < cols ? (int)(n - j0) : cols;
   for (int idx = threadIdx.x; idx < cnt * NS; idx += kGemvRows) {
     const int j = idx % cnt, s = idx / cnt;
-    xs[s][j] = X[(size_t)s * ldx + j0 + j];
+    xs[s][j] = NS <= 2 || s < nv ? X[(size_t)s * ldx + j0 + j] : make_double2(0, 0);
   }
   __syncthreads();
   if (i >= n) return;
@@ -1029,7 +1030,7 @@ __global__ void __launch_bounds__(kGemvRows) gemv_partial_kernel(const double2 *
 // warp per column, lanes stride down the column.
 template <int NS>
 __global__ void __launch_bounds__(256) gemv_t_kernel(const double2 *A, int64_t lda, int64_t n, const double2 *X,
-                                                     int64_t ldx, double2 *Y) {
+                                                     int64_t ldx, int nv, double2 *Y) {
   const int lane = threadIdx.x & 31;
   const int64_t j = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (j >= n) return;
@@ -1041,7 +1042,7 @@ __global__ void __launch_bounds__(256) gemv_t_kernel(const double2 *A, int64_t l
     const double2 m = __ldcs(col + i);
 #pragma unroll
     for (int s = 0; s < NS; s++) {
-      const double2 x = X[(size_t)s * ldx + i];
+      const double2 x = X[(size_t)(NS <= 2 ? s : min(s, nv - 1)) * ldx + i];
       acc[s].x += m.x * x.x - m.y * x.y;
       acc[s].y += m.x * x.y + m.y * x.x;
     }
@@ -1810,8 +1811,14 @@ int lu_factor_t(Ctx *c, T *A, int precision, int batch) {
   return MOM_OK;
 }
 
+// Vectors that the single-launch solve and the residual take at a time: 8, 4, 2
+// or 1, the last chunk filled up with zero columns: a launch costs nearly the
+// same for any number (FP32 at 7,260 unknowns, three vectors as four 0.99 ms, as
+// two and one 1.50; seven 1.53 and 2.52).
+inline int chunk_of(int left) { return left > 4 ? 8 : left > 2 ? 4 : left; }
+
 // X (n x nrhs, ld n) <- A^{-1} X (TR: A^{-T} X) with the factors in place;
-// Y is scratch.
+// Y and Z are scratch of nrhs columns rounded up to whole chunks.
 template <typename T, bool TR = false>
 int getrs_t(Ctx *c, const T *A, double2 *X, double2 *Y, double2 *Z, int nrhs) {
   const int64_t n = c->n;
@@ -1828,12 +1835,12 @@ int getrs_t(Ctx *c, const T *A, double2 *X, double2 *Y, double2 *Z, int nrhs) {
            : ns == 4 ? (void *)trsv_flow_kernel<T, 4, TR>
                      : (void *)trsv_flow_kernel<T, 8, TR>;
   };
-  const size_t tile_elems = TR ? (size_t)rpc * (nb + 1) : (size_t)nb * (rpc + 64 / sizeof(T));
-  const size_t tile_bytes = ((sizeof(T) * tile_elems + 15) / 16) * 16, inv_bytes = sizeof(T) * nb * nb;
+  const size_t tile_elems = TR ? (size_t)rpc * (nb + 1) : (size_t)nb * (rpc + 32 / sizeof(T));
+  const size_t tile_bytes = ((sizeof(T) * tile_elems + 15) / 16) * 16,
+               inv_bytes = sizeof(T) * nb * (nb + trsv_pad<T, TR>());
   const T *inv = sizeof(T) == sizeof(float2) ? (const T *)c->inv32 : (const T *)c->invd;
   for (int s0 = 0, ns = 0; s0 < nrhs; s0 += ns) {
-    ns = 8;
-    while (ns > nrhs - s0) ns >>= 1;  // chunks of 8, 4, 2, 1 vectors
+    ns = chunk_of(nrhs - s0);
     // shared memory: own rows, then per stage one inverse and (unless direct) one tile
     int stages = 0, direct = 0;
     size_t smem = 0;
@@ -1861,7 +1868,7 @@ int getrs_t(Ctx *c, const T *A, double2 *X, double2 *Y, double2 *Z, int nrhs) {
     ta.nb = nb;
     ta.P = P;
     ta.rpc = rpc;
-    ta.ns = ns;
+    ta.ns = std::min(ns, nrhs - s0);
     ta.inv = inv;
     ta.perm = c->perm;
     ta.X = X + (size_t)s0 * n;
@@ -2277,13 +2284,14 @@ int lu_solve_ex(Ctx *c, int precision, int trans, const double2 *B, double2 *X, 
   const int64_t n = c->n;
   if (c->factored != precision) return fail(c, MOM_ERR_STATE, "matrix not factored in this precision");
   const size_t vec = sizeof(double2) * (size_t)n * nrhs;
+  const size_t vecp = sizeof(double2) * (size_t)n * (nrhs / 8 * 8 + chunk_of(nrhs % 8));  // whole chunks
   if (precision == MOM_PREC_FP64) {
     if (X != B) MOM_CUDA(c, cudaMemcpyAsync(X, B, vec, cudaMemcpyDeviceToDevice, c->stream));
     if (nrhs >= kMultiRhs) {
       MOM_TRY(getrs_multi<double2>(c, c->A, X, nrhs, trans));
     } else {
-      MOM_TRY(ensure_buffer(c, &c->ws, &c->ws_bytes, 2 * vec));
-      double2 *Yw = (double2 *)c->ws, *Zw = (double2 *)((char *)c->ws + vec);
+      MOM_TRY(ensure_buffer(c, &c->ws, &c->ws_bytes, 2 * vecp));
+      double2 *Yw = (double2 *)c->ws, *Zw = (double2 *)((char *)c->ws + vecp);
       if (trans) MOM_TRY((getrs_t<double2, true>(c, c->A, X, Yw, Zw, nrhs)));
       else MOM_TRY((getrs_t<double2, false>(c, c->A, X, Yw, Zw, nrhs)));
     }
@@ -2294,13 +2302,13 @@ int lu_solve_ex(Ctx *c, int precision, int trans, const double2 *B, double2 *X, 
     if (tmo) return fail(c, MOM_ERR_TIMEOUT, "triangular solve barrier timed out");
     return MOM_OK;
   }
-  const int nchunk = (int)((n + kGemvCols - 1) / kGemvCols);
+  const int cols = gemv_cols(c, n), nchunk = (int)((n + cols - 1) / cols);
   const int rblocks = (int)((n + 255) / 256);
-  const size_t off_r = 0, off_d = vec, off_y = 2 * vec, off_p = 3 * vec;
+  const size_t off_r = 0, off_d = vec, off_y = 2 * vec, off_p = 2 * vec + vecp;
   const size_t part = sizeof(double2) * (size_t)nchunk * 8 * n;
   const size_t off_n = off_p + part;
   const size_t off_z = off_n + ((sizeof(double) * rblocks * nrhs + 255) / 256) * 256;
-  MOM_TRY(ensure_buffer(c, &c->ws, &c->ws_bytes, off_z + vec + 256));
+  MOM_TRY(ensure_buffer(c, &c->ws, &c->ws_bytes, off_z + vecp + 256));
   char *ws = (char *)c->ws;
   double2 *R = (double2 *)(ws + off_r), *Dv = (double2 *)(ws + off_d), *Yv = (double2 *)(ws + off_y),
           *Pp = (double2 *)(ws + off_p), *Zv = (double2 *)(ws + off_z);
@@ -2338,25 +2346,25 @@ int lu_solve_ex(Ctx *c, int precision, int trans, const double2 *B, double2 *X, 
       c->launches++;
     }
     for (int s0 = 0, ns = 0; !multi && s0 < nrhs; s0 += ns) {
-      ns = 8;
-      while (ns > nrhs - s0) ns >>= 1;
+      ns = chunk_of(nrhs - s0);
+      const int nv = std::min(ns, nrhs - s0);
       const double2 *xs0 = X + (size_t)s0 * n;
       int nch = nchunk;
       if (trans) {
         const unsigned gb = (unsigned)((n + 7) / 8);
-        if (ns == 1) gemv_t_kernel<1><<<gb, 256, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
-        else if (ns == 2) gemv_t_kernel<2><<<gb, 256, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
-        else if (ns == 4) gemv_t_kernel<4><<<gb, 256, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
-        else gemv_t_kernel<8><<<gb, 256, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
+        if (ns == 1) gemv_t_kernel<1><<<gb, 256, 0, c->stream>>>(c->A, c->lda, n, xs0, n, nv, Pp);
+        else if (ns == 2) gemv_t_kernel<2><<<gb, 256, 0, c->stream>>>(c->A, c->lda, n, xs0, n, nv, Pp);
+        else if (ns == 4) gemv_t_kernel<4><<<gb, 256, 0, c->stream>>>(c->A, c->lda, n, xs0, n, nv, Pp);
+        else gemv_t_kernel<8><<<gb, 256, 0, c->stream>>>(c->A, c->lda, n, xs0, n, nv, Pp);
         nch = 1;
       } else {
         const dim3 gg(rblocks, nchunk);
-        if (ns == 1) gemv_partial_kernel<1><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
-        else if (ns == 2) gemv_partial_kernel<2><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
-        else if (ns == 4) gemv_partial_kernel<4><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
-        else gemv_partial_kernel<8><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
+        if (ns == 1) gemv_partial_kernel<1><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, nv, cols, Pp);
+        else if (ns == 2) gemv_partial_kernel<2><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, nv, cols, Pp);
+        else if (ns == 4) gemv_partial_kernel<4><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, nv, cols, Pp);
+        else gemv_partial_kernel<8><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, nv, cols, Pp);
       }
-      residual_kernel<<<dim3(rblocks, ns), 256, 0, c->stream>>>(B + (size_t)s0 * n, n, Pp, nch, n, ns,
+      residual_kernel<<<dim3(rblocks, nv), 256, 0, c->stream>>>(B + (size_t)s0 * n, n, Pp, nch, n, ns,
                                                                 R + (size_t)s0 * n, n, rn2 + (size_t)s0 * rblocks);
       c->launches += 2;
     }
@@ -2386,7 +2394,7 @@ int lu_solve_ex(Ctx *c, int precision, int trans, const double2 *B, double2 *X, 
 
 int matvec_acc(Ctx *c, const double2 *X, int nrhs, double2 *Y, double sign) {
   const int64_t n = c->n;
-  const int nchunk = (int)((n + kGemvCols - 1) / kGemvCols);
+  const int cols = gemv_cols(c, n), nchunk = (int)((n + cols - 1) / cols);
   const int rblocks = (int)((n + kGemvRows - 1) / kGemvRows);
   MOM_TRY(ensure_buffer(c, &c->ws, &c->ws_bytes, sizeof(double2) * (size_t)nchunk * 8 * n));
   double2 *Pp = (double2 *)c->ws;
@@ -2395,10 +2403,10 @@ int matvec_acc(Ctx *c, const double2 *X, int nrhs, double2 *Y, double sign) {
     while (ns > nrhs - s0) ns >>= 1;
     const double2 *xs0 = X + (size_t)s0 * n;
     const dim3 gg(rblocks, nchunk);
-    if (ns == 1) gemv_partial_kernel<1><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
-    else if (ns == 2) gemv_partial_kernel<2><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
-    else if (ns == 4) gemv_partial_kernel<4><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
-    else gemv_partial_kernel<8><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, Pp);
+    if (ns == 1) gemv_partial_kernel<1><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, ns, cols, Pp);
+    else if (ns == 2) gemv_partial_kernel<2><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, ns, cols, Pp);
+    else if (ns == 4) gemv_partial_kernel<4><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, ns, cols, Pp);
+    else gemv_partial_kernel<8><<<gg, kGemvRows, 0, c->stream>>>(c->A, c->lda, n, xs0, n, ns, cols, Pp);
     acc_partials_kernel<<<dim3((unsigned)((n + 255) / 256), ns), 256, 0, c->stream>>>(Y + (size_t)s0 * n, n, Pp,
                                                                                      nchunk, n, ns, sign);
     c->launches += 2;
