@@ -734,11 +734,15 @@ int mom_gpu_sweep_many(int32_t nctx, mom_ctx **ctx, const int32_t *nwl, const do
   std::vector<std::thread> th;
   th.reserve(nctx);
   for (int i = 0; i < nctx; i++)
+    if (ctx[i]) ctx[i]->crowded = nctx >= kCrowd;
+  for (int i = 0; i < nctx; i++)
     th.emplace_back([&, i]() {
       st[i] = mom_gpu_sweep(ctx[i], nwl[i], omega[i], ri[i], nsrc, src, precision, tol, maxit, csca[i], cabs[i],
                             nullptr);
     });
   for (auto &t : th) t.join();
+  for (int i = 0; i < nctx; i++)
+    if (ctx[i]) ctx[i]->crowded = false;
   int rc = MOM_OK;
   for (int i = 0; i < nctx; i++) {
     if (status) status[i] = st[i];

@@ -1635,9 +1635,12 @@ int lu_enqueue_cluster(Ctx *c, T *A, const LuWork &w, int batch) {
     }
     return MOM_OK;
   };
+  const bool ahead = c->lookahead && !c->crowded;
   // stream 2 joins the stream (and any capture open on it)
-  MOM_CUDA(c, cudaEventRecord(c->la_ev[0], sa));
-  MOM_CUDA(c, cudaStreamWaitEvent(sb, c->la_ev[0], 0));
+  if (ahead) {
+    MOM_CUDA(c, cudaEventRecord(c->la_ev[0], sa));
+    MOM_CUDA(c, cudaStreamWaitEvent(sb, c->la_ev[0], 0));
+  }
   MOM_TRY(panel(0, sa, false));
   for (int64_t j0 = 0; j0 < n; j0 += nb) {
     const int64_t t0 = j0 + nb;
@@ -1645,7 +1648,7 @@ int lu_enqueue_cluster(Ctx *c, T *A, const LuWork &w, int batch) {
       MOM_TRY(swaps(j0, 0, 0, j0, c->perm));
       break;
     }
-    if (c->lookahead && t0 + nb < n) {
+    if (ahead && t0 + nb < n) {
       MOM_TRY(swaps(j0, t0, t0 + nb, 0, nullptr));
       MOM_TRY(update(j0, t0, t0 + nb, 0, false));
       MOM_CUDA(c, cudaEventRecord(c->la_ev[1], sa));
@@ -1662,8 +1665,10 @@ int lu_enqueue_cluster(Ctx *c, T *A, const LuWork &w, int batch) {
     }
   }
   // stream 2 rejoins stream 1 (closes any capture branch it holds)
-  MOM_CUDA(c, cudaEventRecord(c->la_ev[2], sb));
-  MOM_CUDA(c, cudaStreamWaitEvent(sa, c->la_ev[2], 0));
+  if (ahead) {
+    MOM_CUDA(c, cudaEventRecord(c->la_ev[2], sb));
+    MOM_CUDA(c, cudaStreamWaitEvent(sa, c->la_ev[2], 0));
+  }
   {
     // the inverses of every diagonal block, which the solves need
     ProfScope pd(c, kProfDiagInv);
@@ -1764,7 +1769,7 @@ int lu_factor_t(Ctx *c, T *A, int precision, int batch) {
                                         (uintptr_t)wait_polls(c, 0), (uintptr_t)wait_polls(c, 1),
                                         (uintptr_t)use_lookahead(c, precision), (uintptr_t)c->lookahead,
                                         (uintptr_t)batch,       (uintptr_t)c->panel_cluster, (uintptr_t)c->la_ctas,
-                                        (uintptr_t)(c->la_from * 1e6)};
+                                        (uintptr_t)(c->la_from * 1e6), (uintptr_t)c->crowded};
     for (Ctx::LuGraph *h : c->lu_graphs)
       if (h->exec && h->key == key) g = h;
     if (!g) {
