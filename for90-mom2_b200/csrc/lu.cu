@@ -1137,6 +1137,16 @@ struct LuWork {
 constexpr int kXSlots = 16;
 constexpr size_t kXSlotBytes = 128 << 10;
 
+// Panels per outer block (MOM_LU_OUTER, else): three in the mixed path below
+// 16,384 unknowns, where the chain of panels and narrow updates bounds the
+// factorisation and a shorter block makes the narrow updates cheaper; four from
+// there on, where the wide updates' memory traffic does.  Whole calls, four and
+// three: 8,640 unknowns 32.2 and 30.0 ms, 11,760 55.8 and 54.1, 15,360 92.2 and
+// 91.0, 17,340 120.3 and 121.3, 34,560 650 and 675.
+int outer_of(const Ctx *c, bool f32) {
+  return c->outer_panels > 0 ? c->outer_panels : f32 && c->n < 16384 ? 3 : 4;
+}
+
 // slot < 0: the tuned placement (0 without a table)
 int lu_workspace(Ctx *c, int precision, LuWork &w, int slot = -1) {
   const int nb = c->nb, P = c->nsm;
@@ -1158,7 +1168,7 @@ int lu_workspace(Ctx *c, int precision, LuWork &w, int slot = -1) {
   const size_t o_map = take(sizeof(int) * 256 * 2 * kMaxGroup);
   const size_t o_w2 = take(esz * (size_t)nb * 16 * nb);
   const size_t o_tc =
-      take(precision == MOM_PREC_MIXED ? tc_cgemm_work_bytes((int)c->n, (int)c->n, c->outer_panels * nb) : 0);
+      take(precision == MOM_PREC_MIXED ? tc_cgemm_work_bytes((int)c->n, (int)c->n, outer_of(c, true) * nb) : 0);
   MOM_TRY(ensure_buffer(c, &c->ws, &c->ws_bytes, off));
   char *b = (char *)c->ws;
   char *x = b + o_x + (size_t)slot * kXSlotBytes;
@@ -1293,7 +1303,7 @@ int lu_enqueue(Ctx *c, T *A, int precision, const LuWork &w) {
                                   cudaMemcpyDeviceToDevice, c->stream));
     return MOM_OK;
   };
-  const int NB = c->outer_panels * nb;  // outer block: trailing updates run with K = NB
+  const int NB = outer_of(c, precision == MOM_PREC_MIXED) * nb;  // outer block: trailing updates run with K = NB
   for (int64_t J0 = 0; J0 < n; J0 += NB) {
     const int64_t NBc = std::min<int64_t>(NB, n - J0);
     for (int64_t j0 = J0; j0 < J0 + NBc; j0 += nb) {
@@ -1372,7 +1382,7 @@ int lu_enqueue(Ctx *c, T *A, int precision, const LuWork &w) {
 }
 
 // The mixed-precision factorisation with look-ahead.  Right-looking over
-// outer blocks of NB = outer_panels * 64 columns as lu_enqueue, reordered so
+// outer blocks of NB = outer_of() * 64 columns as lu_enqueue, reordered so
 // that the next outer block is factored on the second stream while the
 // trailing update of the current one runs:
 //   stream 1: J's interchanges on every column outside J; the block-row
@@ -1396,7 +1406,7 @@ template <typename T>
 int lu_enqueue_la(Ctx *c, T *A, const LuWork &w) {
   const int64_t n = c->n, lda = c->lda;
   const int nb = c->nb;
-  const int NB = c->outer_panels * nb;
+  const int NB = outer_of(c, true) * nb;
   cudaStream_t sa = c->stream, sb = c->stream2;
   if (sizeof(T) != sizeof(float2)) return fail(c, MOM_ERR_ARG, "the look-ahead schedule serves the mixed path");
   MOM_CUDA(c, cudaMemsetAsync(c->dinfo, 0, sizeof(int) * 4, sa));
@@ -1574,9 +1584,9 @@ int lu_enqueue_la(Ctx *c, T *A, const LuWork &w) {
 // mixed calls, tensor cores against library FP32 GEMMs: 2,160 unknowns 4.96 and
 // 5.05 ms, 2,940 6.8 and 7.1 ms, 4,860 12.6 and 16.2 ms; no difference below).
 constexpr int64_t kTcFromOrder = 2048;
-// From this order on the FP32 factorisation goes by outer blocks of 256 columns
-// (lu_enqueue_la): its updates read and write the trailing matrix four times
-// less, which the 64-column updates are bound by.  Whole calls, 256 against 64
+// From this order on the FP32 factorisation goes by outer blocks (lu_enqueue_la):
+// its updates read and write the trailing matrix three or four times less, which
+// the 64-column updates are bound by.  Whole calls, blocks of 256 against 64
 // columns: 7,260 unknowns 25.4 and 24.3 ms, 8,640 33.0 and 33.7 ms, 11,760 56.9
 // and 67.3 ms.
 constexpr int64_t kOuterFromOrder = 8192;
@@ -1694,8 +1704,8 @@ int lu_issue(Ctx *c, T *A, int precision, const LuWork &w, int batch);
 // The look-ahead schedule serves the mixed path (tensor-core trailing
 // updates) with at least two outer blocks.
 bool use_lookahead(const Ctx *c, int precision) {
-  return c->lookahead && precision == MOM_PREC_MIXED && c->outer_panels <= 16 &&
-         c->n > 2 * (int64_t)c->outer_panels * c->nb;
+  return c->lookahead && precision == MOM_PREC_MIXED && outer_of(c, true) <= 16 &&
+         c->n > 2 * (int64_t)outer_of(c, true) * c->nb;
 }
 
 // Captures the factorisation of this precision into g (replacing what g held).
@@ -1765,7 +1775,7 @@ int lu_factor_t(Ctx *c, T *A, int precision, int batch) {
                                         (uintptr_t)A,         (uintptr_t)c->ws,    (uintptr_t)c->ws_bytes,
                                         (uintptr_t)c->ipiv,   (uintptr_t)c->invd,  (uintptr_t)c->perm,
                                         (uintptr_t)c->dinfo,  (uintptr_t)c->nsm,   (uintptr_t)c->prof,
-                                        (uintptr_t)tune_hash(c), (uintptr_t)c->outer_panels, (uintptr_t)c->inv32,
+                                        (uintptr_t)tune_hash(c), (uintptr_t)outer_of(c, precision == MOM_PREC_MIXED), (uintptr_t)c->inv32,
                                         (uintptr_t)wait_polls(c, 0), (uintptr_t)wait_polls(c, 1),
                                         (uintptr_t)use_lookahead(c, precision), (uintptr_t)c->lookahead,
                                         (uintptr_t)batch,       (uintptr_t)c->panel_cluster, (uintptr_t)c->la_ctas,

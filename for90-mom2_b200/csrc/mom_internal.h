@@ -231,7 +231,7 @@ struct Ctx {
   // too tall for it (over 32,768 rows in FP32, 16,384 in FP64 with 16 CTAs) on
   // CTAs that exchange through global memory.
   int panel_cluster = 0;
-  int outer_panels = 4;  // panels per outer block of the LU (MOM_LU_OUTER): trailing GEMMs have K = 64 * this
+  int outer_panels = 0;  // panels per outer block of the LU (MOM_LU_OUTER; 0: by order): trailing GEMMs have K = 64 * this
   // Permittivity gradients by the point-pair forms of adjoint_eps_impl.cuh;
   // MOM_ADJ_EPS_PLAIN=0 selects the all-dual adj_pair_kernel.
   int adj_eps_plain = 1;
