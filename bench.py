@@ -421,13 +421,13 @@ def run_ours(args, rank, local_rank, world):
     if cnt:
         bytes_ = sum(2.0 * 8 * (n - k * nb) * nb for k in range(n // nb)) * psteps  # FP32 panel read + write
         ach = bytes_ / (ms * 1e-3) / 1e9
-        # DRAM bytes of one panel launch at m = 3520 rows (ncu capture of the panel
-        # kernel), scaled by rows to the average panel height of this order
-        traffic = 1.841e6 * (n / 2.0) / 3520.0
-        roofs["panel"] = {"kernel": "panel_kernel<float2> (pivoted panel, one device-wide exchange per column)",
+        # DRAM bytes of one panel (four subpanels of 0.539 MB, ncu capture at 3,648
+        # rows), scaled by rows to the average panel height of this order
+        traffic = 4 * 0.539e6 * (n / 2.0) / 3648.0
+        roofs["panel"] = {"kernel": "panel_reg_kernel<float2> (pivoted panel in the registers of one cluster, one exchange per column)",
                           "bound": "hbm", "achieved": ach, "unit": "GB/s", "peak": hbm_gbs, "frac": ach / hbm_gbs,
-                          "traffic": traffic, "traffic_note": "bytes per launch, ncu at 3520 rows scaled by rows",
-                          "peak_note": "%s; latency-bound: one device-wide pivot exchange per column" % peak_src}
+                          "traffic": traffic, "traffic_note": "bytes per launch, ncu at 3648 rows scaled by rows",
+                          "peak_note": "%s; latency-bound: one pivot exchange per column over the cluster" % peak_src}
     ms, cnt = prof["pair"]
     if cnt:
         # 169 point pairs x 88 FLOP per unordered face pair (each evaluated once and
