@@ -105,10 +105,11 @@ __device__ __forceinline__ double2 mul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 // 1 / z, zero for a zero z, with |z|^2 near one after a scaling by a power of
-// two, its reciprocal by one iteration from the hardware estimate, and no
+// two, its reciprocal by Newton-Raphson from the hardware estimate, and no
 // branch, so that the chain overlaps the update.  FP32: |z|^2 and the
-// reciprocal as sums of two FP32 numbers, so the quotients round once (the
-// same in FP64 arithmetic measured 150 cycles more per column).
+// reciprocal as sums of two FP32 numbers (Dekker's double-length arithmetic),
+// so the quotients round once (the same in FP64 arithmetic measured 150 cycles
+// more per column).
 __device__ __forceinline__ float2 recip_of(float2 z) {
   const unsigned e = max(__float_as_uint(z.x) & 0x7f800000u, __float_as_uint(z.y) & 0x7f800000u);
   const float s = __uint_as_float(0x7f000000u - min(e, 0x7e800000u));
@@ -122,15 +123,16 @@ __device__ __forceinline__ float2 recip_of(float2 z) {
   const float qx = xh + (fmaf(x, r, -xh) + x * rl), qy = yh + (fmaf(y, r, -yh) + y * rl);
   return d != 0.0f ? make_float2(qx * s, -qy * s) : make_float2(0.f, 0.f);
 }
-// FP64: a third-order iteration, and one residual correction of the quotients.
+// FP64: one Newton-Raphson step for the reciprocal from the FP32 estimate of
+// |z|^2 (2^-104 at least after the scaling, so in FP32's range), to 2^-45, and
+// one step of iterative refinement of the quotients, x / d + (x - q d) / d.
 __device__ __forceinline__ double2 recip_of(double2 z) {
   const unsigned e = max((unsigned)__double2hiint(z.x) & 0x7ff00000u, (unsigned)__double2hiint(z.y) & 0x7ff00000u);
   const double s = __hiloint2double((int)(0x7fd00000u - min(e, 0x7fc00000u)), 0);
   const double x = z.x * s, y = z.y * s, d = fma(x, x, y * y);
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double t = fma(-d, r, 1.0);
-  r = fma(r, fma(t, t, t), r);
+  float r0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"((float)d));
+  const double r = fma((double)r0, fma(-d, (double)r0, 1.0), (double)r0);
   double qx = x * r, qy = y * r;
   qx = fma(fma(-qx, d, x), r, qx);
   qy = fma(fma(-qy, d, y), r, qy);

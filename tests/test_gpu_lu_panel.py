@@ -45,6 +45,29 @@ def test_general_matrix(subdiv, prec, kind):
     s.close()
 
 
+@pytest.mark.parametrize("k", [-300, 0, 300])
+def test_multipliers_of_a_scaled_column(k):
+    """One column of multipliers a / z in an identity: x_0 = q_0 / z and x_i = q_i - (a_i / z) q_0."""
+    s = problem(2)
+    n = 2 * s.N
+    rng = np.random.default_rng(7)
+    z = np.ldexp(1.0, k) * (1.3 - 1.1j)
+    A = np.eye(n, dtype=np.complex128)
+    A[:, 0] = z * rng.uniform(-0.6, 0.6, n)
+    A[1:, 0] += 1j * z * rng.uniform(-0.2, 0.2, n - 1)
+    A[0, 0] = z
+    q = s.srcvec(OM, RI[0], M.src_pw(0, 90, 0), want_host=True)[:, 0]
+    s.set_matrix(A, M.FP64)
+    x = s.solve(M.FP64)[:, 0]
+    wide = np.clongdouble
+    li, x0 = A[1:, 0].astype(wide) / wide(z), q[0].astype(wide) / wide(z)
+    # the quotient (3 u per part), two complex products (sqrt(5) u each) and the sum: below 16 u each
+    u = 2.0 ** -53
+    assert abs(x[0] - x0) <= 16 * u * abs(x0)
+    assert np.all(np.abs(x[1:] - (q[1:] - li * q[0])) <= 16 * u * (np.abs(li * q[0]) + np.abs(q[1:])))
+    s.close()
+
+
 def test_tallest_cluster_panels():
     s = problem(5)
     assert 2 * s.N == 24576
