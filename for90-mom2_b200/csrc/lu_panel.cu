@@ -663,6 +663,9 @@ __global__ void __launch_bounds__(kStThreads) swap_trsm_kernel(SwapTrsmArgs<E> a
     const int src = s_src[4 * i + g];
     if (on && (right || src != 4 * i + g)) x[i] = q[src];
   }
+  // The column's four lanes read rows that another of them stores below; the
+  // loop's own barrier is not reached when no row leaves (the last panel).
+  __syncwarp();
   // the rows that leave: all loads of a column before its stores
   for (int o0 = 0; o0 < nout; o0 += 64) {
     E v[16];

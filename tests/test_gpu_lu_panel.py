@@ -68,6 +68,26 @@ def test_multipliers_of_a_scaled_column(k):
     s.close()
 
 
+@pytest.mark.parametrize("prec", [M.FP64, M.MIXED])
+def test_interchanges_within_the_panel(prec):
+    """Unitary diagonal blocks in a matrix that is tiny elsewhere: every panel's pivots lie among its own 64 rows,
+    so no row leaves it (in a general matrix that is the last panel only), and every column left and right of it
+    is interchanged within those rows."""
+    s = problem(3)
+    n = 2 * s.N
+    rng = np.random.default_rng(11)
+    A = 1e-6 * (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)))
+    for k in range(0, n, 64):
+        g = rng.standard_normal((64, 64)) + 1j * rng.standard_normal((64, 64))
+        A[k:k + 64, k:k + 64] = np.linalg.qr(g)[0]
+    q = s.srcvec(OM, RI[0], M.src_pw(0, 90, 0), want_host=True)
+    s.set_matrix(A, prec)
+    x = s.solve(prec)
+    eta = np.linalg.norm(A @ x - q) / (np.linalg.norm(A) * np.linalg.norm(x))
+    assert eta <= (n * 2.0 ** -53 if prec == M.FP64 else 1e-12)
+    s.close()
+
+
 def test_tallest_cluster_panels():
     s = problem(5)
     assert 2 * s.N == 24576
