@@ -73,6 +73,9 @@ __device__ __forceinline__ void st_async16(unsigned addr, uint4 v, unsigned mbar
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same in two parts, with work between them.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ bool mbar_poll(unsigned bar, unsigned parity) {
   unsigned done;
   asm volatile(
@@ -172,7 +175,9 @@ struct __align__(16) PanelMsg {
 // of the next one, and the columns right of it, take the rank-W update of the
 // last one as they are loaded, so the cluster keeps its SMs for the whole panel
 // (beside a GEMM that would take them between launches).  What other CTAs of
-// the cluster wrote is read through L2 after a cluster barrier.
+// the cluster wrote is read through L2 after a cluster barrier: that at a
+// subpanel's end, and for the columns updated in place one whose two halves
+// stand on either side of the subpanel's pivot chain.
 template <typename E, int W, int R, int T>
 __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
   using Msg = PanelMsg<E, W>;
@@ -427,6 +432,9 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
             if (on) A[row + (j0 + j) * a.lda] = y[j];
         }
       }
+      // released here, acquired before step 4, which reads these columns' rows
+      // whichever CTA owns them (the messages order nothing but themselves)
+      cluster_arrive();
     }
     propose(0, []() {});
     columns(std::integral_constant<int, W>{}, first, 0, W / 2);
@@ -435,6 +443,7 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
     if (wid == 0 && lane < W) s_top[lane] = top;
     // (a CTA whose wait ran out stores nothing more)
     const int stop = __syncthreads_or(dead ? 1 : 0);
+    if (carry) cluster_wait();
     if (!stop) {
 #pragma unroll
       for (int r = 0; r < R; r++)

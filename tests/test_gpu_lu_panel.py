@@ -88,6 +88,29 @@ def test_interchanges_within_the_panel(prec):
     s.close()
 
 
+@pytest.mark.parametrize("prec", [M.FP64, M.MIXED])
+def test_one_launch_panels_equal_single_subpanels(prec, monkeypatch):
+    """A panel beside the update before it runs in one launch, whose subpanels exchange rows between CTAs; alone
+    it runs as one launch per subpanel.  Both are backward stable, so the solutions differ by at most twice the
+    bound of the backward error times the condition number."""
+    rng = np.random.default_rng(5)
+    xs = []
+    for ahead in ("1", "0"):
+        monkeypatch.setenv("MOM_LOOKAHEAD", ahead)
+        s = problem(3)
+        n = 2 * s.N
+        if not xs:
+            A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+        q = s.srcvec(OM, RI[0], M.src_pw(0, 90, 0), want_host=True)
+        s.set_matrix(A, prec)
+        xs.append(s.solve(prec))
+        bound = n * 2.0 ** -53 if prec == M.FP64 else 1e-12
+        assert np.linalg.norm(A @ xs[-1] - q) <= bound * np.linalg.norm(A) * np.linalg.norm(xs[-1])
+        s.close()
+    cond = np.linalg.norm(A) * np.linalg.norm(np.linalg.inv(A))
+    assert np.linalg.norm(xs[0] - xs[1]) <= 2 * bound * cond * np.linalg.norm(xs[1])
+
+
 def test_tallest_cluster_panels():
     s = problem(5)
     assert 2 * s.N == 24576
