@@ -41,6 +41,9 @@ namespace {
 
 constexpr int kRegMaxCluster = 16;
 constexpr int kPanelNb = 64;
+// Polls that a wait goes on for after it ran out: the messages under way, of
+// which there is one from every CTA, land in that time.
+constexpr long long kPanelDrainPolls = 1LL << 22;
 
 struct RegPanelArgs {
   void *A;
@@ -76,6 +79,18 @@ __device__ __forceinline__ void cluster_barrier() {
 // The same in two parts, with work between them.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// The same, suspended for a while.
 __device__ __forceinline__ bool mbar_poll(unsigned bar, unsigned parity) {
   unsigned done;
   asm volatile(
@@ -260,7 +275,7 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
 #pragma unroll
     for (int i = 0; i < kSend; i++) {
       const int q = tid + i * T;
-      if (q < CL * kMsgChunks)
+      if (q < CL * kMsgChunks && !dead)
         st_async16(to_msg[i] + par * (unsigned)sizeof(s_in[0]), src[q % kMsgChunks], to_bar[i] + 8u * par);
     }
   };
@@ -276,26 +291,28 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
       // 1. the CTAs' messages of column c: the largest key wins
       const int par = (ph + c) & 1;
       const unsigned bar = par ? bar1 : bar0, phase = (unsigned)((ph + c) >> 1) & 1u;
-      if (!dead) {
+      //    A wait of more than a.spin polls fails the factorisation, whichever
+      //    thread it is, and goes on: every CTA sends its message, so the
+      //    exchange stays in step and no phase is armed twice or left behind.
+      //    Past the second limit (a message is lost) the thread is dead: it
+      //    sends nothing more, which ends the other CTAs' waits in the same
+      //    way, and the phase, still armed, is not armed again.
+      if (!dead && !mbar_test(bar, phase)) {
         long long it = 0;
-        while (!mbar_poll(bar, phase)) {
-          if (++it >= a.spin) {
-            dead = true;
-            break;
-          }
-        }
+        do {
+          if (++it == a.spin) atomicExch(a.timeout, 1);
+          dead = it - a.spin >= kPanelDrainPolls;
+        } while (!dead && !mbar_poll(bar, phase));
       }
-      if (tid == 0) {
-        if (dead) atomicExch(a.timeout, 1);
+      if (tid == 0 && !dead)
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(tx) : "memory");
-      }
       const unsigned k = lane < CL ? s_in[par][lane].mag : 0u;
       const unsigned g = __reduce_max_sync(0xffffffffu, k);
       const Msg *in = &s_in[par][__ffs(__ballot_sync(0xffffffffu, k == g)) - 1];
       // no candidate at all (every entry NaN): no interchange, a failed pivot
       const bool none = g == 0u;
       int p = none ? c : (int)in->pos;
-      if (p < c || p >= m) p = c;  // only after a wait that ran out
+      if (p < c || p >= m) p = c;  // only in a dead thread
       E rp = {0, 0};
       if (!none) rp = in->rp;
       const bool live = rp.x != 0 || rp.y != 0;
@@ -441,10 +458,15 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
     columns(std::integral_constant<int, W / 2>{}, first, W / 2, W);
     ph += W;
     if (wid == 0 && lane < W) s_top[lane] = top;
-    // (a CTA whose wait ran out stores nothing more)
-    const int stop = __syncthreads_or(dead ? 1 : 0);
-    if (carry) cluster_wait();
-    if (!stop) {
+    // (a CTA with a dead thread stores nothing more, and its row moves are none)
+    dead = __syncthreads_or(dead ? 1 : 0) != 0;
+    if (s > a.s0) cluster_wait();
+    if (dead && a.map && cta == 0 && tid < 2 * W) {
+      int *map = a.map + blockIdx.y * a.batch_map + 2 * W * s + tid;
+      map[0] = -1;
+      map[128] = first;
+    }
+    if (!dead) {
 #pragma unroll
       for (int r = 0; r < R; r++)
 #pragma unroll
@@ -487,7 +509,8 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
       }
     }
     // every column of the cluster is in place; and no CTA leaves while messages
-    // to it can be under way (all have been waited for unless a wait ran out)
+    // to it can be under way: all have been waited for, or, where a thread is
+    // dead, every CTA has spent kPanelDrainPolls since the last was sent
     cluster_barrier();
   }
 }

@@ -111,6 +111,29 @@ def test_one_launch_panels_equal_single_subpanels(prec, monkeypatch):
     assert np.linalg.norm(xs[0] - xs[1]) <= 2 * bound * cond * np.linalg.norm(xs[1])
 
 
+@pytest.mark.parametrize("prec", [M.FP64, M.MIXED])
+def test_bounded_wait_of_the_cluster_panels(prec):
+    """A limit of one poll runs out in the first wait for another CTA's message: the factorisation reports it,
+    also in FP64, which has no residual check, and the same context solves again with the default limits."""
+    s = problem(3)
+    n = 2 * s.N
+    rng = np.random.default_rng(3)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    q = s.srcvec(OM, RI[0], M.src_pw(0, 90, 0), want_host=True)
+    for limit in (0, 1, 0):
+        s.set_wait_limits(limit, 0, 0)
+        s.set_matrix(A, prec)
+        if limit:
+            with pytest.raises(M.MomError) as e:
+                s.solve(prec)
+            assert e.value.status == M.MOM_ERR_TIMEOUT and "panel" in str(e.value)
+            continue
+        x = s.solve(prec)
+        eta = np.linalg.norm(A @ x - q) / (np.linalg.norm(A) * np.linalg.norm(x))
+        assert eta <= (n * 2.0 ** -53 if prec == M.FP64 else 1e-12)
+    s.close()
+
+
 def test_tallest_cluster_panels():
     s = problem(5)
     assert 2 * s.N == 24576
