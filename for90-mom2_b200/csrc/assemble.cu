@@ -1473,9 +1473,9 @@ int adjoint_eps(Ctx *c, double omega, const double *ri, int d, int R, const doub
   a.W = W;
   const int nobj = R == 0 ? 1 : R;
   if (c->adj_eps_plain) {
-    // one objective (or the dense W) per pair of launches
     AdjEpsArgs e;
     e.F = D.F;
+    e.no = nobj;
     e.n = c->n;
     e.N = c->N;
     e.qrel = D.qrel;
@@ -1498,34 +1498,38 @@ int adjoint_eps(Ctx *c, double omega, const double *ri, int d, int R, const doub
     e.dc2 = der(a.c2);
     e.Z = val(a.Zsi);
     e.dZ = der(a.Zsi);
+    e.lam = lam;
+    e.xv = xv;
     e.W = W;
-    const dim3 far((D.F + kEpsThreads - 1) / kEpsThreads, (D.F + kEpsTests - 1) / kEpsTests);
-    const unsigned near = (unsigned)((D.nnear + kEpsThreads - 1) / kEpsThreads);
+    // Test faces per CTA as in domain_blocks: few enough that the half of the
+    // CTAs that has work fills the resident slots (3 per SM) kEpsWaves times: a
+    // test face is 71 us.  80 faces, one source: 0.26 ms; with eight test
+    // faces per CTA and one lane per near pair 1.18 (a pass per objective).
+    const unsigned cols = (D.F + kEpsThreads - 1) / kEpsThreads;
+    e.tests = kEpsTests;
+    while (e.tests > 1 && (int64_t)cols * ((D.F + e.tests - 1) / e.tests) < 2 * kEpsWaves * 3 * c->nsm) e.tests /= 2;
+    const dim3 far(cols, (D.F + e.tests - 1) / e.tests);
+    const int lanes = D.nnear < 128 * (int64_t)c->nsm ? 4 : 1;  // as in domain_blocks
+    const unsigned near = (unsigned)((D.nnear * lanes + kEpsThreads - 1) / kEpsThreads);
     const size_t parts = (size_t)far.x * far.y + near;
     MOM_TRY(ensure_buffer(c, &c->adj_part, &c->adj_part_bytes, sizeof(double2) * parts * nobj));
-    for (int o = 0; o < nobj; o++) {
-      e.lam = R ? lam + (size_t)o * c->n : nullptr;
-      e.xv = R ? xv + (size_t)o * c->n : nullptr;
-      e.part = (double2 *)c->adj_part + parts * o;
-      switch (c->nq) {
-        case 1: launch_adj_eps<1>(far, near, c->stream, e); break;
-        case 3: launch_adj_eps<3>(far, near, c->stream, e); break;
-        case 4: launch_adj_eps<4>(far, near, c->stream, e); break;
-        case 7: launch_adj_eps<7>(far, near, c->stream, e); break;
-        case 13: launch_adj_eps<13>(far, near, c->stream, e); break;
-        default: return fail(c, MOM_ERR_ARG, "unsupported number of quadrature points");
-      }
-      c->launches += near ? 2 : 1;
-      MOM_CUDA(c, cudaGetLastError());
+    e.part = (double2 *)c->adj_part;
+    switch (c->nq) {
+      case 1: launch_adj_eps<1>(far, near, lanes, c->stream, e); break;
+      case 3: launch_adj_eps<3>(far, near, lanes, c->stream, e); break;
+      case 4: launch_adj_eps<4>(far, near, lanes, c->stream, e); break;
+      case 7: launch_adj_eps<7>(far, near, lanes, c->stream, e); break;
+      case 13: launch_adj_eps<13>(far, near, lanes, c->stream, e); break;
+      default: return fail(c, MOM_ERR_ARG, "unsupported number of quadrature points");
     }
+    c->launches += near ? 2 : 1;
+    MOM_CUDA(c, cudaGetLastError());
     std::vector<double> h(2 * parts * nobj);
     MOM_CUDA(c, cudaMemcpyAsync(h.data(), c->adj_part, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream));
     MOM_CUDA(c, cudaStreamSynchronize(c->stream));
-    for (int o = 0; o < nobj; o++) {
-      out[2 * o] = out[2 * o + 1] = 0;
-      for (size_t b = 0; b < parts; b++)
-        for (int i = 0; i < 2; i++) out[2 * o + i] += h[2 * (parts * o + b) + i];
-    }
+    for (int i = 0; i < 2 * nobj; i++) out[i] = 0;
+    for (size_t b = 0; b < parts; b++)
+      for (int i = 0; i < 2 * nobj; i++) out[i] += h[2 * nobj * b + i];
     return MOM_OK;
   }
   const dim3 grid((D.F + kAdjThreads - 1) / kAdjThreads, D.F);
