@@ -36,14 +36,15 @@ constexpr int kRevTile = 8;     // faces staged at a time
 constexpr int kRevVals = 43;    // per point and objective: R_i (3), then 20 complex sums
 
 struct RevArgs {
-  int F, no;               // faces, objectives of this launch (1 or 2, the same x)
-  const double *qrel, *qabs, *cp;
-  const double2 *coef;     // [no + 1][F][8]: lambda of each objective, then x: aJ, bJ[3], aM, bM[3]
+  int F, no;               // faces, objectives of a set (1 or 2, the same x); sets: blockIdx.z
+  const double *qrel, *cp;
+  const double2 *coef;     // [set][no + 1][F][8]: lambda of each objective, then x: aJ, bJ[3], aM, bM[3]
   const unsigned *near_bits;
   double kr, ki;
   Cd c1, c2, Z;
   int per_split;           // faces per split (blockIdx.y)
-  double *part;            // [split][no][F NQ][kRevVals]
+  double *part;            // [set][split][no][F NQ][kRevVals], the sets set_part doubles apart
+  size_t set_part;
 };
 
 __device__ __forceinline__ Cd cvdot(const Cv &a, const Cv &b, Cd acc) {
@@ -77,6 +78,8 @@ __global__ void __launch_bounds__(kRevThreads) rev_field_kernel(RevArgs a) {
   double *s_face = s_acc + (16 * (NO + 1) + 3 * NO) * kT;   // [kRevTile][kFace]: coefs, cp, qrel
   const int tid = threadIdx.x;
   const int P = a.F * NQ, i = blockIdx.x * kT + tid;
+  a.coef += (size_t)blockIdx.z * (NO + 1) * a.F * 8;
+  a.part += blockIdx.z * a.set_part;
   const bool valid = i < P;
   const int m = valid ? i / NQ : 0, t = valid ? i % NQ : 0;
   const double w = c_qw[t];
@@ -280,13 +283,14 @@ struct RevStaticArgs {
   int64_t nnear;
   const int *near_m, *near_n;
   const double *qrel, *qabs, *cp, *area;
-  const double *mu;
   const FaceGeo *geo;
   const double2 *coef;  // as RevArgs
-  const double2 *xv;    // x on the unknowns
+  const double2 *xv;    // x on the unknowns, the sets set_x apart
+  size_t set_x;
   Cd k2, c1, c2, Z;
-  double *part;         // the fields' slot: [no][F NQ][kRevVals]
-  double *pair;         // [nnear][9][no][4]: d/d(source coordinate); minus its share of the test vertices
+  double *part;         // the fields' slot: [no][F NQ][kRevVals], the sets set_part apart
+  size_t set_part;
+  double *pair;         // [set][nnear][9][no][4]: d/d(source coordinate); minus its share of the test vertices
 };
 
 // First entry of row m of the near list (sorted by test face).
@@ -300,13 +304,19 @@ __device__ __forceinline__ int64_t near_row(const int *near_m, int64_t nnear, in
   return lo;
 }
 
-// Fields of the near faces' closed-form terms at every point, added up in
-// list order and written as one more split of rev_field_kernel's output (no
-// dF/dX and no force: those are rev_static_kernel's).
+// Fields of the near faces' closed-form terms at every point, written as one
+// more split of rev_field_kernel's output (no dF/dX and no force: those are
+// rev_static_kernel's).  kStaticLanes threads per point with every
+// kStaticLanes-th near face each, added up in a fixed order.  Bound by the
+// latency of point_static: one thread per point took 388 us over 80 faces.
+constexpr int kStaticLanes = 8;
 template <int NQ>
 __global__ void __launch_bounds__(64) rev_static_field_kernel(RevStaticArgs a) {
-  const int P = a.F * NQ, i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P) return;
+  const int P = a.F * NQ, at = blockIdx.x * blockDim.x + threadIdx.x, lane = at % kStaticLanes;
+  const bool live = at / kStaticLanes < P;
+  const int i = live ? at / kStaticLanes : 0;
+  a.coef += (size_t)blockIdx.y * (a.no + 1) * a.F * 8;
+  a.part += blockIdx.y * a.set_part;
   const int m = i / NQ, t = i % NQ;
   const double w = c_qw[t];
   const double *r = a.qabs + (size_t)i * 3;
@@ -315,7 +325,7 @@ __global__ void __launch_bounds__(64) rev_static_field_kernel(RevStaticArgs a) {
   Cd F[2][4];  // J, M: field (3), divergence
   for (int h = 0; h < 2; h++)
     for (int k = 0; k < 4; k++) F[h][k] = {0, 0};
-  for (int64_t j = near_row(a.near_m, a.nnear, m); j < a.nnear && a.near_m[j] == m; j++) {
+  for (int64_t j = near_row(a.near_m, a.nnear, m) + lane; j < a.nnear && a.near_m[j] == m; j += kStaticLanes) {
     const int n = a.near_n[j];
     PointStatic<double> ps;
     point_static(r, a.geo[n], ps);
@@ -348,6 +358,16 @@ __global__ void __launch_bounds__(64) rev_static_field_kernel(RevStaticArgs a) {
         F[1][k] = cadd(F[1][k], csc((&K[0].x)[k], iA));
       }
   }
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int s = 1; s < kStaticLanes; s *= 2) {
+        F[h][k].re += __shfl_xor_sync(0xffffffffu, F[h][k].re, s);
+        F[h][k].im += __shfl_xor_sync(0xffffffffu, F[h][k].im, s);
+      }
+  if (!live || lane != 0) return;
   const double *qr = a.qrel + (size_t)i * 3;
   for (int o = 0; o < a.no; o++) {
     double *out = a.part + ((size_t)o * P + i) * kRevVals;
@@ -374,6 +394,9 @@ template <int NQ>
 __global__ void __launch_bounds__(64) rev_static_kernel(RevStaticArgs a) {
   const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (item >= a.nnear * 9) return;
+  a.coef += (size_t)blockIdx.y * (a.no + 1) * a.F * 8;
+  a.xv += blockIdx.y * a.set_x;
+  a.pair += (size_t)blockIdx.y * a.nnear * 36 * a.no;
   const int64_t j = item / 9;
   const int seed = (int)(item % 9);
   const int m = a.near_m[j], n = a.near_n[j];
@@ -476,27 +499,70 @@ struct RevChainArgs {
   int64_t nnear;
   const int *near_m, *near_n;
   const double *mu, *sl;
-  const double2 *lam, *xv;  // the launch's objectives: [no][n], x
+  const double2 *lam, *xv;  // the launch's objectives: [set][no][n], x (set_x apart)
   int64_t n;
+  size_t set_x, set_part;
   const double *part, *pair;
-  double *out;              // [no][F][9]
+  double *out;              // [set][no][F][9]
 };
 
-// One warp per (face, objective): the chain rule to the face's nine
-// coordinates, every sum in a fixed order.
+// One CTA per (face, objective of a set, set): the chain rule to the face's nine
+// coordinates, every sum in a fixed order.  Bound by latency: the sums over
+// splits and points and those over near faces are spread over the threads (one
+// warp, and nine of its lanes for the near faces, took 280 us over 80 faces).
+constexpr int kChainThreads = 128;
 template <int NQ>
-__global__ void __launch_bounds__(32) rev_chain_kernel(RevChainArgs a) {
-  const int f = blockIdx.x, o = blockIdx.y, lane = threadIdx.x;
+__global__ void __launch_bounds__(kChainThreads) rev_chain_kernel(RevChainArgs a) {
+  constexpr int kWarps = kChainThreads / 32;
+  const int f = blockIdx.x, o = blockIdx.y, lane = threadIdx.x % 32, wid = threadIdx.x / 32;
   const int P = a.F * NQ;
-  __shared__ double s_sum[9 + 40], s_v[9], s_u[3][3], s_l[3];
+  a.lam += (size_t)blockIdx.z * a.no * a.n;
+  a.xv += blockIdx.z * a.set_x;
+  a.part += blockIdx.z * a.set_part;
+  a.pair += (size_t)blockIdx.z * a.nnear * 36 * a.no;
+  a.out += (size_t)blockIdx.z * a.no * a.F * 9;
+  __shared__ double s_sum[9 + 40], s_w[kWarps][9 + 40], s_n[kWarps][9], s_v[9], s_u[3][3], s_l[3];
   for (int e = lane; e < 49; e += 32) {
     double acc = 0;
-    for (int s = 0; s < a.splits; s++)
-      for (int t = 0; t < NQ; t++) {
-        const double *p = a.part + (((size_t)s * a.no + o) * P + (size_t)f * NQ + t) * kRevVals;
-        if (e < 9) acc += c_qn[t][e / 3 == 0 ? 2 : e / 3 - 1] * p[e % 3];
-        else acc += p[3 + e - 9];
+#pragma unroll 4
+    for (int b = wid; b < a.splits * NQ; b += kWarps) {
+      const int s = b / NQ, t = b % NQ;
+      const double *p = a.part + (((size_t)s * a.no + o) * P + (size_t)f * NQ + t) * kRevVals;
+      acc += e < 9 ? c_qn[t][e / 3 == 0 ? 2 : e / 3 - 1] * p[e % 3] : p[3 + e - 9];
+    }
+    s_w[wid][e] = acc;
+  }
+  // closed-form terms: as the source face, and as the test face
+  {
+    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    const int64_t r0 = near_row(a.near_m, a.nnear, f);
+    for (int64_t j = r0 + threadIdx.x; j < a.nnear && a.near_m[j] == f; j += kChainThreads) {
+      const int mp = a.near_n[j];  // the pair (mp, f): the near relation is symmetric
+      int64_t lo = near_row(a.near_m, a.nnear, mp), hi = near_row(a.near_m, a.nnear, mp + 1);
+      while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (a.near_n[mid] < f) lo = mid + 1;
+        else hi = mid;
       }
+#pragma unroll
+      for (int c = 0; c < 9; c++) {
+        for (int u = 0; u < 3; u++) v[c] += a.pair[((size_t)(j * 9 + 3 * u + c % 3) * a.no + o) * 4 + 1 + c / 3];
+        v[c] += a.pair[((size_t)(lo * 9 + c) * a.no + o) * 4];
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 9; c++)
+#pragma unroll
+      for (int s = 1; s < 32; s *= 2) v[c] += __shfl_xor_sync(0xffffffffu, v[c], s);
+    if (lane == 0)
+#pragma unroll
+      for (int c = 0; c < 9; c++) s_n[wid][c] = v[c];
+  }
+  __syncthreads();
+  if (wid > 0) return;
+  for (int e = lane; e < 49; e += 32) {
+    double acc = 0;
+    for (int k = 0; k < kWarps; k++) acc += s_w[k][e];
     s_sum[e] = acc;
   }
   __syncwarp();
@@ -522,22 +588,9 @@ __global__ void __launch_bounds__(32) rev_chain_kernel(RevChainArgs a) {
     for (int k = 0; k < 3; k++) s_u[p][k] = gu[k];
     s_l[p] = gl;
   }
-  // closed-form terms: as the source face, and as the test face
   if (lane < 9) {
     double acc = s_sum[lane];
-    const int64_t r0 = near_row(a.near_m, a.nnear, f);
-    for (int64_t j = r0; j < a.nnear && a.near_m[j] == f; j++) {
-      for (int v = 0; v < 3; v++)
-        acc += a.pair[((size_t)(j * 9 + 3 * v + lane % 3) * a.no + o) * 4 + 1 + lane / 3];
-      const int mp = a.near_n[j];  // the pair (mp, f): the near relation is symmetric
-      int64_t lo = near_row(a.near_m, a.nnear, mp), hi = near_row(a.near_m, a.nnear, mp + 1);
-      while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (a.near_n[mid] < f) lo = mid + 1;
-        else hi = mid;
-      }
-      acc += a.pair[((size_t)(lo * 9 + lane) * a.no + o) * 4];
-    }
+    for (int k = 0; k < kWarps; k++) acc += s_n[k][lane];
     s_v[lane] = acc;
   }
   __syncwarp();
@@ -558,9 +611,9 @@ __global__ void __launch_bounds__(32) rev_chain_kernel(RevChainArgs a) {
 }
 
 template <int NQ>
-int rev_launch(Ctx *c, RevArgs ra, const RevStaticArgs &sa, const RevChainArgs &ca, int splits) {
+int rev_launch(Ctx *c, const RevArgs &ra, const RevStaticArgs &sa, const RevChainArgs &ca, int splits, int sets) {
   const int P = ra.F * NQ;
-  const dim3 grid((P + kRevThreads - 1) / kRevThreads, splits);
+  const dim3 grid((P + kRevThreads - 1) / kRevThreads, splits, sets);
   const size_t smem = rev_smem<NQ>(ra.no);
   if (ra.no == 2) {
     MOM_CUDA(c, cudaFuncSetAttribute(rev_field_kernel<NQ, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -569,41 +622,54 @@ int rev_launch(Ctx *c, RevArgs ra, const RevStaticArgs &sa, const RevChainArgs &
     MOM_CUDA(c, cudaFuncSetAttribute(rev_field_kernel<NQ, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     rev_field_kernel<NQ, 1><<<grid, kRevThreads, smem, c->stream>>>(ra);
   }
-  rev_static_field_kernel<NQ><<<(P + 63) / 64, 64, 0, c->stream>>>(sa);
-  if (sa.nnear > 0) rev_static_kernel<NQ><<<(unsigned)((sa.nnear * 9 + 63) / 64), 64, 0, c->stream>>>(sa);
-  rev_chain_kernel<NQ><<<dim3(ca.F, ca.no), 32, 0, c->stream>>>(ca);
+  rev_static_field_kernel<NQ><<<dim3((P * kStaticLanes + 63) / 64, sets), 64, 0, c->stream>>>(sa);
+  if (sa.nnear > 0) rev_static_kernel<NQ><<<dim3((unsigned)((sa.nnear * 9 + 63) / 64), sets), 64, 0, c->stream>>>(sa);
+  rev_chain_kernel<NQ><<<dim3(ca.F, ca.no, sets), kChainThreads, 0, c->stream>>>(ca);
   c->launches += sa.nnear > 0 ? 4 : 3;
   MOM_CUDA(c, cudaGetLastError());
   return MOM_OK;
 }
 
+// Sets of objectives that rev_nodes takes at once: as many as leave one split
+// of the faces each in a few waves of CTAs.
+int rev_sets(const Ctx *c, const DomDev &D) {
+  return std::max(1, 8 * c->nsm / ((D.F * c->nq + kRevThreads - 1) / kRevThreads));
+}
+
 // d Re(lambda_o^T A_d x_o) / d(coordinates of domain d's face vertices) for
-// objectives o0 .. o0 + no - 1 (the same x): out[no][F][9].
-int rev_nodes(Ctx *c, int d, const AdjPairArgs &m, int o0, int no, std::vector<double> &out) {
+// objectives o0 .. o0 + sets no - 1, no of the same x after another:
+// out[sets][no][F][9].
+int rev_nodes(Ctx *c, int d, const AdjPairArgs &m, int o0, int no, int sets, std::vector<double> &out) {
   DomDev &D = c->dom[d];
   MOM_TRY(nfield_geometry(c, D));
   const int F = D.F, P = F * c->nq;
-  // a few waves of two CTAs per SM
+  // a few waves of two CTAs per SM, two faces at least per CTA (the sums over a
+  // split's faces are a serial chain, 9 us per face with 13 points)
   const int blocks = (P + kRevThreads - 1) / kRevThreads;
-  const int want = std::max(1, std::min(F / kRevTile, 8 * c->nsm / blocks));
-  const int per = ((F + want - 1) / want + kRevTile - 1) / kRevTile * kRevTile, splits = (F + per - 1) / per;
-  const size_t b_coef = sizeof(double2) * 8 * (size_t)F * (no + 1);
-  const size_t slot = sizeof(double) * kRevVals * (size_t)P * no;
-  const size_t b_part = slot * (splits + 1), b_pair = sizeof(double) * 36 * (size_t)no * std::max<int64_t>(1, D.nnear);
-  const size_t b_out = sizeof(double) * 9 * (size_t)F * no;
+  const int want = std::max(1, std::min(F / 2, 8 * c->nsm / (blocks * sets)));
+  const int per = (F + want - 1) / want, splits = (F + per - 1) / per;
+  const size_t b_coef = sizeof(double2) * 8 * (size_t)F * (no + 1) * sets;
+  const size_t slot = sizeof(double) * kRevVals * (size_t)P * no, set_part = slot / sizeof(double) * (splits + 1);
+  const size_t b_part = sizeof(double) * set_part * sets;
+  const size_t b_pair = sizeof(double) * 36 * (size_t)no * std::max<int64_t>(1, D.nnear) * sets;
+  const size_t b_out = sizeof(double) * 9 * (size_t)F * no * sets;
   MOM_TRY(ensure_buffer(c, &c->adj_part, &c->adj_part_bytes, b_coef + b_part + b_pair + b_out));
   char *b = (char *)c->adj_part;
   double2 *coef = (double2 *)b;
   const double2 *lam = m.lam + (size_t)o0 * m.n, *xv = m.xv + (size_t)o0 * m.n;
+  const size_t set_x = (size_t)no * m.n;
   const dim3 cg((F + 127) / 128, no);
-  face_current_kernel<<<cg, 128, 0, c->stream>>>(F, c->N, D.hpar, D.sl, D.mu, lam, m.n, coef);
-  face_current_kernel<<<cg.x, 128, 0, c->stream>>>(F, c->N, D.hpar, D.sl, D.mu, xv, m.n, coef + 8 * (size_t)F * no);
-  c->launches += 2;
+  for (int s = 0; s < sets; s++) {
+    double2 *cs = coef + 8 * (size_t)F * (no + 1) * s;
+    face_current_kernel<<<cg, 128, 0, c->stream>>>(F, c->N, D.hpar, D.sl, D.mu, lam + s * set_x, m.n, cs);
+    face_current_kernel<<<cg.x, 128, 0, c->stream>>>(F, c->N, D.hpar, D.sl, D.mu, xv + s * set_x, m.n,
+                                                     cs + 8 * (size_t)F * no);
+    c->launches += 2;
+  }
   RevArgs ra;
   ra.F = F;
   ra.no = no;
   ra.qrel = D.qrel;
-  ra.qabs = D.qabs;
   ra.cp = D.cp;
   ra.coef = coef;
   ra.near_bits = D.near_bits;
@@ -614,6 +680,7 @@ int rev_nodes(Ctx *c, int d, const AdjPairArgs &m, int o0, int no, std::vector<d
   ra.Z = {m.Zsi.re.v, m.Zsi.im.v};
   ra.per_split = per;
   ra.part = (double *)(b + b_coef);
+  ra.set_part = set_part;
   RevStaticArgs sa;
   sa.t = m.t;
   sa.F = F;
@@ -625,15 +692,16 @@ int rev_nodes(Ctx *c, int d, const AdjPairArgs &m, int o0, int no, std::vector<d
   sa.qabs = D.qabs;
   sa.cp = D.cp;
   sa.area = D.area;
-  sa.mu = D.mu;
   sa.geo = reinterpret_cast<const FaceGeo *>(D.nf_geo);
   sa.coef = coef;
   sa.xv = xv;
+  sa.set_x = set_x;
   sa.k2 = {ra.kr * ra.kr - ra.ki * ra.ki, 2 * ra.kr * ra.ki};
   sa.c1 = ra.c1;
   sa.c2 = ra.c2;
   sa.Z = ra.Z;
   sa.part = (double *)(b + b_coef + slot * splits);
+  sa.set_part = set_part;
   sa.pair = (double *)(b + b_coef + b_part);
   RevChainArgs ca;
   ca.t = m.t;
@@ -648,18 +716,20 @@ int rev_nodes(Ctx *c, int d, const AdjPairArgs &m, int o0, int no, std::vector<d
   ca.lam = lam;
   ca.xv = xv;
   ca.n = m.n;
+  ca.set_x = set_x;
+  ca.set_part = set_part;
   ca.part = ra.part;
   ca.pair = sa.pair;
   ca.out = (double *)(b + b_coef + b_part + b_pair);
   switch (c->nq) {
-    case 1: MOM_TRY(rev_launch<1>(c, ra, sa, ca, splits)); break;
-    case 3: MOM_TRY(rev_launch<3>(c, ra, sa, ca, splits)); break;
-    case 4: MOM_TRY(rev_launch<4>(c, ra, sa, ca, splits)); break;
-    case 7: MOM_TRY(rev_launch<7>(c, ra, sa, ca, splits)); break;
-    case 13: MOM_TRY(rev_launch<13>(c, ra, sa, ca, splits)); break;
+    case 1: MOM_TRY(rev_launch<1>(c, ra, sa, ca, splits, sets)); break;
+    case 3: MOM_TRY(rev_launch<3>(c, ra, sa, ca, splits, sets)); break;
+    case 4: MOM_TRY(rev_launch<4>(c, ra, sa, ca, splits, sets)); break;
+    case 7: MOM_TRY(rev_launch<7>(c, ra, sa, ca, splits, sets)); break;
+    case 13: MOM_TRY(rev_launch<13>(c, ra, sa, ca, splits, sets)); break;
     default: return fail(c, MOM_ERR_ARG, "unsupported number of quadrature points");
   }
-  out.resize(9 * (size_t)F * no);
+  out.resize(9 * (size_t)F * no * sets);
   MOM_CUDA(c, cudaMemcpyAsync(out.data(), ca.out, b_out, cudaMemcpyDeviceToHost, c->stream));
   MOM_CUDA(c, cudaStreamSynchronize(c->stream));
   return MOM_OK;

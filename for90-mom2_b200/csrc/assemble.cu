@@ -1579,12 +1579,16 @@ int adjoint_nodes(Ctx *c, double omega, const double *ri, int R, const double2 *
     a.xv = xv;
     a.W = nullptr;
     if (c->adj_vertex_reverse) {
-      // objectives of one source share x: two at a time
-      for (int o = 0, no = 0; o < R; o += no) {
-        no = o + 1 < R && obj_src[o] == obj_src[o + 1] ? 2 : 1;
+      // objectives of one source share x: two make a set, and as many sets at a
+      // time as the domain's size leaves room for
+      const int most = rev_sets(c, D);
+      auto pair_at = [&](int o) { return o + 1 < R && obj_src[o] == obj_src[o + 1]; };
+      for (int o = 0, no = 0, sets = 0; o < R; o += no * sets) {
+        no = pair_at(o) ? 2 : 1;
+        for (sets = 1; sets < most && o + no * sets < R && pair_at(o + no * sets) == (no == 2); sets++) {}
         std::vector<double> h;
-        MOM_TRY(rev_nodes(c, d, a, o, no, h));
-        for (int k = 0; k < no; k++)
+        MOM_TRY(rev_nodes(c, d, a, o, no, sets, h));
+        for (int k = 0; k < no * sets; k++)
           for (int e = 0; e < 9 * D.F; e++)
             out[((size_t)(o + k) * total + off[d] + D.h_fnode[e / 3]) * 3 + e % 3] -= h[(size_t)k * 9 * D.F + e];
       }

@@ -54,3 +54,22 @@ def launches(ns, **kw):
 
 def test_eps_gradient_launches():
     assert launches(4, eps_dom=1) == launches(1, eps_dom=1)
+
+
+@pytest.mark.parametrize("subdiv,quad,ns", [(0, "tri_gl1", 1), (0, "tri_gl13", 4), (1, "tri_gl3", 3), (2, "tri_gl4", 2),
+                                            (1, "tri_gl7", 4), (2, "tri_gl13", 3)])
+def test_vertex_gradient_of_several_sources(subdiv, quad, ns, monkeypatch):
+    out = []
+    for plain in ("1", "0"):
+        monkeypatch.setenv("MOM_ADJ_VERTEX_PLAIN", plain)
+        s = solved(subdiv, quad, ns)
+        out.append(s.adjoint(OM, RI, SRCS[:ns], M.FP64, nodes=True)["dnodes"])
+        s.close()
+    for a, b in zip(*out):
+        for k in range(ns):
+            assert close(a[k], b[k])
+
+
+def test_vertex_gradient_launches():
+    """Three more sources cost two small launches per source and domain, which prepare their currents."""
+    assert launches(4, nodes=True) - launches(1, nodes=True) <= 3 * 2 * 2
