@@ -68,31 +68,38 @@ __device__ __forceinline__ Cd ld_c(const double2 *p) {
 }
 __device__ __forceinline__ Cv ld_v(const double2 *p) { return {ld_c(p), ld_c(p + 1), ld_c(p + 2)}; }
 
-// The affine currents of a face about its centroid: a = sum_p v_p sl_p / 2,
-// b = -sum_p v_p sl_p mu_p / 2, for the J and M halves of vector v + s ldv,
-// s = blockIdx.y: coef[s][F][8] = aJ, bJ[3], aM, bM[3].
+// The affine current of face f about its centroid, of the J (h = 0) or M half of
+// vector v: a = sum_p v_p sl_p / 2, b = -sum_p v_p sl_p mu_p / 2 into o[4] = a, b.
+__device__ __forceinline__ void face_current(int f, int h, int N, const int *hpar, const double *sl, const double *mu,
+                                             const double2 *v, double2 *o) {
+  Cd a = {0, 0}, b[3] = {{0, 0}, {0, 0}, {0, 0}};
+#pragma unroll
+  for (int p = 0; p < 3; p++) {
+    const double2 c = v[hpar[3 * f + p] + (h ? N : 0)];
+    const double s = 0.5 * sl[3 * f + p];
+    a.re += s * c.x;
+    a.im += s * c.y;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const double t = s * mu[9 * (size_t)f + 3 * p + i];
+      b[i].re -= t * c.x;
+      b[i].im -= t * c.y;
+    }
+  }
+  o[0] = make_double2(a.re, a.im);
+#pragma unroll
+  for (int i = 0; i < 3; i++) o[1 + i] = make_double2(b[i].re, b[i].im);
+}
+
+// Those of every face and of the vectors v + s ldv, s = blockIdx.y:
+// coef[s][F][8] = aJ, bJ[3], aM, bM[3].
 __global__ void face_current_kernel(int F, int N, const int *hpar, const double *sl, const double *mu,
                                     const double2 *v, int64_t ldv, double2 *coef) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= F) return;
   v += (size_t)blockIdx.y * ldv;
-  for (int h = 0; h < 2; h++) {
-    Cd a = {0, 0}, b[3] = {{0, 0}, {0, 0}, {0, 0}};
-    for (int p = 0; p < 3; p++) {
-      const double2 c = v[hpar[3 * f + p] + (h ? N : 0)];
-      const double s = 0.5 * sl[3 * f + p];
-      a.re += s * c.x;
-      a.im += s * c.y;
-      for (int i = 0; i < 3; i++) {
-        const double t = s * mu[9 * (size_t)f + 3 * p + i];
-        b[i].re -= t * c.x;
-        b[i].im -= t * c.y;
-      }
-    }
-    double2 *o = coef + 8 * ((size_t)blockIdx.y * F + f) + 4 * h;
-    o[0] = make_double2(a.re, a.im);
-    for (int i = 0; i < 3; i++) o[1 + i] = make_double2(b[i].re, b[i].im);
-  }
+  for (int h = 0; h < 2; h++)
+    face_current(f, h, N, hpar, sl, mu, v, coef + 8 * ((size_t)blockIdx.y * F + f) + 4 * h);
 }
 
 constexpr int kNfThreads = 128;
@@ -104,7 +111,11 @@ struct NfArgs {
   const double *cp;      // [F][3]
   const double *area;    // [F]
   const FaceGeo *geo;    // [F]
-  const double2 *coef;   // [sources][F][8] (the launch's first source)
+  int N;
+  const int *hpar;
+  const double *sl, *mu;
+  const double2 *x;      // the launch's solutions, ldx apart
+  int64_t ldx;
   double thr2;           // (3 avelen)^2
   double kr, ki;         // k = ri w / c0
   Cd k2;                 // k^2
@@ -115,10 +126,10 @@ struct NfArgs {
   double2 *part;         // [split][nsrc][npts][6]: E, H
 };
 
-// The closed-form parts of face n at r for one source's currents, added to
-// E, H (times 4 pi: the caller scales the sums).
-__device__ __noinline__ void nfield_static(const NfArgs &a, const double *r, const double *D0, int n, int ns, Cv *E,
-                                           Cv *H) {
+// The closed-form parts of face n at r for the currents cur of ns sources,
+// added to E, H (times 4 pi: the caller scales the sums).
+__device__ __noinline__ void nfield_static(const NfArgs &a, const double *r, const double *D0, int n,
+                                           const double2 *cur, int ns, Cv *E, Cv *H) {
   PointStatic<double> ps;
   point_static(r, a.geo[n], ps);
   const double iA = 1.0 / a.area[n];
@@ -136,7 +147,7 @@ __device__ __noinline__ void nfield_static(const NfArgs &a, const double *r, con
   const Cv P = {gr[0], gr[1], gr[2]}, Lv = {l[0], l[1], l[2]};
 #pragma unroll 1
   for (int s = 0; s < ns; s++) {
-    const double2 *c = a.coef + ((size_t)s * a.F + n) * 8;
+    const double2 *c = cur + 8 * s;
     const Cd aJ = ld_c(c), aM = ld_c(c + 4), z = {iA, 0};
     const Cv bJ = ld_v(c + 1), bM = ld_v(c + 5);
     // int (a r' + b) / A over R and R: a (mL + rho S) + b S
@@ -171,14 +182,16 @@ __global__ void __launch_bounds__(kNfThreads) nfield_kernel(NfArgs a) {
   for (int base = n0; base < n1; base += kNfTile) {
     const int cnt = min(kNfTile, n1 - base);
     __syncthreads();
-    for (int e = threadIdx.x; e < cnt * (kCoef + 3 + 3 * NQ); e += kNfThreads) {
-      const int f = e / (kCoef + 3 + 3 * NQ), k = e % (kCoef + 3 + 3 * NQ), n = base + f;
-      double v;
-      if (k < kCoef)
-        v = k / 16 < a.nsrc ? reinterpret_cast<const double *>(a.coef + ((size_t)(k / 16) * a.F + n) * 8)[k % 16] : 0.0;
-      else if (k < kCoef + 3) v = a.cp[3 * n + k - kCoef];
-      else v = a.qrel[(size_t)n * NQ * 3 + k - kCoef - 3];
-      s_face[f][k] = v;
+    for (int e = threadIdx.x; e < cnt * 2 * NS; e += kNfThreads) {
+      const int f = e / (2 * NS), s = e / 2 % NS, h = e % 2;
+      double2 *o = reinterpret_cast<double2 *>(s_face[f]) + 8 * s + 4 * h;
+      if (s < a.nsrc) face_current(base + f, h, a.N, a.hpar, a.sl, a.mu, a.x + s * a.ldx, o);
+      else
+        for (int i = 0; i < 4; i++) o[i] = make_double2(0, 0);
+    }
+    for (int e = threadIdx.x; e < cnt * (3 + 3 * NQ); e += kNfThreads) {
+      const int f = e / (3 + 3 * NQ), k = e % (3 + 3 * NQ), n = base + f;
+      s_face[f][kCoef + k] = k < 3 ? a.cp[3 * n + k] : a.qrel[(size_t)n * NQ * 3 + k - 3];
     }
     __syncthreads();
     if (!valid) continue;
@@ -233,7 +246,7 @@ __global__ void __launch_bounds__(kNfThreads) nfield_kernel(NfArgs a) {
         E[s] = cvadd(E[s], cvadd(cvadd(cvscale(a.c1, uj), cvscale(csc(cmul(a.c2, aJ), 2.0), P1)), km));
         H[s] = cvadd(H[s], cvsub(cvadd(cvscale(a.ic2, um), cvscale(csc(cmul(a.ic1, aM), 2.0), P1)), kj));
       }
-      if (near) nfield_static(a, r, D0, base + f, min(NS, a.nsrc), E, H);
+      if (near) nfield_static(a, r, D0, base + f, reinterpret_cast<const double2 *>(fc), min(NS, a.nsrc), E, H);
     }
   }
   if (!valid) return;
@@ -247,17 +260,25 @@ __global__ void __launch_bounds__(kNfThreads) nfield_kernel(NfArgs a) {
   }
 }
 
-// E, H [nsrc][npts][3]: the splits' parts in split order.
+// E, H [nsrc][npts][3]: the splits' parts, LANES threads per value with every
+// LANES-th split each, added up in a fixed order.
+template <int LANES>
 __global__ void nfield_sum_kernel(int npts, int nsrc, int splits, const double2 *part, double2 *E, double2 *H) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, e = idx / LANES;
+  const int lane = (int)(idx % LANES);
   const int64_t per = (int64_t)nsrc * npts * 6;
-  if (e >= per) return;
   double2 v = make_double2(0, 0);
-  for (int s = 0; s < splits; s++) {
+  for (int s = lane; s < splits && e < per; s += LANES) {
     const double2 p = part[s * per + e];
     v.x += p.x;
     v.y += p.y;
   }
+#pragma unroll
+  for (int w = 1; w < LANES; w *= 2) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, w);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, w);
+  }
+  if (e >= per || lane != 0) return;
   const int64_t at = e / 6;
   const int i = (int)(e % 6);
   (i < 3 ? E : H)[at * 3 + i % 3] = v;
@@ -312,16 +333,13 @@ int scat_fields(Ctx *c, int d, double omega, const double *ri, int nsrc, const d
   DomDev &D = c->dom[d];
   MOM_TRY(nfield_geometry(c, D));
   const int F = D.F;
-  // faces per split: eight CTAs per SM in all, at least one tile of faces each
+  // Faces per split: eight CTAs per SM in all, down to one face each, since a
+  // split's faces are a serial chain (8 us per near face with 13 points).
   const int blocks = (npts + kNfThreads - 1) / kNfThreads;
-  const int want = std::max(1, std::min((F + kNfTile - 1) / kNfTile, 8 * c->nsm / blocks));
-  const int per = ((F + want - 1) / want + kNfTile - 1) / kNfTile * kNfTile, splits = (F + per - 1) / per;
-  const size_t b_coef = sizeof(double2) * 8 * (size_t)F * nsrc;
-  const size_t b_part = sizeof(double2) * 6 * (size_t)npts * std::min(nsrc, 4) * splits;
-  MOM_TRY(ensure_buffer(c, &c->adj_part, &c->adj_part_bytes, b_coef + b_part));
-  double2 *coef = (double2 *)c->adj_part;
-  face_current_kernel<<<dim3((F + 127) / 128, nsrc), 128, 0, c->stream>>>(F, c->N, D.hpar, D.sl, D.mu, X, ldx, coef);
-  c->launches++;
+  const int want = std::max(1, std::min(F, 8 * c->nsm / blocks));
+  const int per = (F + want - 1) / want, splits = (F + per - 1) / per;
+  MOM_TRY(ensure_buffer(c, &c->adj_part, &c->adj_part_bytes,
+                        sizeof(double2) * 6 * (size_t)npts * std::min(nsrc, 4) * splits));
   const double k0 = omega / kC0;
   NfArgs a;
   a.F = F;
@@ -342,11 +360,16 @@ int scat_fields(Ctx *c, int d, double omega, const double *ri, int nsrc, const d
   a.pts = pts;
   a.npts = npts;
   a.per_split = per;
-  a.part = (double2 *)((char *)c->adj_part + b_coef);
+  a.part = (double2 *)c->adj_part;
+  a.N = c->N;
+  a.hpar = D.hpar;
+  a.sl = D.sl;
+  a.mu = D.mu;
+  a.ldx = ldx;
   for (int s0 = 0; s0 < nsrc; s0 += 4) {
     const int ns = std::min(4, nsrc - s0);
     a.nsrc = ns;
-    a.coef = coef + 8 * (size_t)F * s0;
+    a.x = X + (size_t)s0 * ldx;
     const int nl = ns == 1 ? 1 : (ns == 2 ? 2 : 4);
     const dim3 grid(blocks, splits);
     switch (c->nq) {
@@ -358,8 +381,11 @@ int scat_fields(Ctx *c, int d, double omega, const double *ri, int nsrc, const d
       default: return fail(c, MOM_ERR_ARG, "unsupported number of quadrature points");
     }
     const int64_t vals = (int64_t)ns * npts * 6;
-    nfield_sum_kernel<<<(unsigned)((vals + 255) / 256), 256, 0, c->stream>>>(
-        npts, ns, splits, a.part, E + (size_t)s0 * npts * 3, H + (size_t)s0 * npts * 3);
+    double2 *Eo = E + (size_t)s0 * npts * 3, *Ho = H + (size_t)s0 * npts * 3;
+    if (splits > 16)  // few points (eight CTAs per SM at most: under 10,000)
+      nfield_sum_kernel<32><<<(unsigned)((vals * 32 + 255) / 256), 256, 0, c->stream>>>(npts, ns, splits, a.part, Eo, Ho);
+    else
+      nfield_sum_kernel<1><<<(unsigned)((vals + 255) / 256), 256, 0, c->stream>>>(npts, ns, splits, a.part, Eo, Ho);
     c->launches += 2;
     MOM_CUDA(c, cudaGetLastError());
   }

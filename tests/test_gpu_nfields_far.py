@@ -65,3 +65,23 @@ def test_cross_terms_far_away(built, dist):
         assert np.abs(e[i] - f).max() <= bound * size
         assert np.abs(h[i] + f).max() <= bound * size
     s.close()
+
+
+@pytest.mark.parametrize("subdiv", [0, 1, 2])
+@pytest.mark.parametrize("ns", [1, 3, 9])
+def test_splits_of_the_faces(built, subdiv, ns):
+    """The faces are split according to the number of points: one, a few and thousands give the same fields."""
+    nodes, faces = meshgen.icosphere(subdiv, 50.0)
+    s = M.Solver(0)
+    s.set_problem(M.Problem.from_arrays(nodes, faces, np.ones(len(faces), int), 1e-9, [[1], [-1]]))
+    om = M.omega_of(600e-9)
+    rng = np.random.default_rng(1)
+    x = rng.standard_normal((2 * s.N, ns)) + 1j * rng.standard_normal((2 * s.N, ns))
+    pts = rng.uniform(-1.5e-7, 1.5e-7, (20000, 3))
+    whole = s.scat_fields(om, 1.0, pts, x=x)
+    # sums of 13 points per face in another order; terms up to 100 times the sum
+    tol = 100 * 13 * len(faces) * 2.0 ** -53
+    for n in (1, 129, 2500):
+        for a, b in zip(s.scat_fields(om, 1.0, pts[:n], x=x), whole):
+            assert np.abs(a - b[:, :n]).max() <= tol * np.abs(b[:, :n]).max()
+    s.close()
