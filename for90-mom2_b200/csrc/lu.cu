@@ -2085,10 +2085,20 @@ static int lu_factor(Ctx *c, int precision, int batch) {
   return lu_factor_t<double2>(c, c->A, precision, batch);
 }
 
+// From this order on the mixed path factorises several representations one after
+// the other: their updates then run on the tensor cores, where at once they are
+// batched library FP32 GEMMs.  Below, the batch shares the panels' latency.
+// Whole calls, at once and one by one: two representations of 3,570 / 4,446 /
+// 7,056 unknowns 16.0 and 17.4 / 24.5 and 23.0 / 69 and 48 ms, eight of 3,570 /
+// 4,446 / 4,920 / 7,056 56 and 71 / 90 and 95 / 111 and 109 / 262 and 196 ms.  In
+// FP64 (ZGEMM both ways) at once is faster throughout.
+constexpr int64_t kOneByOneFromOrder = 4608;
+
 // Every representation's matrix: at once where the cluster panels serve the
 // order, else one after the other.
 int lu_factor_reps(Ctx *c, int precision) {
-  const bool at_once = precision == MOM_PREC_MIXED ? on_cluster<float2>(c, c->n) : on_cluster<double2>(c, c->n);
+  const bool at_once = precision == MOM_PREC_MIXED ? on_cluster<float2>(c, c->n) && c->n < kOneByOneFromOrder
+                                                   : on_cluster<double2>(c, c->n);
   int rc = MOM_OK;
   for (int r = 0; r < (at_once ? 1 : c->nga) && rc == MOM_OK; r++) {
     select_rep(c, r);
