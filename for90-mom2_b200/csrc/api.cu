@@ -62,6 +62,23 @@ void Ctx::LuGraph::reset() {
   tc_flops = 0;
 }
 
+bool device_alloc(Ctx *c, void **p, size_t bytes) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  if (c->blk && c->blk_bytes > c->blk_min && cudaStreamSynchronize(c->stream) == cudaSuccess) {
+    cudaFree(c->blk);
+    c->blk = nullptr;
+    c->blk_bytes = 0;
+    if (cudaMalloc(&c->blk, c->blk_min) == cudaSuccess) {
+      c->blk_bytes = c->blk_min;
+      if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+    }
+    cudaGetLastError();
+  }
+  *p = nullptr;
+  return false;
+}
+
 int ensure_buffer(Ctx *c, void **p, size_t *cap, size_t bytes) {
   if (*p && *cap >= bytes) return MOM_OK;
   if (*p) {
@@ -71,11 +88,8 @@ int ensure_buffer(Ctx *c, void **p, size_t *cap, size_t bytes) {
     *cap = 0;
   }
   const size_t want = std::max<size_t>(bytes, 1 << 20);
-  if (cudaMalloc(p, want) != cudaSuccess) {
-    cudaGetLastError();
-    *p = nullptr;
+  if (!device_alloc(c, p, want))
     return fail(c, MOM_ERR_ALLOC, "device allocation of " + std::to_string(want) + " bytes failed");
-  }
   *cap = want;
   return MOM_OK;
 }
@@ -317,8 +331,7 @@ int ensure_rhs(Ctx *c, int nsrc) {
   cudaFree(c->X);
   c->B = c->X = nullptr;
   c->BX_cap = 0;
-  if (cudaMalloc(&c->B, need) != cudaSuccess || cudaMalloc(&c->X, need) != cudaSuccess) {
-    cudaGetLastError();
+  if (!device_alloc(c, (void **)&c->B, need) || !device_alloc(c, (void **)&c->X, need)) {
     return fail(c, MOM_ERR_ALLOC, "right-hand side allocation failed");
   }
   c->BX_cap = need;
@@ -328,9 +341,8 @@ int ensure_rhs(Ctx *c, int nsrc) {
 int ensure_a32(Ctx *c) {
   if (c->A32_all) return MOM_OK;
   const size_t bytes = sizeof(float2) * (size_t)c->lda * c->n * c->nga;
-  if (cudaMalloc(&c->A32_all, bytes) != cudaSuccess ||
-      cudaMalloc(&c->inv32_all, sizeof(float2) * 2 * (size_t)c->nb * c->n * c->nga) != cudaSuccess) {
-    cudaGetLastError();
+  if (!device_alloc(c, (void **)&c->A32_all, bytes) ||
+      !device_alloc(c, (void **)&c->inv32_all, sizeof(float2) * 2 * (size_t)c->nb * c->n * c->nga)) {
     cudaFree(c->A32_all);
     c->A32_all = nullptr;
     return fail(c, MOM_ERR_ALLOC, "FP32 matrix allocation failed");
@@ -571,6 +583,7 @@ int mom_gpu_set_problem(mom_ctx *c, int32_t nedges_total, int32_t ndom, const mo
   c->removed.assign(1, {});
   c->removed_off.assign(2, 0);
   c->edge_bnd.assign(c->N, MOM_BND_NONE);
+  c->blk_min = c->blk_bytes;
   if (cudaMalloc(&c->blk, c->blk_bytes) != cudaSuccess || alloc_representations(c, 1) != MOM_OK) {
     cudaGetLastError();
     free_problem(c);

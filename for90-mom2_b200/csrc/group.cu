@@ -164,17 +164,22 @@ int alloc_representations(Ctx *c, int nga) {
 }
 
 // Room for the face-pair blocks of several group actions at once (the gather
-// adds them to the matrices in one pass) where it leaves the FP32 copies and
-// 4 GiB free; otherwise of fewer, down to what there is.
+// adds them to the matrices in one pass), of as many as fit 1 GiB and a sixteenth
+// of the free memory: other contexts and the buffers to come have prior claim
+// (what is beyond blk_min is also given back when an allocation fails).  Eight
+// actions fit up to about 2,100 unknowns per representation, four to 3,000, and
+// the problem's own buffer holds two of two domains.  Gather with eight actions,
+// one pass and these: 2,268 unknowns 1.3 and 1.6 ms, 4,920 6.1 and 10.5 (of a
+// call of 112), 12,480 40 and 66 (of 583); an action at a time 7.7, 31 and 220.
 void grow_blocks(Ctx *c, int nga) {
   size_t one = 0;
   for (const auto &D : c->dom) one = std::max(one, sizeof(double2) * 18 * (size_t)D.F * D.F);
   size_t fr = 0, tot = 0;
   if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return;
-  const size_t keep = c->A_bytes / 2 + (size_t(4) << 30);
+  const size_t most = std::min(fr / 16, size_t(1) << 30);
   for (; nga > 1 && one * nga > c->blk_bytes; nga /= 2) {
     double2 *b = nullptr;
-    if (fr < one * nga + keep) continue;
+    if (one * nga > most) continue;
     if (cudaMalloc(&b, one * nga) != cudaSuccess) {
       cudaGetLastError();
       continue;

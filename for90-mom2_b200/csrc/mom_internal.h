@@ -172,6 +172,7 @@ struct Ctx {
   size_t A_bytes = 0, A32_bytes = 0;
   double2 *blk = nullptr;  // face-pair blocks [source F][test F][9][2] of the largest domain
   size_t blk_bytes = 0;    //   (for several group actions) or, when blk_fused, of every domain at blk + blk_off[d]
+  size_t blk_min = 0;      // what the problem needs without the group; the rest is given back when memory runs short
   bool blk_fused = false;
   std::vector<size_t> blk_off;  // [ndom], in double2
   int *dmap = nullptr;     // [ndom][N]: domain edge of each global edge, -1 if none
@@ -329,6 +330,8 @@ int cuda_fail(Ctx *c, cudaError_t e, const char *where);
   } while (0)
 
 int ensure_buffer(Ctx *c, void **p, size_t *cap, size_t bytes);
+// cudaMalloc, again after giving back what the block buffer has beyond blk_min.
+bool device_alloc(Ctx *c, void **p, size_t bytes);
 
 // Points A, A32, ipiv, perm, invd, inv32 at representation r's buffers.
 inline void select_rep(Ctx *c, int r) {

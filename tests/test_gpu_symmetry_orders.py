@@ -34,3 +34,25 @@ def test_large_mixed_representations(built):
         sig[prec] = np.concatenate(s.cross_sections(om, ri[0], srcs))
     assert np.abs(sig[M.MIXED] - sig[M.FP64]).max() <= 1e-6 * np.abs(sig[M.FP64]).min()
     s.close()
+
+
+def test_memory_of_a_group(built):
+    """Setting a group takes the memory of its matrices and, for the blocks of several actions at once, 1 GiB at most."""
+    import torch
+    nodes, faces = meshgen.octasphere(5, 50.0)
+    fn, ff, lines = meshgen.symmetry_fragment(nodes, faces, [0, 1])
+    p = M.Problem.from_arrays(fn, ff, np.ones(len(ff), int), 1e-9, [[1], [-1]])
+    p.set_lines(np.concatenate([np.asarray(lines[ax], np.int32).reshape(-1, 2) for ax in (0, 1)]),
+                np.concatenate([np.full(len(lines[ax]), 10 + ax, np.int32) for ax in (0, 1)]))
+    for ax, name in enumerate(("xplane", "yplane")):
+        p.classify_edges(10 + ax, name)
+    s = M.Solver(0)
+    s.set_problem(p)
+    before = torch.cuda.mem_get_info()[0]
+    s.set_symmetry(["mxp", "myp"], p)
+    taken = before - torch.cuda.mem_get_info()[0]
+    n = -(-2 * s.N // 64) * 64
+    # three more matrices and diagonal inverses; mapped geometry and near pairs of three actions and two domains
+    # (432 bytes of closed forms per pair, at most 100 pairs per face)
+    assert taken <= 3 * 16 * n * (n + 128) + 6 * 440 * 100 * len(ff) + (1 << 30)
+    s.close()
