@@ -8,16 +8,21 @@
 //   Ahat[2i+1][2l+1] = Re L
 // and U12 viewed as real 2k x nc (its own interleaved storage), C -= Ahat B.
 // Accuracy: each operand is split into two FP16 numbers, high part and
-// remainder, after a scaling by a power of two per row of L21 and per column
-// of U12 that puts its largest entry just below 2^15; the MMA accumulates
-// hi*hi + hi*lo + lo*hi (three kind::f16 passes into one FP32 TMEM
-// accumulator) and the epilogue undoes the scaling.  An entry keeps 22 bits, or
-// 2^-40 of its row's (column's) largest entry.  Three passes on TF32 parts keep
-// no more (the tensor core cuts the remainder to TF32) at half the rate and
-// twice the operand bytes.  Measured, relative Frobenius error of C - L U
-// against FP64, Gaussian operands (rows and columns scaled by any powers of
-// two alike), k = 16 / 48 / 64 / 128 / 256: 2.0e-7 / 4.3e-7 / 5.3e-7 / 9.8e-7 /
-// 1.9e-6, with TF32 parts 3.0e-7 / 7.5e-7 / 9.6e-7 / 1.9e-6 / 3.7e-6.
+// remainder, after scalings by powers of two: per column of L21 (and inversely
+// per row of U12) one that brings the columns' largest entries level, then per
+// row of L21 and per column of U12 one that puts its largest entry just below
+// 2^15; the MMA accumulates hi*hi + hi*lo + lo*hi (three kind::f16 passes into
+// one FP32 TMEM accumulator) and the epilogue undoes the scaling.  An entry
+// keeps 22 bits, or 2^-40 of its row's (column's) largest scaled entry: rows of
+// A of any sizes, which grade L by column against U by row, cost nothing, and
+// an error in column j of the update stays below k 2^-39 of the largest
+// entry of column j of |L| |U|, as every column of L has an entry at its level.
+// Three passes on TF32 parts keep no more (the tensor core cuts the remainder
+// to TF32) at half the rate and twice the operand bytes.  Measured, relative
+// Frobenius error of C - L U against FP64, Gaussian operands (rows and columns
+// scaled by any powers of two alike), k = 16 / 48 / 64 / 128 / 256: 2.0e-7 /
+// 4.3e-7 / 5.3e-7 / 9.8e-7 / 1.9e-6, with TF32 parts 3.0e-7 / 7.5e-7 / 9.6e-7 /
+// 1.9e-6 / 3.7e-6.
 //
 // Kernel: persistent, one CTA per SM, 128 x 256 output tiles, K blocks of
 // 32 halves (one 64-byte swizzle row) staged by TMA in a 4-deep ring (three
@@ -40,6 +45,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstdint>
 #include <cstring>
 
@@ -337,6 +343,49 @@ __device__ __forceinline__ float scale_of(unsigned bits, float *inv) {
 __device__ __forceinline__ unsigned mag_bits(float2 z) {
   return max(__float_as_uint(fabsf(z.x)), __float_as_uint(fabsf(z.y)));
 }
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float((unsigned)(127 + e) << 23); }
+
+// level[l]: biased exponent of the largest finite entry of column l of the
+// complex block L (m x k, ld; tr: of the transpose of a k x m block), -1 if there
+// is none.  One CTA per column (tr: per four, whose entries lie side by side).
+__global__ void __launch_bounds__(256) col_level_kernel(const float2 *L, int64_t ld, int m, int k, int *level, bool tr) {
+  __shared__ unsigned s_max[8][4];
+  const int per = tr ? 4 : 1, l0 = blockIdx.x * per;
+  unsigned b[4] = {0u, 0u, 0u, 0u};
+  auto take = [&](unsigned &o, float2 z) {
+    const unsigned v = mag_bits(z);
+    if (v < 0x7f800000u) o = max(o, v);
+  };
+  if (!tr) {
+#pragma unroll 8
+    for (int i = threadIdx.x; i < m; i += 256) take(b[0], L[i + (int64_t)l0 * ld]);
+  } else {
+#pragma unroll 2
+    for (int i = threadIdx.x; i < m; i += 256)
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (l0 + q < k) take(b[q], L[l0 + q + (int64_t)i * ld]);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    b[q] = __reduce_max_sync(0xffffffffu, b[q]);
+    if (threadIdx.x % 32 == 0) s_max[threadIdx.x / 32][q] = b[q];
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < per && l0 + (int)threadIdx.x < k) {
+    unsigned v = 0u;
+    for (int w = 0; w < 8; w++) v = max(v, s_max[w][threadIdx.x]);
+    level[l0 + threadIdx.x] = v == 0u ? -1 : (int)(v >> 23);
+  }
+}
+// The highest level, by a whole warp; and by how many powers of two column l is
+// raised to it.
+__device__ __forceinline__ int top_level(const int *level, int k) {
+  int t = -1;
+  for (int l = threadIdx.x % 32; l < k; l += 32) t = max(t, level[l]);
+  return __reduce_max_sync(0xffffffffu, t);
+}
+__device__ __forceinline__ int raised(int level, int top) { return level < 0 ? 0 : min(126, top - level); }
 // v = hi + lo up to FP16 rounding of the remainder
 __device__ __forceinline__ void split_half(float v, __half *hi, __half *lo) {
   *hi = __float2half_rn(v);
@@ -345,27 +394,32 @@ __device__ __forceinline__ void split_half(float v, __half *hi, __half *lo) {
 
 // Ahat_hi / Ahat_lo (2m x Kp halves, row-major) from the complex block L
 // (m x k, ld), or (tr) from the transpose of a k x m block: L(i, l) = P[l + i
-// ld], and the rows' inverse scales.  One CTA (32 x 8 threads) per 32 rows:
-// their largest entries first, then 32 x 32 tiles through shared memory, the
+// ld], its columns raised to one level, and the rows' inverse scales.  One CTA
+// (32 x 8 threads) per 32 rows: their largest entries first, then 32 x 32 tiles through shared memory, the
 // complex block read along its contiguous direction both times (the second
 // time from L2) and the expanded rows written as pairs of halves.
 __global__ void __launch_bounds__(256) expand_a_kernel(const float2 *L, int64_t ld, int m, int k, int Kp, __half *hi,
-                                                       __half *lo, float *rinv, bool tr) {
+                                                       __half *lo, float *rinv, const int *level, bool tr) {
   __shared__ float2 t[32][33];  // [l][i] of the tile
   __shared__ unsigned s_max[32];
   const int i0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
+  const int top = top_level(level, k);
+  auto at = [&](float2 z, int l) {
+    const float up = pow2(raised(level[l], top));
+    return make_float2(z.x * up, z.y * up);
+  };
   if (ty == 0) s_max[tx] = 0u;
   __syncthreads();
   if (!tr) {
     unsigned b = 0u;
     if (i0 + tx < m)
-      for (int l = ty; l < k; l += 8) b = max(b, mag_bits(L[i0 + tx + (int64_t)l * ld]));
+      for (int l = ty; l < k; l += 8) b = max(b, mag_bits(at(L[i0 + tx + (int64_t)l * ld], l)));
     atomicMax(&s_max[tx], b);
   } else {
     for (int r = ty; r < 32; r += 8) {
       unsigned b = 0u;
       if (i0 + r < m)
-        for (int l = tx; l < k; l += 32) b = max(b, mag_bits(L[l + (int64_t)(i0 + r) * ld]));
+        for (int l = tx; l < k; l += 32) b = max(b, mag_bits(at(L[l + (int64_t)(i0 + r) * ld], l)));
       b = __reduce_max_sync(0xffffffffu, b);
       if (tx == 0) s_max[r] = b;
     }
@@ -375,10 +429,10 @@ __global__ void __launch_bounds__(256) expand_a_kernel(const float2 *L, int64_t 
     for (int r = ty; r < 32; r += 8) {
       if (!tr) {
         const int i = i0 + tx, l = l0 + r;
-        t[r][tx] = (i < m && l < k) ? L[i + (int64_t)l * ld] : make_float2(0.f, 0.f);
+        t[r][tx] = (i < m && l < k) ? at(L[i + (int64_t)l * ld], l) : make_float2(0.f, 0.f);
       } else {
         const int l = l0 + tx, i = i0 + r;
-        t[tx][r] = (i < m && l < k) ? L[l + (int64_t)i * ld] : make_float2(0.f, 0.f);
+        t[tx][r] = (i < m && l < k) ? at(L[l + (int64_t)i * ld], l) : make_float2(0.f, 0.f);
       }
     }
     __syncthreads();
@@ -402,22 +456,30 @@ __global__ void __launch_bounds__(256) expand_a_kernel(const float2 *L, int64_t 
 }
 
 // B_hi / B_lo (nc x Kp halves, K contiguous) from the complex block U (k x nc,
-// ld) and the columns' inverse scales: one warp per column.
+// ld), its rows lowered by what L's columns were raised, and the columns'
+// inverse scales: one warp per column.  An entry's two scalings are one power of
+// two (applied in halves, since it may leave FP32's range).
 __global__ void __launch_bounds__(256) split_b_kernel(const float2 *U, int64_t ld, int k, int nc, int Kp, __half *hi,
-                                                      __half *lo, float *cinv) {
+                                                      __half *lo, float *cinv, const int *level) {
   const int lane = threadIdx.x & 31, j = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (j >= nc) return;
   const float2 *u = U + (int64_t)j * ld;
-  unsigned b = 0u;
-  for (int l = lane; l < k; l += 32) b = max(b, mag_bits(u[l]));
-  float inv;
-  const float sc = scale_of(__reduce_max_sync(0xffffffffu, b), &inv);
-  if (lane == 0) cinv[j] = inv;
+  const int top = top_level(level, k);
+  int b = INT_MIN;  // bits of the largest magnitude, less the powers of two
+  for (int l = lane; l < k; l += 32) {
+    const unsigned v = mag_bits(u[l]);
+    if (v != 0u) b = max(b, (int)v - (raised(level[l], top) << 23));
+  }
+  b = __reduce_max_sync(0xffffffffu, b);
+  const int s = b == INT_MIN ? 0 : min(126, max(-126, 141 - (b >> 23)));
+  if (lane == 0) cinv[j] = pow2(-s);
   for (int l = lane; l < Kp / 2; l += 32) {
     const float2 z = l < k ? u[l] : make_float2(0.f, 0.f);
+    const int f = s - (l < k ? raised(level[l], top) : 0);
+    const float f1 = pow2(f >> 1), f2 = pow2(f - (f >> 1));
     __half2 h, g;
-    split_half(z.x * sc, &h.x, &g.x);
-    split_half(z.y * sc, &h.y, &g.y);
+    split_half(z.x * f1 * f2, &h.x, &g.x);
+    split_half(z.y * f1 * f2, &h.y, &g.y);
     reinterpret_cast<__half2 *>(hi + (int64_t)j * Kp)[l] = h;
     reinterpret_cast<__half2 *>(lo + (int64_t)j * Kp)[l] = g;
   }
@@ -481,13 +543,17 @@ int tc_cgemm_update(Ctx *c, float2 *C, int64_t ldc, const float2 *L, int64_t ldl
   // the expansion of L first: its place must not depend on nc (reuse_a)
   __half *ahi = (__half *)take(sizeof(__half) * (size_t)Mr * Kp), *alo = (__half *)take(sizeof(__half) * (size_t)Mr * Kp);
   float *rinv = (float *)take(sizeof(float) * m);
+  int *level = (int *)take(sizeof(int) * k);
   __half *bhi = (__half *)take(sizeof(__half) * (size_t)nc * Kp), *blo = (__half *)take(sizeof(__half) * (size_t)nc * Kp);
   float *cinv = (float *)take(sizeof(float) * nc);
   if (!reuse_a) {
-    expand_a_kernel<<<(unsigned)((m + 31) / 32), dim3(32, 8), 0, c->stream>>>(L, ldl, m, k, Kp, ahi, alo, rinv, trans_l);
-    c->launches++;
+    col_level_kernel<<<(unsigned)(trans_l ? (k + 3) / 4 : k), 256, 0, c->stream>>>(L, ldl, m, k, level, trans_l);
+    expand_a_kernel<<<(unsigned)((m + 31) / 32), dim3(32, 8), 0, c->stream>>>(L, ldl, m, k, Kp, ahi, alo, rinv, level,
+                                                                               trans_l);
+    c->launches += 2;
   }
-  split_b_kernel<<<(unsigned)((nc + 7) / 8), 256, 0, c->stream>>>(U, ldu, k, nc, Kp, bhi, blo, cinv);
+  split_b_kernel<<<(unsigned)((nc + 7) / 8), 256, 0, c->stream>>>(U, ldu, k, nc, Kp, bhi, blo, cinv,
+                                                                         level);
   c->launches++;
   CUtensorMap mAhi, mAlo, mBhi, mBlo;
   MOM_TRY(make_map(c, &mAhi, ahi, Mr, Kp, kBM));
@@ -528,7 +594,7 @@ int tc_init_kernels(Ctx *c) {
 
 size_t tc_cgemm_work_bytes(int m, int nc, int k) {
   const size_t Kp = padded_k(k);
-  return 2 * up256(sizeof(__half) * 2 * (size_t)m * Kp) + up256(sizeof(float) * m) +
+  return 2 * up256(sizeof(__half) * 2 * (size_t)m * Kp) + up256(sizeof(float) * m) + up256(sizeof(int) * k) +
          2 * up256(sizeof(__half) * (size_t)nc * Kp) + up256(sizeof(float) * nc);
 }
 

@@ -134,6 +134,26 @@ def test_bounded_wait_of_the_cluster_panels(prec):
     s.close()
 
 
+@pytest.mark.parametrize("ns", [1, 70])
+@pytest.mark.parametrize("exponent", [20, 40])
+def test_rows_of_two_sizes(exponent, ns):
+    """Half of the rows are 2^-exponent times the others: the mixed factorisation, before any refinement, solves
+    a system whose rows differ from these by n 2^-24 of their own size (FP32 arithmetic throughout), and the
+    small rows' part of an update is not lost where both kinds are pivots of one block."""
+    s = problem(4)
+    n = 2 * s.N
+    rng = np.random.default_rng(9)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    A[rng.permutation(n)[:n // 2 + 29]] *= 2.0 ** -exponent
+    srcs = W.incidences(ns)
+    q = s.srcvec(OM, RI[0], srcs, want_host=True)
+    s.set_matrix(A, M.MIXED)
+    x = s.solve(M.MIXED, 1e30, 1)
+    r = np.abs(A @ x - q)
+    assert np.all(r <= n * 2.0 ** -24 * (np.abs(A) @ np.abs(x)))
+    s.close()
+
+
 def test_tallest_cluster_panels():
     s = problem(5)
     assert 2 * s.N == 24576
