@@ -8,11 +8,13 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <thread>
 #include <vector>
 
 #include "mom_internal.h"
+#include "sweep_policy.h"
 
 namespace mom {
 
@@ -746,8 +748,12 @@ int mom_gpu_sweep_many(int32_t nctx, mom_ctx **ctx, const int32_t *nwl, const do
   std::vector<int> st(nctx, MOM_OK);
   std::vector<std::thread> th;
   th.reserve(nctx);
+  std::vector<int> device(nctx);
+  for (int i = 0; i < nctx; i++) device[i] = ctx[i] ? ctx[i]->device : -1;
+  std::unique_ptr<bool[]> crowded(new bool[nctx]);
+  crowded_contexts(nctx, device.data(), crowded.get());
   for (int i = 0; i < nctx; i++)
-    if (ctx[i]) ctx[i]->crowded = nctx >= kCrowd;
+    if (ctx[i]) ctx[i]->crowded = crowded[i];
   for (int i = 0; i < nctx; i++)
     th.emplace_back([&, i]() {
       st[i] = mom_gpu_sweep(ctx[i], nwl[i], omega[i], ri[i], nsrc, src, precision, tol, maxit, csca[i], cabs[i],

@@ -28,12 +28,6 @@ constexpr int kMaxQ = 13;
 constexpr size_t kBlasWorkspace = 64u << 20;
 
 constexpr int kMaxGroup = MOM_MAX_GROUP;
-// Contexts of one sweep from which on each factorises on one stream.  The device
-// serves eight queues of launches: a second branch per context makes contexts
-// wait for one another.  Sweeps of up to 3,840 unknowns, with and without the
-// branch: 4 contexts 172 and 192 ms, 8 contexts 149 and 149 (four particles) and
-// 103 and 90 (two), 12 contexts 147 and 138, 16 contexts 144 and 127.
-constexpr int kCrowd = 8;
 
 // One element of a symmetry group (group_action, symmetry.f90:24-40): point
 // action J (row-major, j[3 i + k] = J(i, k)), det J, the special-action id
@@ -221,7 +215,7 @@ struct Ctx {
     void reset();
   };
   std::vector<LuGraph *> lu_graphs;  // by key (one per precision and representation)
-  std::atomic<bool> crowded{false};  // kCrowd contexts or more at work: LU without the look-ahead branch
+  std::atomic<bool> crowded{false};  // kCrowd contexts or more at work on the device: LU without the look-ahead branch
   bool use_graph = true;   // MOM_LU_GRAPH=0 turns graph replay off (every launch issued eagerly)
   // Panel parallelism: CTAs per panel as a function of the panel's rows m,
   // autotuned per (matrix order, precision) at the first factorisation
