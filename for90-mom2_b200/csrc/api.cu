@@ -430,7 +430,7 @@ int mom_gpu_create(int32_t device, mom_ctx **out) {
             cublasSetStream(c->blas2, c->stream2) == CUBLAS_STATUS_SUCCESS &&
             cudaMalloc(&c->blas_ws2, kBlasWorkspace) == cudaSuccess &&
             cublasSetWorkspace(c->blas2, c->blas_ws2, kBlasWorkspace) == CUBLAS_STATUS_SUCCESS;
-  for (int i = 0; ok && i < 3; i++) ok = cudaEventCreateWithFlags(&c->la_ev[i], cudaEventDisableTiming) == cudaSuccess;
+  for (int i = 0; ok && i < 4; i++) ok = cudaEventCreateWithFlags(&c->la_ev[i], cudaEventDisableTiming) == cudaSuccess;
   if (!ok || lu_init_kernels(c) != MOM_OK || tc_init_kernels(c) != MOM_OK) {
     cudaGetLastError();
     cublasDestroy(c->blas);

@@ -1597,7 +1597,8 @@ constexpr int64_t kOuterFromOrder = 8192;
 //   stream 1: panel J's interchanges and U12 on the next panel's 64 columns and
 //             their update; then the same on the columns right of them (and
 //             the interchanges left of J) and the large update, beside
-//   stream 2: panel J+1, one launch on one cluster, so that it keeps its SMs.
+//   stream 2: the expansion of L21 for the tensor cores, and panel J+1, one
+//             launch on one cluster, so that it keeps its SMs.
 // A panel is a serial chain of 64 pivot decisions on 16 SMs (64-126 us); the
 // large update takes the other SMs, so whichever is longer hides the other.
 template <typename T>
@@ -1659,6 +1660,17 @@ int lu_enqueue_cluster(Ctx *c, T *A, const LuWork &w, int batch) {
       break;
     }
     if (ahead && t0 + nb < n) {
+      // stream 2 waits for the next panel's columns: meanwhile it prepares L21
+      // for the large update
+      const bool tc = f32 && batch == 1 && n >= kTcFromOrder && n - (t0 + nb) > nb;
+      if constexpr (f32)
+        if (tc) {
+          MOM_CUDA(c, cudaEventRecord(c->la_ev[0], sa));
+          MOM_CUDA(c, cudaStreamWaitEvent(sb, c->la_ev[0], 0));
+          ProfScope ps(c, kProfGemm, sb);
+          MOM_TRY(tc_cgemm_expand(c, sb, A + t0 + j0 * lda, lda, (int)(n - t0), nb, w.tcw));
+          MOM_CUDA(c, cudaEventRecord(c->la_ev[3], sb));
+        }
       MOM_TRY(swaps(j0, t0, t0 + nb, 0, nullptr));
       MOM_TRY(update(j0, t0, t0 + nb, 0, false));
       MOM_CUDA(c, cudaEventRecord(c->la_ev[1], sa));
@@ -1666,7 +1678,8 @@ int lu_enqueue_cluster(Ctx *c, T *A, const LuWork &w, int batch) {
       MOM_TRY(panel(t0, sb, true));
       MOM_CUDA(c, cudaEventRecord(c->la_ev[2], sb));
       MOM_TRY(swaps(j0, t0 + nb, n, j0, c->perm));
-      MOM_TRY(update(j0, t0 + nb, n, std::max(8, c->nsm - c->panel_cluster), false));
+      if (tc) MOM_CUDA(c, cudaStreamWaitEvent(sa, c->la_ev[3], 0));
+      MOM_TRY(update(j0, t0 + nb, n, std::max(8, c->nsm - c->panel_cluster), tc));
       MOM_CUDA(c, cudaStreamWaitEvent(sa, c->la_ev[2], 0));
     } else {
       MOM_TRY(swaps(j0, t0, n, j0, c->perm));
@@ -2255,9 +2268,11 @@ int getrs_multi(Ctx *c, const T *F, double2 *X, int nrhs, int trans) {
   const bool tc = f32 && nrhs >= kMultiTc;
   const size_t ybytes = sizeof(T) * (size_t)n * nrhs, o_w = ((ybytes + 255) / 256) * 256;
   const size_t wbytes = tc ? tc_cgemm_work_bytes((int)n, nrhs, kTriRows) : 0;
-  MOM_TRY(ensure_buffer(c, &c->ws2, &c->ws2_bytes, o_w + wbytes + 1024));
+  const size_t o_l = o_w + (wbytes + 255) / 256 * 256;
+  MOM_TRY(ensure_buffer(c, &c->ws2, &c->ws2_bytes, o_l + sizeof(int) * 2 * n + 1024));
   T *Y = (T *)c->ws2;
   float *tw = (float *)((char *)c->ws2 + o_w);
+  int *levels = (int *)((char *)c->ws2 + o_l);  // [after, before][n]
   const T *inv = f32 ? (const T *)c->inv32 : (const T *)c->invd;
   ProfScope ps(c, kProfTrsv);
   const dim3 pg((unsigned)((n + 255) / 256), nrhs);
@@ -2278,9 +2293,10 @@ int getrs_multi(Ctx *c, const T *F, double2 *X, int nrhs, int trans) {
     if (tc)
       return tc_cgemm_update(c, reinterpret_cast<float2 *>(Y + i0), n, reinterpret_cast<const float2 *>(Ab), lda,
                              reinterpret_cast<const float2 *>(Y + K0), n, m, nrhs, rows, tw, c->dinfo + 2, 0, false,
-                             trans != 0);
+                             trans != 0, levels + (lower ? 0 : n) + K0);
     return blas_gemm<T>(c, trans ? CUBLAS_OP_T : CUBLAS_OP_N, m, nrhs, rows, -1.0, Ab, lda, Y + K0, n, 1.0, Y + i0, n);
   };
+  if (tc) MOM_TRY(tc_block_levels(c, reinterpret_cast<const float2 *>(F), lda, (int)n, kTriRows, trans != 0, levels, levels + n));
   // forward: L (unit lower), or U^T; backward: U, or L^T (unit upper)
   for (int64_t K0 = 0; K0 < n; K0 += kTriRows) MOM_TRY(step(K0, true, std::min<int64_t>(K0 + kTriRows, n), n));
   for (int64_t K0 = (n - 1) / kTriRows * kTriRows; K0 >= 0; K0 -= kTriRows) MOM_TRY(step(K0, false, 0, K0));

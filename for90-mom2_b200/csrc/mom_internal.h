@@ -121,7 +121,7 @@ struct Ctx {
   cudaStream_t stream2 = nullptr;
   cublasHandle_t blas2 = nullptr;
   void *blas_ws2 = nullptr;
-  cudaEvent_t la_ev[3] = {nullptr, nullptr, nullptr};
+  cudaEvent_t la_ev[4] = {nullptr, nullptr, nullptr, nullptr};
   int lookahead = 1;       // MOM_LOOKAHEAD=0 turns it off
   // Defaults from a sweep on a B200 at n = 30,720 (the cap 32/48/64 and the
   // fraction 0.9/0.95/all within 3% of each other; these were the fastest).
@@ -402,7 +402,9 @@ int panel_init_kernels(Ctx *c);
 // tc_gemm.cu: C -= L U (complex FP32) on the tensor cores, FP32-accurate
 int tc_cgemm_update(Ctx *c, float2 *C, int64_t ldc, const float2 *L, int64_t ldl, const float2 *U, int64_t ldu, int m,
                     int nc, int k, float *work, int *err, int max_ctas = 0, bool reuse_a = false,
-                    bool trans_l = false);
+                    bool trans_l = false, const int *levels = nullptr);
+int tc_cgemm_expand(Ctx *c, cudaStream_t st, const float2 *L, int64_t ldl, int m, int k, float *work);
+int tc_block_levels(Ctx *c, const float2 *F, int64_t lda, int n, int rows, bool trans, int *after, int *before);
 size_t tc_cgemm_work_bytes(int m, int nc, int k);
 int tc_init_kernels(Ctx *c);
 

@@ -345,6 +345,13 @@ __device__ __forceinline__ unsigned mag_bits(float2 z) {
 }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((unsigned)(127 + e) << 23); }
 
+// The larger of m and the magnitude of z, if that is finite.
+__device__ __forceinline__ void take_mag(unsigned &m, float2 z) {
+  const unsigned v = mag_bits(z);
+  if (v < 0x7f800000u) m = max(m, v);
+}
+__device__ __forceinline__ int level_of(unsigned bits) { return bits == 0u ? -1 : (int)(bits >> 23); }
+
 // level[l]: biased exponent of the largest finite entry of column l of the
 // complex block L (m x k, ld; tr: of the transpose of a k x m block), -1 if there
 // is none.  One CTA per column (tr: per four, whose entries lie side by side).
@@ -352,19 +359,15 @@ __global__ void __launch_bounds__(256) col_level_kernel(const float2 *L, int64_t
   __shared__ unsigned s_max[8][4];
   const int per = tr ? 4 : 1, l0 = blockIdx.x * per;
   unsigned b[4] = {0u, 0u, 0u, 0u};
-  auto take = [&](unsigned &o, float2 z) {
-    const unsigned v = mag_bits(z);
-    if (v < 0x7f800000u) o = max(o, v);
-  };
   if (!tr) {
 #pragma unroll 8
-    for (int i = threadIdx.x; i < m; i += 256) take(b[0], L[i + (int64_t)l0 * ld]);
+    for (int i = threadIdx.x; i < m; i += 256) take_mag(b[0], L[i + (int64_t)l0 * ld]);
   } else {
 #pragma unroll 2
     for (int i = threadIdx.x; i < m; i += 256)
 #pragma unroll
       for (int q = 0; q < 4; q++)
-        if (l0 + q < k) take(b[q], L[l0 + q + (int64_t)i * ld]);
+        if (l0 + q < k) take_mag(b[q], L[l0 + q + (int64_t)i * ld]);
   }
 #pragma unroll
   for (int q = 0; q < 4; q++) {
@@ -375,17 +378,54 @@ __global__ void __launch_bounds__(256) col_level_kernel(const float2 *L, int64_t
   if ((int)threadIdx.x < per && l0 + (int)threadIdx.x < k) {
     unsigned v = 0u;
     for (int w = 0; w < 8; w++) v = max(v, s_max[w][threadIdx.x]);
-    level[l0 + threadIdx.x] = v == 0u ? -1 : (int)(v >> 23);
+    level[l0 + threadIdx.x] = level_of(v);
   }
 }
-// The highest level, by a whole warp; and by how many powers of two column l is
-// raised to it.
-__device__ __forceinline__ int top_level(const int *level, int k) {
-  int t = -1;
-  for (int l = threadIdx.x % 32; l < k; l += 32) t = max(t, level[l]);
-  return __reduce_max_sync(0xffffffffu, t);
+
+// The levels of every operand of a blocked substitution at once: column l (TR:
+// row l) of the n x n factors over the rows (columns) after its block of `rows`
+// into after[l] and over those before it into before[l].  Reads the factors
+// once (HBM bound, 75 us at 7,680 unknowns), where a launch per operand added 9
+// us to each of the 60 updates of a solve.
+template <bool TR>
+__global__ void __launch_bounds__(1024) block_levels_kernel(const float2 *F, int64_t lda, int n, int rows, int *after,
+                                                            int *before) {
+  __shared__ unsigned s_max[2][32][33];
+  const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
+  // TR: a warp reads 32 rows of a column, else 32 rows of one of its column's
+  const int l = TR ? blockIdx.x * 32 + lane : blockIdx.x * 4 + wid / 8;
+  unsigned b[2] = {0u, 0u};
+  if (l < n) {
+    const int k0 = l / rows * rows, k1 = min(n, k0 + rows);
+    const int first = TR ? wid : (wid % 8) * 32 + lane, step = TR ? 32 : 256;
+#pragma unroll 8
+    for (int i = first; i < n; i += step)
+      if (i < k0 || i >= k1) take_mag(b[i < k0], TR ? F[l + (int64_t)i * lda] : F[i + (int64_t)l * lda]);
+  }
+#pragma unroll
+  for (int q = 0; q < 2; q++) s_max[q][wid][lane] = TR ? b[q] : __reduce_max_sync(0xffffffffu, b[q]);
+  __syncthreads();
+  if (threadIdx.x < (TR ? 32 : 4)) {
+    const int at = TR ? blockIdx.x * 32 + threadIdx.x : blockIdx.x * 4 + threadIdx.x;
+    for (int q = 0; q < 2 && at < n; q++) {
+      unsigned v = 0u;
+      for (int w = 0; w < (TR ? 32 : 8); w++) v = max(v, TR ? s_max[q][w][threadIdx.x] : s_max[q][threadIdx.x * 8 + w][0]);
+      (q ? before : after)[at] = level_of(v);
+    }
+  }
 }
-__device__ __forceinline__ int raised(int level, int top) { return level < 0 ? 0 : min(126, top - level); }
+// By how many powers of two each of the k columns is raised to the highest
+// level, staged by a CTA of 256 threads (every warp finds the top).
+constexpr int kMaxK = 1024;
+__device__ __forceinline__ void stage_raise(const int *level, int k, int *up) {
+  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
+  int top = -1;
+#pragma unroll 8
+  for (int l = tid % 32; l < k; l += 32) top = max(top, level[l]);
+  top = __reduce_max_sync(0xffffffffu, top);
+  for (int l = tid; l < k; l += 256) up[l] = level[l] < 0 ? 0 : min(126, top - level[l]);
+  __syncthreads();
+}
 // v = hi + lo up to FP16 rounding of the remainder
 __device__ __forceinline__ void split_half(float v, __half *hi, __half *lo) {
   *hi = __float2half_rn(v);
@@ -395,7 +435,8 @@ __device__ __forceinline__ void split_half(float v, __half *hi, __half *lo) {
 // Ahat_hi / Ahat_lo (2m x Kp halves, row-major) from the complex block L
 // (m x k, ld), or (tr) from the transpose of a k x m block: L(i, l) = P[l + i
 // ld], its columns raised to one level, and the rows' inverse scales.  One CTA
-// (32 x 8 threads) per 32 rows: their largest entries first, then 32 x 32 tiles through shared memory, the
+// (32 x 8 threads) per 32 rows and gridDim.y-th of the columns: the rows' largest
+// entries first, then 32 x 32 tiles through shared memory, the
 // complex block read along its contiguous direction both times (the second
 // time from L2) and the expanded rows written as pairs of halves.
 __global__ void __launch_bounds__(256) expand_a_kernel(const float2 *L, int64_t ld, int m, int k, int Kp, __half *hi,
@@ -403,28 +444,32 @@ __global__ void __launch_bounds__(256) expand_a_kernel(const float2 *L, int64_t 
   __shared__ float2 t[32][33];  // [l][i] of the tile
   __shared__ unsigned s_max[32];
   const int i0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
-  const int top = top_level(level, k);
+  __shared__ int s_up[kMaxK];
+  if (ty == 0) s_max[tx] = 0u;
+  stage_raise(level, k, s_up);
   auto at = [&](float2 z, int l) {
-    const float up = pow2(raised(level[l], top));
+    const float up = pow2(s_up[l]);
     return make_float2(z.x * up, z.y * up);
   };
-  if (ty == 0) s_max[tx] = 0u;
-  __syncthreads();
   if (!tr) {
     unsigned b = 0u;
-    if (i0 + tx < m)
+    if (i0 + tx < m) {
+#pragma unroll 8
       for (int l = ty; l < k; l += 8) b = max(b, mag_bits(at(L[i0 + tx + (int64_t)l * ld], l)));
+    }
     atomicMax(&s_max[tx], b);
   } else {
     for (int r = ty; r < 32; r += 8) {
       unsigned b = 0u;
-      if (i0 + r < m)
+      if (i0 + r < m) {
+#pragma unroll 8
         for (int l = tx; l < k; l += 32) b = max(b, mag_bits(at(L[l + (int64_t)(i0 + r) * ld], l)));
+      }
       b = __reduce_max_sync(0xffffffffu, b);
       if (tx == 0) s_max[r] = b;
     }
   }
-  for (int l0 = 0; l0 < Kp / 2; l0 += 32) {
+  for (int l0 = 32 * blockIdx.y; l0 < Kp / 2; l0 += 32 * gridDim.y) {
     __syncthreads();
     for (int r = ty; r < 32; r += 8) {
       if (!tr) {
@@ -462,20 +507,23 @@ __global__ void __launch_bounds__(256) expand_a_kernel(const float2 *L, int64_t 
 __global__ void __launch_bounds__(256) split_b_kernel(const float2 *U, int64_t ld, int k, int nc, int Kp, __half *hi,
                                                       __half *lo, float *cinv, const int *level) {
   const int lane = threadIdx.x & 31, j = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  __shared__ int s_up[kMaxK];
+  const float2 *u = U + (int64_t)min(j, nc - 1) * ld;
+  stage_raise(level, k, s_up);
   if (j >= nc) return;
-  const float2 *u = U + (int64_t)j * ld;
-  const int top = top_level(level, k);
   int b = INT_MIN;  // bits of the largest magnitude, less the powers of two
+#pragma unroll 8
   for (int l = lane; l < k; l += 32) {
     const unsigned v = mag_bits(u[l]);
-    if (v != 0u) b = max(b, (int)v - (raised(level[l], top) << 23));
+    if (v != 0u) b = max(b, (int)v - (s_up[l] << 23));
   }
   b = __reduce_max_sync(0xffffffffu, b);
   const int s = b == INT_MIN ? 0 : min(126, max(-126, 141 - (b >> 23)));
   if (lane == 0) cinv[j] = pow2(-s);
+#pragma unroll 8
   for (int l = lane; l < Kp / 2; l += 32) {
     const float2 z = l < k ? u[l] : make_float2(0.f, 0.f);
-    const int f = s - (l < k ? raised(level[l], top) : 0);
+    const int f = s - (l < k ? s_up[l] : 0);
     const float f1 = pow2(f >> 1), f2 = pow2(f - (f >> 1));
     __half2 h, g;
     split_half(z.x * f1 * f2, &h.x, &g.x);
@@ -523,16 +571,48 @@ size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
 }  // namespace
 
+// The expansion of L into the operands of tc_cgemm_update (own: room for its
+// columns' levels unless they are known).
+static void expand_a(Ctx *c, cudaStream_t st, const float2 *L, int64_t ldl, int m, int k, __half *ahi, __half *alo,
+                     float *rinv, int *own, const int *levels, bool trans_l) {
+  if (!levels) {
+    col_level_kernel<<<(unsigned)(trans_l ? (k + 3) / 4 : k), 256, 0, st>>>(L, ldl, m, k, own, trans_l);
+    c->launches++;
+  }
+  // few rows: their columns over several CTAs, each of which looks for the
+  // largest entries itself (20 us for 1,664 x 256, 10 with eight)
+  const int rb = (m + 31) / 32, cb = std::max(1, std::min((k + 31) / 32, 2 * c->nsm / rb));
+  expand_a_kernel<<<dim3(rb, cb), dim3(32, 8), 0, st>>>(L, ldl, m, k, padded_k(k), ahi, alo, rinv, levels ? levels : own,
+                                                        trans_l);
+  c->launches++;
+}
+
+// The expansion of L (m x k) alone, on stream st, for calls of tc_cgemm_update
+// with the same m, k and work and reuse_a.
+int tc_cgemm_expand(Ctx *c, cudaStream_t st, const float2 *L, int64_t ldl, int m, int k, float *work) {
+  const size_t half = up256(sizeof(__half) * 2 * (size_t)m * padded_k(k));
+  char *w = reinterpret_cast<char *>(work);
+  expand_a(c, st, L, ldl, m, k, (__half *)w, (__half *)(w + half), (float *)(w + 2 * half),
+           (int *)(w + 2 * half + up256(sizeof(float) * m)), nullptr, false);
+  MOM_CUDA(c, cudaGetLastError());
+  return MOM_OK;
+}
+
 // C (m x nc complex FP32, ldc) -= L (m x k, ldl) * U (k x nc, ldu) on the
 // tensor cores (two FP16 parts per operand, FP32-accurate).  m must be a
 // multiple of 64, k of 16.  work: tc_cgemm_work_bytes(m, nc, k) of device
 // scratch.  max_ctas > 0 caps the persistent grid.  reuse_a: work already holds
-// the expansion of this L (the previous call on the same stream had the same L,
-// m and k).  trans_l: L is given as its k x m transpose at L (ld ldl).
+// the expansion of this L (of the previous call, or of tc_cgemm_expand, with the
+// same L, m and k).  trans_l: L is given as its k x m transpose at L (ld ldl).  levels:
+// those of L's columns if they are known (tc_block_levels).
 int tc_cgemm_update(Ctx *c, float2 *C, int64_t ldc, const float2 *L, int64_t ldl, const float2 *U, int64_t ldu, int m,
-                    int nc, int k, float *work, int *err, int max_ctas, bool reuse_a, bool trans_l) {
+                    int nc, int k, float *work, int *err, int max_ctas, bool reuse_a, bool trans_l, const int *levels) {
   if (m <= 0 || nc <= 0 || k <= 0) return MOM_OK;
   if ((2 * m) % kBM != 0 || (2 * k) % 32 != 0) return fail(c, MOM_ERR_ARG, "tc_cgemm_update: unsupported shape");
+  for (int k0 = 0; k > kMaxK && k0 < k; k0 += kMaxK)  // (no LU or solve has that many)
+    MOM_TRY(tc_cgemm_update(c, C, ldc, L + k0 * (trans_l ? 1 : ldl), ldl, U + k0, ldu, m, nc, std::min(kMaxK, k - k0), work,
+                            err, max_ctas, false, trans_l));
+  if (k > kMaxK) return MOM_OK;
   const int Mr = 2 * m, Kp = padded_k(k);
   char *w = reinterpret_cast<char *>(work);
   auto take = [&](size_t bytes) {
@@ -540,20 +620,15 @@ int tc_cgemm_update(Ctx *c, float2 *C, int64_t ldc, const float2 *L, int64_t ldl
     w += up256(bytes);
     return p;
   };
-  // the expansion of L first: its place must not depend on nc (reuse_a)
+  // the expansion of L first: its place must not depend on nc (tc_cgemm_expand)
   __half *ahi = (__half *)take(sizeof(__half) * (size_t)Mr * Kp), *alo = (__half *)take(sizeof(__half) * (size_t)Mr * Kp);
   float *rinv = (float *)take(sizeof(float) * m);
-  int *level = (int *)take(sizeof(int) * k);
+  int *own = (int *)take(sizeof(int) * k);
+  const int *level = levels ? levels : own;
   __half *bhi = (__half *)take(sizeof(__half) * (size_t)nc * Kp), *blo = (__half *)take(sizeof(__half) * (size_t)nc * Kp);
   float *cinv = (float *)take(sizeof(float) * nc);
-  if (!reuse_a) {
-    col_level_kernel<<<(unsigned)(trans_l ? (k + 3) / 4 : k), 256, 0, c->stream>>>(L, ldl, m, k, level, trans_l);
-    expand_a_kernel<<<(unsigned)((m + 31) / 32), dim3(32, 8), 0, c->stream>>>(L, ldl, m, k, Kp, ahi, alo, rinv, level,
-                                                                               trans_l);
-    c->launches += 2;
-  }
-  split_b_kernel<<<(unsigned)((nc + 7) / 8), 256, 0, c->stream>>>(U, ldu, k, nc, Kp, bhi, blo, cinv,
-                                                                         level);
+  if (!reuse_a) expand_a(c, c->stream, L, ldl, m, k, ahi, alo, rinv, own, levels, trans_l);
+  split_b_kernel<<<(unsigned)((nc + 7) / 8), 256, 0, c->stream>>>(U, ldu, k, nc, Kp, bhi, blo, cinv, level);
   c->launches++;
   CUtensorMap mAhi, mAlo, mBhi, mBlo;
   MOM_TRY(make_map(c, &mAhi, ahi, Mr, Kp, kBM));
@@ -582,6 +657,17 @@ int tc_cgemm_update(Ctx *c, float2 *C, int64_t ldc, const float2 *L, int64_t ldl
   }
   c->launches++;
   c->tc_flops += 6.0 * Mr * (double)nc * 2 * k;  // three passes, 2 FLOP per real MAC
+  MOM_CUDA(c, cudaGetLastError());
+  return MOM_OK;
+}
+
+// Levels for the updates of a substitution by blocks of `rows` rows with the n x n
+// factors F (trans: their transpose): after[l] for the updates of the rows after
+// l's block, before[l] for those before it.
+int tc_block_levels(Ctx *c, const float2 *F, int64_t lda, int n, int rows, bool trans, int *after, int *before) {
+  if (trans) block_levels_kernel<true><<<(n + 31) / 32, 1024, 0, c->stream>>>(F, lda, n, rows, after, before);
+  else block_levels_kernel<false><<<(n + 3) / 4, 1024, 0, c->stream>>>(F, lda, n, rows, after, before);
+  c->launches++;
   MOM_CUDA(c, cudaGetLastError());
   return MOM_OK;
 }
