@@ -214,12 +214,10 @@ __device__ void face_build(const AdjTopo &t, int f, int snode, int scoord, FaceA
     for (int i = 0; i < 3; i++) o.mu[e][i] = o.bn[e][i] - o.cp[i];
 }
 
-// blocks_from_moments in the scalar type S, with the test face's geometry in
-// type GM, the source face's in GN and the centroid offset in GD (S by
-// default).
-template <typename S, typename GM = S, typename GN = GM, typename GD = GM>
-__device__ void blocks_generic(const Moments<S> &M, const GM mu[3][3], const GN nu[3][3], const GM slp[3],
-                               const GN slq[3], const GD d[3], Cx<S> fD, Cx<S> fH, double fK, bool self, Cx<S> *Sb,
+// blocks_from_moments in the scalar type S.
+template <typename S>
+__device__ void blocks_generic(const Moments<S> &M, const S mu[3][3], const S nu[3][3], const S slp[3],
+                               const S slq[3], const S d[3], Cx<S> fD, Cx<S> fH, double fK, bool self, Cx<S> *Sb,
                                Cx<S> *Kb) {
   Cx<S> KBv[3], KDmF[3];
   KBv[0] = {d[1] * M.KF[2].re - d[2] * M.KF[1].re + M.KE[0].re, d[1] * M.KF[2].im - d[2] * M.KF[1].im + M.KE[0].im};
@@ -233,7 +231,7 @@ __device__ void blocks_generic(const Moments<S> &M, const GM mu[3][3], const GN 
   Cx<S> beta[3], bq[3], cq[3];
 #pragma unroll
   for (int q = 0; q < 3; q++) {
-    const GN *v = nu[q];
+    const S *v = nu[q];
     beta[q] = {v[0] * M.TB[0].re + v[1] * M.TB[1].re + v[2] * M.TB[2].re,
                v[0] * M.TB[0].im + v[1] * M.TB[1].im + v[2] * M.TB[2].im};
     const auto dn0 = d[1] * v[2] - d[2] * v[1], dn1 = d[2] * v[0] - d[0] * v[2], dn2 = d[0] * v[1] - d[1] * v[0];
@@ -244,7 +242,7 @@ __device__ void blocks_generic(const Moments<S> &M, const GM mu[3][3], const GN 
   }
 #pragma unroll
   for (int p = 0; p < 3; p++) {
-    const GM *u = mu[p];
+    const S *u = mu[p];
     const Cx<S> alpha = {u[0] * M.TC[0].re + u[1] * M.TC[1].re + u[2] * M.TC[2].re,
                          u[0] * M.TC[0].im + u[1] * M.TC[1].im + u[2] * M.TC[2].im};
     const Cx<S> ap = {u[0] * KBv[0].re + u[1] * KBv[1].re + u[2] * KBv[2].re,
@@ -254,7 +252,7 @@ __device__ void blocks_generic(const Moments<S> &M, const GM mu[3][3], const GN 
                         {u[0] * KDmF[1].re - u[1] * KDmF[0].re, u[0] * KDmF[1].im - u[1] * KDmF[0].im}};
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-      const GN *v = nu[q];
+      const S *v = nu[q];
       const auto uv = u[0] * v[0] + u[1] * v[1] + u[2] * v[2];
       const auto ss = slp[p] * slq[q];
       const Cx<S> cD = {M.TA.re - beta[q].re - alpha.re + uv * M.TD.re, M.TA.im - beta[q].im - alpha.im + uv * M.TD.im};

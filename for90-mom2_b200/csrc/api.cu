@@ -122,7 +122,6 @@ void free_domain(DomDev &D) {
   cudaFree(D.inc_node);
   cudaFree(D.inc_face);
   cudaFree(D.nf_geo);
-  cudaFree(D.nf_bn);
   free_shg(D);
   D = DomDev();
 }

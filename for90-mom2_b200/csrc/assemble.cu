@@ -100,14 +100,10 @@ __device__ __forceinline__ void zero(Cx<T> &a) {
 
 // Point-pair loop.  rho_t: test point offsets (stride 3), rho_s: source
 // offsets with stride sstride between coordinates; w from constant memory.
-// SMOOTH selects the singularity-subtracted kernels (green.f90:40-97).  The
-// geometry has its own types (the value type T by default): G for the test
-// points, GS for the source points, GD for the centroid offset; the adjoint
-// runs T = dual numbers on plain FP64 geometry (permittivity) or on one dual
-// and one plain face (vertex coordinates).
-template <typename T, int NQ, bool SMOOTH, bool LOSSLESS = false, int LANES = 1, typename G = T, typename GS = G,
-          typename GD = G>
-__device__ __forceinline__ void pair_moments(const G *rho_t, const GS *rho_s, int sstride, const GD d[3], T kr, T ki,
+// SMOOTH selects the singularity-subtracted kernels (green.f90:40-97).  LANES
+// threads share a pair, each taking every LANES-th test point from `lane` on.
+template <typename T, int NQ, bool SMOOTH, bool LOSSLESS = false, int LANES = 1>
+__device__ __forceinline__ void pair_moments(const T *rho_t, const T *rho_s, int sstride, const T d[3], T kr, T ki,
                                              Moments<T> &M, int lane = 0) {
   zero(M.TA);
   zero(M.TD);
@@ -124,14 +120,14 @@ __device__ __forceinline__ void pair_moments(const G *rho_t, const GS *rho_s, in
   const T k2r = kr * kr - ki * ki, k2i = 2 * kr * ki;
 #pragma unroll 1
   for (int t = LANES > 1 ? lane : 0; t < NQ; t += LANES) {
-    const G rx = rho_t[3 * t], ry = rho_t[3 * t + 1], rz = rho_t[3 * t + 2];
-    const G wt = (G)c_qw[t];
+    const T rx = rho_t[3 * t], ry = rho_t[3 * t + 1], rz = rho_t[3 * t + 2];
+    const T wt = (T)c_qw[t];
     const auto ax = d[0] + rx, ay = d[1] + ry, az = d[2] + rz;
     Cx<T> G0 = {0, 0}, P0 = {0, 0}, G1[3] = {{0, 0}, {0, 0}, {0, 0}}, P1[3] = {{0, 0}, {0, 0}, {0, 0}};
 #pragma unroll
     for (int s = 0; s < NQ; s++) {
-      const GS sx = rho_s[(3 * s) * sstride], sy = rho_s[(3 * s + 1) * sstride], sz = rho_s[(3 * s + 2) * sstride];
-      const GS ws = (GS)c_qw[s];
+      const T sx = rho_s[(3 * s) * sstride], sy = rho_s[(3 * s + 1) * sstride], sz = rho_s[(3 * s + 2) * sstride];
+      const T ws = (T)c_qw[s];
       const auto dx = ax - sx, dy = ay - sy, dz = az - sz;
       const auto R2 = dx * dx + dy * dy + dz * dz;
       T gre, gim, pre, pim;
@@ -182,7 +178,7 @@ __device__ __forceinline__ void pair_moments(const G *rho_t, const GS *rho_s, in
       P1[2].re += pre * sz; P1[2].im += pim * sz;
     }
     // Test-side sums.
-    const G rr[3] = {rx, ry, rz};
+    const T rr[3] = {rx, ry, rz};
     M.TA.re += wt * (rx * G1[0].re + ry * G1[1].re + rz * G1[2].re);
     M.TA.im += wt * (rx * G1[0].im + ry * G1[1].im + rz * G1[2].im);
     M.TD.re += wt * G0.re;

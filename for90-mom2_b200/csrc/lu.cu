@@ -1399,9 +1399,9 @@ int lu_enqueue(Ctx *c, T *A, int precision, const LuWork &w) {
 // (instead of panel by panel) gives the same factors; the columns left of
 // the block are swapped at the same time (they hold L of earlier blocks,
 // which nothing reads any more).  Blocks whose trailing height is above
-// la_from * n, or whose panels need more than half of the SMs (over about
-// 30,800 rows: at most 416 rows per FP32 panel CTA), run without the overlap
-// (the panel would take too many SMs from the larger GEMM).
+// la_from * n, or with more than about 30,800 rows (where panels that exchange
+// through global memory, at most 416 rows per CTA, need half of the SMs), run
+// without the overlap.
 template <typename T>
 int lu_enqueue_la(Ctx *c, T *A, const LuWork &w) {
   const int64_t n = c->n, lda = c->lda;
@@ -1710,10 +1710,6 @@ int lu_enqueue_cluster(Ctx *c, T *A, const LuWork &w, int batch) {
   return MOM_OK;
 }
 
-// The schedule in use: by the cluster panels when all of them fit one cluster.
-template <typename T>
-int lu_issue(Ctx *c, T *A, int precision, const LuWork &w, int batch);
-
 // The look-ahead schedule serves the mixed path (tensor-core trailing
 // updates) with at least two outer blocks.
 bool use_lookahead(const Ctx *c, int precision) {
@@ -1721,7 +1717,8 @@ bool use_lookahead(const Ctx *c, int precision) {
          c->n > 2 * (int64_t)outer_of(c, true) * c->nb;
 }
 
-// Captures the factorisation of this precision into g (replacing what g held).
+// The schedule in use: by 64-column panels where all of them fit one cluster, by
+// outer blocks in the mixed path from kOuterFromOrder on.
 template <typename T>
 int lu_issue(Ctx *c, T *A, int precision, const LuWork &w, int batch) {
   // (with several matrices at once the 64-column updates fill the GPU)
@@ -1731,6 +1728,7 @@ int lu_issue(Ctx *c, T *A, int precision, const LuWork &w, int batch) {
   return use_lookahead(c, precision) ? lu_enqueue_la<T>(c, A, w) : lu_enqueue<T>(c, A, precision, w);
 }
 
+// Captures the factorisation of this precision into g (replacing what g held).
 template <typename T>
 int lu_capture(Ctx *c, T *A, int precision, const LuWork &w, int batch, Ctx::LuGraph &g,
                const std::vector<uintptr_t> &key) {
@@ -1966,10 +1964,6 @@ int lu_init_kernels(Ctx *c) {
 }
 
 namespace {
-}  // namespace
-
-namespace {
-
 
 // Autotuner of the panel parallelism.  The panel is latency bound: one
 // device-wide pivot exchange per column, whose cost grows with the number of

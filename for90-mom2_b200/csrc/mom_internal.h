@@ -96,7 +96,6 @@ struct DomDev {
   int *inc_node = nullptr, *inc_face = nullptr;
   // Face geometry of the near-field kernel (uploaded on first use).
   void *nf_geo = nullptr;
-  double *nf_bn = nullptr;
   // Symmetry group actions on this domain, [nga] (element 0 is the identity,
   // which uses the arrays above).
   std::vector<ActDev> act;

@@ -314,16 +314,12 @@ static int nfield_geometry(Ctx *c, DomDev &D) {
     for (int i = 0; i < 3; i++) g.n[i] = D.h_nrm[3 * (size_t)f + i];
   }
   void *pg = nullptr;
-  double *pb = nullptr;
-  if (cudaMalloc(&pg, sizeof(FaceGeo) * F) != cudaSuccess || cudaMalloc(&pb, sizeof(double) * 9 * F) != cudaSuccess) {
+  if (cudaMalloc(&pg, sizeof(FaceGeo) * F) != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(pg);
     return fail(c, MOM_ERR_ALLOC, "near-field geometry allocation failed");
   }
   D.nf_geo = pg;
-  D.nf_bn = pb;
   MOM_CUDA(c, cudaMemcpyAsync(pg, geo.data(), sizeof(FaceGeo) * F, cudaMemcpyHostToDevice, c->stream));
-  MOM_CUDA(c, cudaMemcpyAsync(pb, D.h_bn.data(), sizeof(double) * 9 * F, cudaMemcpyHostToDevice, c->stream));
   return MOM_OK;
 }
 
