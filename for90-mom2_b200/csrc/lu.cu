@@ -1586,9 +1586,9 @@ int lu_enqueue_la(Ctx *c, T *A, const LuWork &w) {
 constexpr int64_t kTcFromOrder = 2048;
 // From this order on the FP32 factorisation goes by outer blocks (lu_enqueue_la):
 // its updates read and write the trailing matrix three or four times less, which
-// the 64-column updates are bound by.  Whole calls, blocks of 256 against 64
-// columns: 7,260 unknowns 25.4 and 24.3 ms, 8,640 33.0 and 33.7 ms, 11,760 56.9
-// and 67.3 ms.
+// the 64-column updates are bound by.  Whole calls, outer blocks against 64
+// columns: 6,000 unknowns 18.5 and 16.3 ms, 7,260 24.4 and 22.3, 8,640 31.4 and
+// 31.5, 10,140 42.2 and 44.4, 11,760 54.0 and 62.3.
 constexpr int64_t kOuterFromOrder = 8192;
 
 // The factorisation when every panel fits one thread-block cluster: right

@@ -33,10 +33,11 @@
 //   warps 4-11 epilogue: tcgen05.ld the accumulator, C -= acc (coalesced);
 //             two warps per 32 rows, so that enough of C is in flight to keep
 //             up with the MMAs of a K = 512 tile
-// Bound: with n = 15,360 and K = 512 a tile's MMAs take 6.6 us, its operands
-// 786 KB through L2 and its part of C 262 KB of HBM traffic; the 59 trailing
-// updates of the factorisation take 27.7 ms (43.3 ms with TF32 parts, two
-// stages and four epilogue warps; 18.3 ms at the bf16 rate).
+// Bound: with n = 15,360 and blocks of 192 columns (real K = 384) a tile's MMAs
+// take 5 us, its operands 590 KB through L2 and its part of C 262 KB of HBM
+// traffic; the trailing updates of the factorisation take 34 ms (with 256 columns
+// 27.7, for dearer narrow updates between them; with TF32 parts, two stages and
+// four epilogue warps 43.3; 18.3 at the bf16 rate).
 // Every mbarrier wait is bounded; on timeout the kernel records the error,
 // stops issuing work, waits (bounded) for its own copies and for the MMAs
 // already issued, frees TMEM and exits.
