@@ -15,8 +15,9 @@
 // one FP32 TMEM accumulator) and the epilogue undoes the scaling.  An entry
 // keeps 22 bits, or 2^-40 of its row's (column's) largest scaled entry: rows of
 // A of any sizes, which grade L by column against U by row, cost nothing, and
-// an error in column j of the update stays below k 2^-39 of the largest
-// entry of column j of |L| |U|, as every column of L has an entry at its level.
+// what smaller entries lose beyond the 22 bits stays, in column j of the update,
+// below k 2^-39 of the largest entry of column j of |L| |U|, as every column of L
+// has an entry at its level.
 // Three passes on TF32 parts keep no more (the tensor core cuts the remainder
 // to TF32) at half the rate and twice the operand bytes.  Measured, relative
 // Frobenius error of C - L U against FP64, Gaussian operands (rows and columns
