@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
   constexpr int kRegWarps = T / 32;
   constexpr int kMsgChunks = (int)(sizeof(Msg) / 16);
   __shared__ Msg s_in[2][kRegMaxCluster];
-  __shared__ Msg s_out[kRegWarps];
+  __shared__ Msg s_out[2][kRegWarps];
   __shared__ unsigned s_wmag[2][kRegWarps];
   __shared__ __align__(8) unsigned long long s_bar[2];
   __shared__ E s_l11[W][W + 1];
@@ -237,7 +237,10 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
   // warp's best lane leaves its row in shared memory once it is up to date
   // (after `rest`), and after the barrier every thread sends its pieces of the
   // best warp's to the CTAs (one warp writing and sending its row after the
-  // barrier measured 3-10% slower).
+  // barrier measured 3-10% slower).  The rows alternate by column: a warp that
+  // has every CTA's message may write the next one while another warp of its
+  // CTA still sends its pieces of this one (to other CTAs: nothing here waits
+  // for those), and is past the next barrier before it writes the one after.
   auto propose = [&](int c, auto rest) {
     unsigned bm = 0u;
     int bp = pos[0], br = 0;
@@ -259,7 +262,7 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
     const E brp = recip_of(bv);
     rest();
     if (lane == best) {
-      Msg &o = s_out[wid];
+      Msg &o = s_out[par][wid];
       s_wmag[par][wid] = wm;
       o.mag = wm;
       o.pos = (unsigned short)bp;
@@ -271,7 +274,7 @@ __global__ void __launch_bounds__(T, 1) panel_reg_kernel(RegPanelArgs a) {
     __syncthreads();
     const unsigned k = s_wmag[par][lane % kRegWarps];
     const unsigned cm = __reduce_max_sync(0xffffffffu, k);
-    const uint4 *src = reinterpret_cast<const uint4 *>(&s_out[__ffs(__ballot_sync(0xffffffffu, k == cm)) - 1]);
+    const uint4 *src = reinterpret_cast<const uint4 *>(&s_out[par][__ffs(__ballot_sync(0xffffffffu, k == cm)) - 1]);
 #pragma unroll
     for (int i = 0; i < kSend; i++) {
       const int q = tid + i * T;

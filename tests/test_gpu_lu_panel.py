@@ -154,6 +154,23 @@ def test_rows_of_two_sizes(exponent, ns):
     s.close()
 
 
+@pytest.mark.parametrize("prec", [M.FP64, M.MIXED])
+def test_panels_of_concurrent_contexts(prec):
+    """Twelve contexts of one problem at once share the SMs, so the warps of a panel's CTA run far apart: every
+    context gives the same cross sections, to the bit, each time."""
+    ctx = [problem(3) for _ in range(12)]
+    lam = np.linspace(500e-9, 800e-9, 6)
+    om = [[M.omega_of(w) for w in lam]] * len(ctx)
+    ri = [[RI] * len(lam)] * len(ctx)
+    first = None
+    for _ in range(8):
+        out = M.sweep_many(ctx, om, ri, [M.src_pw(20, 30, 40)], prec)
+        first = first or out[0]
+        assert all(np.array_equal(a, b) for o in out for a, b in zip(o, first))
+    for s in ctx:
+        s.close()
+
+
 def test_tallest_cluster_panels():
     s = problem(5)
     assert 2 * s.N == 24576
